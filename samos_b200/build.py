@@ -8,6 +8,7 @@ that the built files sit in the source tree and travel with it.
 from __future__ import annotations
 
 import os
+import re
 import subprocess
 import sys
 
@@ -25,7 +26,9 @@ NVCC_COMMON = ["-std=c++17", "-O3", "-lineinfo", "-Xcompiler", "-fPIC"]
 # with -fmad=false: no a*b+c contraction, so device arithmetic follows the
 # reference's evaluation order term by term.  The FP32/BF16 network kernels of
 # the learned warm start have no bit-parity requirement and keep FMA.
-PARITY_UNITS = ("sg_engine.cu", "sg_static.cu")
+PARITY_UNITS = ("sg_engine.cu", "sg_static.cu", "sg_abp_plane_none.cu", "sg_abp_plane_polar.cu",
+                "sg_abp_plane_nematic.cu", "sg_abp_sphere_none.cu", "sg_abp_sphere_polar.cu",
+                "sg_abp_sphere_nematic.cu")
 FREE_UNITS = ("sg_ml.cu",)
 OBJ_DIR = os.path.join(PKG, "_build")
 
@@ -46,18 +49,33 @@ def _sources(d: str, exts: tuple[str, ...]) -> list[str]:
     return sorted(os.path.join(d, f) for f in os.listdir(d) if f.endswith(exts))
 
 
+def _unit_sources(path: str) -> list[str]:
+    """The unit and the project files that it includes, directly or not."""
+    seen, todo = [], [path]
+    while todo:
+        p = todo.pop()
+        if p in seen:
+            continue
+        seen.append(p)
+        for name in re.findall(r'^#include "([^"]+)"', open(p).read(), re.M):
+            todo += [q for q in (os.path.join(CSRC, name), os.path.join(INCLUDE, name)) if os.path.exists(q)]
+    return seen
+
+
 def build_engine(force: bool = False) -> str:
-    srcs = _sources(CSRC, (".cu", ".cuh")) + [os.path.join(INCLUDE, "samos_gpu.h")]
+    srcs = _sources(CSRC, (".cu", ".cuh", ".h")) + [os.path.join(INCLUDE, "samos_gpu.h")]
     if force or _stale(ENGINE_SO, srcs):
         os.makedirs(OBJ_DIR, exist_ok=True)
         objs, procs = [], []
         for unit in PARITY_UNITS + FREE_UNITS:  # independent units, compiled side by side
             obj = os.path.join(OBJ_DIR, unit.replace(".cu", ".o"))
+            objs.append(obj)
+            if not force and not _stale(obj, _unit_sources(os.path.join(CSRC, unit)) + [__file__]):
+                continue
             fmad = ["-fmad=false"] if unit in PARITY_UNITS else []
             cmd = [NVCC, *NVCC_COMMON, *fmad, *ARCH, f"-I{INCLUDE}", "-c", os.path.join(CSRC, unit), "-o", obj]
             print("+", " ".join(cmd), file=sys.stderr)
             procs.append((cmd, subprocess.Popen(cmd)))
-            objs.append(obj)
         for cmd, p in procs:
             if p.wait() != 0:
                 raise subprocess.CalledProcessError(p.returncode, cmd)

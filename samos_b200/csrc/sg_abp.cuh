@@ -83,7 +83,7 @@ constexpr int ABP_NTUNED = (int)(sizeof(ABP_TUNED) / sizeof(ABP_TUNED[0]));
 constexpr int LO_KEYS = 128;  // distinct sort keys the counting sort handles (list lengths 0..126 + padding)
 static_assert(BLOCK == LO_KEYS, "k_lane_order scans one key per thread");
 
-__global__ void __launch_bounds__(BLOCK)
+static __global__ void __launch_bounds__(BLOCK)
 k_lane_order(const Replica* __restrict__ reps, const int* __restrict__ blk_rep, NbList nl,
              uint8_t* __restrict__ order, const int* __restrict__ blist = nullptr) {
   constexpr int NW = BLOCK / 32;
@@ -625,7 +625,7 @@ constexpr int TILE_WIN = 16384;  // slot window per block (bitmap bits)
 constexpr int TILE_MAX = 640;    // distinct neighbour records staged per block
 constexpr int TILE_QMAX = 24;    // list ranks whose positions are staged (deeper ranks read global memory)
 
-__global__ void __launch_bounds__(BLOCK)
+static __global__ void __launch_bounds__(BLOCK)
 k_tile_prep(const Replica* __restrict__ reps, const int* __restrict__ blk_rep, NbList nl, int* __restrict__ tile_n,
             int* __restrict__ tile_slot, uint16_t* __restrict__ nbpos, const int* __restrict__ blist = nullptr) {
   __shared__ uint32_t bm[TILE_WIN / 32];

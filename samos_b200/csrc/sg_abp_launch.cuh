@@ -1,0 +1,107 @@
+// sg_abp_launch.cuh -- variant dispatch of the specialised step kernels for
+// one shape and aligner, instantiated by the sg_abp_*.cu units.
+#pragma once
+#include "sg_abp_launch.h"
+
+namespace sg {
+
+template <int SHAPE, int ALIGN, bool SP, bool ENERGY, int VAR>
+static void launch_abp_v(const AbpLaunch& L) {
+  k_abp_step<SHAPE, ALIGN, SP, ENERGY, VAR><<<L.nblocks, BLOCK, 0, L.stream>>>(
+      L.abp, L.blk_rep, L.clk, L.Gin, L.Gout, L.Hin, L.Hout, L.cur, L.st, L.nl, L.rebuild,
+      L.status, L.apply_e1, L.last, L.epart, L.nblocks, L.lane_order, L.abp0);
+}
+
+// cudaFuncSetAttribute is per device: remember, per kernel, the devices it
+// has been raised on.
+template <typename K>
+static void raise_smem(K kernel, size_t smem, unsigned* done_mask, int device) {
+  const unsigned bit = 1u << (device & 31);
+  if (!(*done_mask & bit)) {
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    *done_mask |= bit;
+  }
+}
+
+template <int SHAPE, int ALIGN, bool SP, bool ENERGY>
+static void launch_abp_flat(const AbpLaunch& L) {
+  constexpr size_t smem = flat_smem_bytes<SHAPE, ENERGY>();
+  static unsigned done = 0;
+  raise_smem(k_abp_flat<SHAPE, ALIGN, SP, ENERGY>, smem, &done, L.device);
+  k_abp_flat<SHAPE, ALIGN, SP, ENERGY><<<L.nblocks, BLOCK, smem, L.stream>>>(
+      L.abp, L.blk_rep, L.clk, L.Gin, L.Gout, L.Hin, L.Hout, L.cur, L.st, L.nl, L.rebuild,
+      L.status, L.apply_e1, L.last, L.epart, L.nblocks);
+}
+
+template <int SHAPE, int ALIGN, bool SP, bool ENERGY, int CH, int MINB>
+static void launch_abp_staged(const AbpLaunch& L) {
+  constexpr size_t smem = staged_smem_bytes<SHAPE, ALIGN, CH>();
+  static unsigned done = 0;
+  raise_smem(k_abp_staged<SHAPE, ALIGN, SP, ENERGY, CH, MINB>, smem, &done, L.device);
+  k_abp_staged<SHAPE, ALIGN, SP, ENERGY, CH, MINB><<<L.nblocks, BLOCK, smem, L.stream>>>(
+      L.abp, L.blk_rep, L.clk, L.Gin, L.Gout, L.Hin, L.Hout, L.cur, L.st, L.nl, L.rebuild,
+      L.status, L.apply_e1, L.last, L.epart, L.nblocks);
+}
+
+template <int SHAPE, int ALIGN, bool SP, bool ENERGY, int MINB>
+static void launch_abp_tile(const AbpLaunch& L) {
+  constexpr size_t smem = tile_smem_bytes<SHAPE, ALIGN>();
+  static unsigned done = 0;
+  raise_smem(k_abp_tile<SHAPE, ALIGN, SP, ENERGY, MINB>, smem, &done, L.device);
+  k_abp_tile<SHAPE, ALIGN, SP, ENERGY, MINB><<<L.nblocks, BLOCK, smem, L.stream>>>(
+      L.abp, L.blk_rep, L.clk, L.Gin, L.Gout, L.Hin, L.Hout, L.cur, L.st, L.nl, L.rebuild,
+      L.status, L.apply_e1, L.last, L.epart, L.nblocks, L.tile_n, L.tile_slot, L.nbpos);
+}
+
+template <int SHAPE, int ALIGN, bool SP>
+static void launch_abp3(const AbpLaunch& L) {
+  // energy-reporting steps: the pipelined kernel (by value for one replica)
+  if (L.energy) {
+    if (L.nrep > 1) launch_abp_v<SHAPE, ALIGN, SP, true, 17>(L);
+    else launch_abp_v<SHAPE, ALIGN, SP, true, 22>(L);
+    return;
+  }
+  // by-value variants carry one replica's parameters: several replicas take the twin
+  switch (L.nrep > 1 ? abp_twin(L.variant) : L.variant) {
+    case 5: launch_abp_flat<SHAPE, ALIGN, SP, false>(L); break;
+    case 6: launch_abp_staged<SHAPE, ALIGN, SP, false, 4, 4>(L); break;
+    case 7: launch_abp_staged<SHAPE, ALIGN, SP, false, 4, 5>(L); break;
+    case 8: launch_abp_tile<SHAPE, ALIGN, SP, false, 5>(L); break;
+    case 9: launch_abp_v<SHAPE, ALIGN, SP, false, 9>(L); break;
+    case 10: launch_abp_v<SHAPE, ALIGN, SP, false, 10>(L); break;
+    case 11: launch_abp_v<SHAPE, ALIGN, SP, false, 11>(L); break;
+    case 12: launch_abp_v<SHAPE, ALIGN, SP, false, 12>(L); break;
+    case 13: launch_abp_v<SHAPE, ALIGN, SP, false, 13>(L); break;
+    case 14: launch_abp_v<SHAPE, ALIGN, SP, false, 14>(L); break;
+    case 15: launch_abp_v<SHAPE, ALIGN, SP, false, 15>(L); break;
+    case 16: launch_abp_v<SHAPE, ALIGN, SP, false, 16>(L); break;
+    case 17: launch_abp_v<SHAPE, ALIGN, SP, false, 17>(L); break;
+    case 18: launch_abp_v<SHAPE, ALIGN, SP, false, 18>(L); break;
+    case 19: launch_abp_v<SHAPE, ALIGN, SP, false, 19>(L); break;
+    case 20: launch_abp_v<SHAPE, ALIGN, SP, false, 20>(L); break;
+    case 21: launch_abp_v<SHAPE, ALIGN, SP, false, 21>(L); break;
+    case 22: launch_abp_v<SHAPE, ALIGN, SP, false, 22>(L); break;
+    case 23: launch_abp_v<SHAPE, ALIGN, SP, false, 23>(L); break;
+    case 24: launch_abp_v<SHAPE, ALIGN, SP, false, 24>(L); break;
+    case 25: launch_abp_v<SHAPE, ALIGN, SP, false, 25>(L); break;
+    case 26: launch_abp_v<SHAPE, ALIGN, SP, false, 26>(L); break;
+    case 27: launch_abp_v<SHAPE, ALIGN, SP, false, 27>(L); break;
+    case 28: launch_abp_v<SHAPE, ALIGN, SP, false, 28>(L); break;
+    case 29: launch_abp_v<SHAPE, ALIGN, SP, false, 29>(L); break;
+    case 30: launch_abp_v<SHAPE, ALIGN, SP, false, 30>(L); break;
+    case 31: launch_abp_v<SHAPE, ALIGN, SP, false, 31>(L); break;
+    case 0: launch_abp_v<SHAPE, ALIGN, SP, false, 0>(L); break;
+    case 1: launch_abp_v<SHAPE, ALIGN, SP, false, 1>(L); break;
+    case 2: launch_abp_v<SHAPE, ALIGN, SP, false, 2>(L); break;
+    case 3: launch_abp_v<SHAPE, ALIGN, SP, false, 3>(L); break;
+    default: launch_abp_v<SHAPE, ALIGN, SP, false, 4>(L); break;
+  }
+}
+
+template <int SHAPE, int ALIGN>
+static void launch_abp_unit(const AbpLaunch& L) {
+  if (L.self_propulsion) launch_abp3<SHAPE, ALIGN, true>(L);
+  else launch_abp3<SHAPE, ALIGN, false>(L);
+}
+
+}  // namespace sg

@@ -1,0 +1,4 @@
+// Step-kernel variants of the active-Brownian program: plane, polar aligner.
+#include "sg_abp_launch.cuh"
+
+void sg::launch_abp_plane_polar(const AbpLaunch& L) { launch_abp_unit<HOT_PLANE, ALIGN_POLAR>(L); }

@@ -1,0 +1,4 @@
+// Step-kernel variants of the active-Brownian program: sphere, no aligner.
+#include "sg_abp_launch.cuh"
+
+void sg::launch_abp_sphere_none(const AbpLaunch& L) { launch_abp_unit<HOT_SPHERE, ABP_ALIGN_NONE>(L); }

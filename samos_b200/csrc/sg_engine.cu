@@ -2,7 +2,7 @@
 // include/samos_gpu.h.  One stream per handle; device buffers are allocated
 // once per configuration and reused by every step.
 #include "samos_gpu.h"
-#include "sg_abp.cuh"
+#include "sg_abp_launch.h"
 
 #include <algorithm>
 #include <cmath>
@@ -1708,47 +1708,6 @@ static int abp_upload(sg_system* s) {
 
 }  // extern "C"
 
-template <int SHAPE, int ALIGN, bool SP, bool ENERGY, int VAR>
-static void launch_abp_v(sg_system* s, bool apply_e1, bool last) {
-  const int b = s->hot_buf;
-  k_abp_step<SHAPE, ALIGN, SP, ENERGY, VAR><<<s->nblocks, BLOCK, 0, s->stream>>>(
-      s->abp, s->blk_rep, s->clk, s->G[b], s->G[1 - b], s->H[b], s->H[1 - b], s->cur, s->st, s->nl, s->rebuild,
-      s->status, apply_e1 ? 1 : 0, last ? 1 : 0, s->epart, s->nblocks, s->lane_order, s->abp0_h);
-}
-
-// cudaFuncSetAttribute is per device: remember, per kernel, the devices it
-// has been raised on.
-template <typename K>
-static void raise_smem(K kernel, size_t smem, unsigned* done_mask, int device) {
-  const unsigned bit = 1u << (device & 31);
-  if (!(*done_mask & bit)) {
-    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    *done_mask |= bit;
-  }
-}
-
-template <int SHAPE, int ALIGN, bool SP, bool ENERGY>
-static void launch_abp_flat(sg_system* s, bool apply_e1, bool last) {
-  const int b = s->hot_buf;
-  constexpr size_t smem = flat_smem_bytes<SHAPE, ENERGY>();
-  static unsigned done = 0;
-  raise_smem(k_abp_flat<SHAPE, ALIGN, SP, ENERGY>, smem, &done, s->device);
-  k_abp_flat<SHAPE, ALIGN, SP, ENERGY><<<s->nblocks, BLOCK, smem, s->stream>>>(
-      s->abp, s->blk_rep, s->clk, s->G[b], s->G[1 - b], s->H[b], s->H[1 - b], s->cur, s->st, s->nl, s->rebuild,
-      s->status, apply_e1 ? 1 : 0, last ? 1 : 0, s->epart, s->nblocks);
-}
-
-template <int SHAPE, int ALIGN, bool SP, bool ENERGY, int CH, int MINB>
-static void launch_abp_staged(sg_system* s, bool apply_e1, bool last) {
-  const int b = s->hot_buf;
-  constexpr size_t smem = staged_smem_bytes<SHAPE, ALIGN, CH>();
-  static unsigned done = 0;
-  raise_smem(k_abp_staged<SHAPE, ALIGN, SP, ENERGY, CH, MINB>, smem, &done, s->device);
-  k_abp_staged<SHAPE, ALIGN, SP, ENERGY, CH, MINB><<<s->nblocks, BLOCK, smem, s->stream>>>(
-      s->abp, s->blk_rep, s->clk, s->G[b], s->G[1 - b], s->H[b], s->H[1 - b], s->cur, s->st, s->nl, s->rebuild,
-      s->status, apply_e1 ? 1 : 0, last ? 1 : 0, s->epart, s->nblocks);
-}
-
 // (Re)derive the tile data from the current lists (after any list build).
 static int tile_prep(sg_system* s) {
   DevBuf& m = s->mem;
@@ -1768,73 +1727,28 @@ static int tile_prep(sg_system* s) {
   return SG_OK;
 }
 
-template <int SHAPE, int ALIGN, bool SP, bool ENERGY, int MINB>
-static void launch_abp_tile(sg_system* s, bool apply_e1, bool last) {
-  const int b = s->hot_buf;  // tile data prepared by step_hot
-  constexpr size_t smem = tile_smem_bytes<SHAPE, ALIGN>();
-  static unsigned done = 0;
-  raise_smem(k_abp_tile<SHAPE, ALIGN, SP, ENERGY, MINB>, smem, &done, s->device);
-  k_abp_tile<SHAPE, ALIGN, SP, ENERGY, MINB><<<s->nblocks, BLOCK, smem, s->stream>>>(
-      s->abp, s->blk_rep, s->clk, s->G[b], s->G[1 - b], s->H[b], s->H[1 - b], s->cur, s->st, s->nl, s->rebuild,
-      s->status, apply_e1 ? 1 : 0, last ? 1 : 0, s->epart, s->nblocks, s->tile_n, s->tile_slot, s->nbpos);
-}
-
-template <int SHAPE, int ALIGN, bool SP>
-static void launch_abp3(sg_system* s, bool apply_e1, bool last, bool energy) {
-  // energy-reporting steps: the pipelined kernel (by value for one replica)
-  if (energy) {
-    if (s->nrep > 1) launch_abp_v<SHAPE, ALIGN, SP, true, 17>(s, apply_e1, last);
-    else launch_abp_v<SHAPE, ALIGN, SP, true, 22>(s, apply_e1, last);
-    return;
-  }
-  // by-value variants carry one replica's parameters: several replicas take the twin
-  switch (s->nrep > 1 ? abp_twin(s->abp_variant) : s->abp_variant) {
-    case 5: launch_abp_flat<SHAPE, ALIGN, SP, false>(s, apply_e1, last); break;
-    case 6: launch_abp_staged<SHAPE, ALIGN, SP, false, 4, 4>(s, apply_e1, last); break;
-    case 7: launch_abp_staged<SHAPE, ALIGN, SP, false, 4, 5>(s, apply_e1, last); break;
-    case 8: launch_abp_tile<SHAPE, ALIGN, SP, false, 5>(s, apply_e1, last); break;
-    case 9: launch_abp_v<SHAPE, ALIGN, SP, false, 9>(s, apply_e1, last); break;
-    case 10: launch_abp_v<SHAPE, ALIGN, SP, false, 10>(s, apply_e1, last); break;
-    case 11: launch_abp_v<SHAPE, ALIGN, SP, false, 11>(s, apply_e1, last); break;
-    case 12: launch_abp_v<SHAPE, ALIGN, SP, false, 12>(s, apply_e1, last); break;
-    case 13: launch_abp_v<SHAPE, ALIGN, SP, false, 13>(s, apply_e1, last); break;
-    case 14: launch_abp_v<SHAPE, ALIGN, SP, false, 14>(s, apply_e1, last); break;
-    case 15: launch_abp_v<SHAPE, ALIGN, SP, false, 15>(s, apply_e1, last); break;
-    case 16: launch_abp_v<SHAPE, ALIGN, SP, false, 16>(s, apply_e1, last); break;
-    case 17: launch_abp_v<SHAPE, ALIGN, SP, false, 17>(s, apply_e1, last); break;
-    case 18: launch_abp_v<SHAPE, ALIGN, SP, false, 18>(s, apply_e1, last); break;
-    case 19: launch_abp_v<SHAPE, ALIGN, SP, false, 19>(s, apply_e1, last); break;
-    case 20: launch_abp_v<SHAPE, ALIGN, SP, false, 20>(s, apply_e1, last); break;
-    case 21: launch_abp_v<SHAPE, ALIGN, SP, false, 21>(s, apply_e1, last); break;
-    case 22: launch_abp_v<SHAPE, ALIGN, SP, false, 22>(s, apply_e1, last); break;
-    case 23: launch_abp_v<SHAPE, ALIGN, SP, false, 23>(s, apply_e1, last); break;
-    case 24: launch_abp_v<SHAPE, ALIGN, SP, false, 24>(s, apply_e1, last); break;
-    case 25: launch_abp_v<SHAPE, ALIGN, SP, false, 25>(s, apply_e1, last); break;
-    case 26: launch_abp_v<SHAPE, ALIGN, SP, false, 26>(s, apply_e1, last); break;
-    case 27: launch_abp_v<SHAPE, ALIGN, SP, false, 27>(s, apply_e1, last); break;
-    case 28: launch_abp_v<SHAPE, ALIGN, SP, false, 28>(s, apply_e1, last); break;
-    case 29: launch_abp_v<SHAPE, ALIGN, SP, false, 29>(s, apply_e1, last); break;
-    case 30: launch_abp_v<SHAPE, ALIGN, SP, false, 30>(s, apply_e1, last); break;
-    case 31: launch_abp_v<SHAPE, ALIGN, SP, false, 31>(s, apply_e1, last); break;
-    case 0: launch_abp_v<SHAPE, ALIGN, SP, false, 0>(s, apply_e1, last); break;
-    case 1: launch_abp_v<SHAPE, ALIGN, SP, false, 1>(s, apply_e1, last); break;
-    case 2: launch_abp_v<SHAPE, ALIGN, SP, false, 2>(s, apply_e1, last); break;
-    case 3: launch_abp_v<SHAPE, ALIGN, SP, false, 3>(s, apply_e1, last); break;
-    default: launch_abp_v<SHAPE, ALIGN, SP, false, 4>(s, apply_e1, last); break;
-  }
-}
-
-template <int SHAPE>
-static void launch_abp(sg_system* s, bool apply_e1, bool last, bool energy) {
+static void launch_abp(sg_system* s, int shape, bool apply_e1, bool last, bool energy) {
   const Program& P = s->prog;
+  const int b = s->hot_buf;
+  AbpLaunch L{};
+  L.abp = s->abp; L.abp0 = s->abp0_h; L.blk_rep = s->blk_rep; L.clk = s->clk;
+  L.Gin = s->G[b]; L.Gout = s->G[1 - b]; L.Hin = s->H[b]; L.Hout = s->H[1 - b];
+  L.cur = s->cur; L.st = s->st; L.nl = s->nl; L.rebuild = s->rebuild; L.status = s->status;
+  L.apply_e1 = apply_e1 ? 1 : 0; L.last = last ? 1 : 0; L.energy = energy;
+  L.epart = s->epart; L.nblocks = s->nblocks; L.lane_order = s->lane_order;
+  L.tile_n = s->tile_n; L.tile_slot = s->tile_slot; L.nbpos = s->nbpos;
+  L.nrep = s->nrep; L.variant = s->abp_variant; L.device = s->device; L.stream = s->stream;
+  L.self_propulsion = P.next == 1;
   const int al = P.nalign == 0 ? ABP_ALIGN_NONE : P.align[0].kind;
-  const bool sp = P.next == 1;
-  if (al == ABP_ALIGN_NONE) { if (sp) launch_abp3<SHAPE, ABP_ALIGN_NONE, true>(s, apply_e1, last, energy);
-                              else launch_abp3<SHAPE, ABP_ALIGN_NONE, false>(s, apply_e1, last, energy); }
-  else if (al == ALIGN_POLAR) { if (sp) launch_abp3<SHAPE, ALIGN_POLAR, true>(s, apply_e1, last, energy);
-                                else launch_abp3<SHAPE, ALIGN_POLAR, false>(s, apply_e1, last, energy); }
-  else { if (sp) launch_abp3<SHAPE, ALIGN_NEMATIC, true>(s, apply_e1, last, energy);
-         else launch_abp3<SHAPE, ALIGN_NEMATIC, false>(s, apply_e1, last, energy); }
+  if (shape == HOT_PLANE) {
+    if (al == ABP_ALIGN_NONE) launch_abp_plane_none(L);
+    else if (al == ALIGN_POLAR) launch_abp_plane_polar(L);
+    else launch_abp_plane_nematic(L);
+  } else {
+    if (al == ABP_ALIGN_NONE) launch_abp_sphere_none(L);
+    else if (al == ALIGN_POLAR) launch_abp_sphere_polar(L);
+    else launch_abp_sphere_nematic(L);
+  }
 }
 
 extern "C" {
@@ -1862,8 +1776,7 @@ static int step_hot(sg_system* s, int shape, bool apply_e1, bool last, bool ener
   }
   if (s->profile) CU(s, cudaEventRecord(s->ev_k0, s->stream));
   if (s->abp_on) {
-    if (shape == HOT_PLANE) launch_abp<HOT_PLANE>(s, apply_e1, last, energy);
-    else launch_abp<HOT_SPHERE>(s, apply_e1, last, energy);
+    launch_abp(s, shape, apply_e1, last, energy);
   } else if (shape == HOT_PLANE) launch_hot<HOT_PLANE>(s, apply_e1, last, energy);
   else launch_hot<HOT_SPHERE>(s, apply_e1, last, energy);
   LAUNCH_CHECK(s);

@@ -290,7 +290,7 @@ __device__ __forceinline__ bool finite3(double a, double b, double c) {
 // ---------------------------------------------------------------------------
 
 // Constrainer::enforce on every particle (samos.cpp:887-888)
-__global__ void k_enforce(Program P, const Replica* __restrict__ reps, const int* __restrict__ blk_rep,
+static __global__ void k_enforce(Program P, const Replica* __restrict__ reps, const int* __restrict__ blk_rep,
                           Dyn d, Stat st, const Clock* __restrict__ frozen, const int* __restrict__ blist = nullptr) {
   const int bid_ = blist ? blist[blockIdx.x] : (int)blockIdx.x;  // block of the packed layout
   const int r = blk_rep[bid_];
@@ -394,7 +394,7 @@ k_step_brownian(Program P, const Replica* __restrict__ reps, const int* __restri
 }
 
 // Skin test over all particles of the current buffer (unfused path)
-__global__ void k_skin(Program P, const Replica* __restrict__ reps, const int* __restrict__ blk_rep,
+static __global__ void k_skin(Program P, const Replica* __restrict__ reps, const int* __restrict__ blk_rep,
                        Dyn d, NbList nl, int* __restrict__ rebuild, int* __restrict__ status, const int* __restrict__ blist = nullptr) {
   const int bid_ = blist ? blist[blockIdx.x] : (int)blockIdx.x;  // block of the packed layout
   const int r = blk_rep[bid_];
@@ -430,7 +430,7 @@ __device__ __forceinline__ void tail_one(const Program& P, const Replica& R, Clo
   C.time_step++;
 }
 
-__global__ void k_tail(Program P, const Replica* __restrict__ reps, Clock* clk, int nrep) {
+static __global__ void k_tail(Program P, const Replica* __restrict__ reps, Clock* clk, int nrep) {
   const int r = blockIdx.x * blockDim.x + threadIdx.x;
   if (r >= nrep) return;
   tail_one(P, reps[r], clk[r]);
@@ -441,7 +441,7 @@ __global__ void k_tail(Program P, const Replica* __restrict__ reps, Clock* clk, 
 // enqueued did nothing (its kernel saw the halt) and neither does this.
 // Otherwise the step counts as executed, and if it flagged a rebuild every
 // replica is halted until the host has rebuilt the lists.
-__global__ void k_tail_batch(Program P, const Replica* __restrict__ reps, Clock* clk, int nrep,
+static __global__ void k_tail_batch(Program P, const Replica* __restrict__ reps, Clock* clk, int nrep,
                              const int* __restrict__ rebuild, int* __restrict__ executed) {
   __shared__ int halted, any;
   if (threadIdx.x == 0) { halted = clk[0].halt; any = 0; }
@@ -457,7 +457,7 @@ __global__ void k_tail_batch(Program P, const Replica* __restrict__ reps, Clock*
   if (threadIdx.x == 0) (*executed)++;
 }
 
-__global__ void k_set_halt(Clock* clk, int nrep, int v) {
+static __global__ void k_set_halt(Clock* clk, int nrep, int v) {
   const int r = blockIdx.x * blockDim.x + threadIdx.x;
   if (r < nrep) clk[r].halt = v;
 }
@@ -468,7 +468,7 @@ __global__ void k_set_halt(Clock* clk, int nrep, int v) {
 // ---------------------------------------------------------------------------
 // pre_enforce: the start-of-step enforce (samos.cpp:887-888) folded in, when
 // no force pass comes between it and this half (forces reused)
-__global__ void k_langevin_a(Program P, const Replica* __restrict__ reps, const int* __restrict__ blk_rep,
+static __global__ void k_langevin_a(Program P, const Replica* __restrict__ reps, const int* __restrict__ blk_rep,
                              const Clock* __restrict__ clk, Dyn d, Stat st, int c, const double* Rn, int pre_enforce) {
   const int r = my_replica(blk_rep);
   if (clk[r].halt) return;  // batched stepping: a rebuild is pending
@@ -528,7 +528,7 @@ __global__ void k_langevin_a(Program P, const Replica* __restrict__ reps, const 
 
 // skin: the step's skin test (neighbour_list.cpp:278-302) on the final
 // positions, folded in
-__global__ void k_langevin_b(Program P, const Replica* __restrict__ reps, const int* __restrict__ blk_rep,
+static __global__ void k_langevin_b(Program P, const Replica* __restrict__ reps, const int* __restrict__ blk_rep,
                              const Clock* __restrict__ clk, Dyn d, Stat st, int c, double* Rn, NbList nl,
                              int* __restrict__ rebuild, int* __restrict__ status, int skin) {
   const int r = my_replica(blk_rep);
@@ -602,7 +602,7 @@ __global__ void k_langevin_b(Program P, const Replica* __restrict__ reps, const 
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ double sign_of(double x) { return x >= 0.0 ? 1.0 : -1.0; }  // integrator_nve.hpp:38
 
-__global__ void k_nve_a(Program P, const Replica* __restrict__ reps, const int* __restrict__ blk_rep,
+static __global__ void k_nve_a(Program P, const Replica* __restrict__ reps, const int* __restrict__ blk_rep,
                         const Clock* __restrict__ clk, Dyn d, Stat st, int c, int pre_enforce) {
   const int r = my_replica(blk_rep);
   if (clk[r].halt) return;  // batched stepping: a rebuild is pending
@@ -633,7 +633,7 @@ __global__ void k_nve_a(Program P, const Replica* __restrict__ reps, const int* 
   store_dyn_moved<true, false>(d, k, p);
 }
 
-__global__ void k_nve_b(Program P, const Replica* __restrict__ reps, const int* __restrict__ blk_rep,
+static __global__ void k_nve_b(Program P, const Replica* __restrict__ reps, const int* __restrict__ blk_rep,
                         const Clock* __restrict__ clk, Dyn d, Stat st, int c, NbList nl, int* __restrict__ rebuild,
                         int* __restrict__ status, int skin) {
   const int r = my_replica(blk_rep);
@@ -672,7 +672,7 @@ __global__ void k_nve_b(Program P, const Replica* __restrict__ reps, const int* 
 // FIRE (integrators/integrator_fire.cpp:34-148)
 // ---------------------------------------------------------------------------
 // first half: half kick, drift, enforce, omega, director rotation (49-66)
-__global__ void k_fire_a(Program P, const Replica* __restrict__ reps, const int* __restrict__ blk_rep,
+static __global__ void k_fire_a(Program P, const Replica* __restrict__ reps, const int* __restrict__ blk_rep,
                          const Clock* __restrict__ clk, Dyn d, Stat st, int pre_enforce,
                          const int* __restrict__ blist = nullptr) {
   const int bid_ = blist ? blist[blockIdx.x] : (int)blockIdx.x;  // block of the packed layout
@@ -703,7 +703,7 @@ __global__ void k_fire_a(Program P, const Replica* __restrict__ reps, const int*
 // order, then a fixed tree over the threads (the same bits for a replica run
 // alone or inside an ensemble).  Returns P, |F|^2, |v|^2, max |F_i|^2, E on
 // thread 0.
-__device__ void fire_sums(const Program& P, const double* part, const double* epart, int nblocks, int b0, int nb,
+static __device__ void fire_sums(const Program& P, const double* part, const double* epart, int nblocks, int b0, int nb,
                           double out[5]) {
   __shared__ double red[5][BLOCK];
   const int t = threadIdx.x;
@@ -730,7 +730,7 @@ __device__ void fire_sums(const Program& P, const double* part, const double* ep
 // FIRE's convergence test and dt / alpha control on the replica's sums
 // (integrator_fire.cpp:96-147).  alpha_mix[r] keeps the alpha the mixing step
 // must use (the value before this update).
-__device__ void fire_control(const Replica& R, Clock& C, int r, int c, const double sums[5], int driver,
+static __device__ void fire_control(const Replica& R, Clock& C, int r, int c, const double sums[5], int driver,
                              double* alpha_mix) {
   if (C.fire_conv_step >= 0 || C.halt) return;
   const double* ip = R.integ_p[c];
@@ -775,7 +775,7 @@ __device__ void fire_control(const Replica& R, Clock& C, int r, int c, const dou
 // `terms` (three arrays of `stride` doubles, indexed by replica offset + id).
 // One warp: 32 terms loaded at a time, then added in order through shuffles,
 // so every lane holds the same sequential sums.
-__device__ void fire_ordered_sums(const double* __restrict__ terms, int stride, int off, int n, double out[3]) {
+static __device__ void fire_ordered_sums(const double* __restrict__ terms, int stride, int off, int n, double out[3]) {
   const int lane = threadIdx.x & 31;
   double sP = 0.0, sF = 0.0, sV = 0.0;
   for (int base = 0; base < n; base += 32) {
@@ -793,7 +793,7 @@ __device__ void fire_ordered_sums(const double* __restrict__ terms, int stride, 
   out[0] = sP; out[1] = sF; out[2] = sV;
 }
 
-__global__ void k_fire_b(Program P, const Replica* __restrict__ reps, const int* __restrict__ blk_rep,
+static __global__ void k_fire_b(Program P, const Replica* __restrict__ reps, const int* __restrict__ blk_rep,
                          Clock* __restrict__ clk, Dyn d, Stat st, double* part, int nblocks, const int* rep_blk0,
                          const int* rep_nblk, const double* epart, int c, int driver, double* alpha_mix,
                          int* __restrict__ fire_cnt, const int* __restrict__ blist = nullptr,
@@ -860,7 +860,7 @@ __global__ void k_fire_b(Program P, const Replica* __restrict__ reps, const int*
 
 // FIRE velocity mixing (110-121) with the pre-update alpha, then the
 // P <= 0 restart that zeroes the velocities (131-142).
-__global__ void k_fire_d(Program P, const Replica* __restrict__ reps, const int* __restrict__ blk_rep,
+static __global__ void k_fire_d(Program P, const Replica* __restrict__ reps, const int* __restrict__ blk_rep,
                          const Clock* __restrict__ clk, Dyn d, const double* alpha_mix, NbList nl, int skin,
                          int* __restrict__ rebuild, int* __restrict__ status, const int* __restrict__ blist = nullptr) {
   const int bid_ = blist ? blist[blockIdx.x] : (int)blockIdx.x;  // block of the packed layout
@@ -907,7 +907,7 @@ __device__ __forceinline__ int cell_of(const Replica& R, double x, double y, dou
 }
 
 // populate wrap (no image update) + cell index + count
-__global__ void k_rb_bin(const Replica* __restrict__ reps, const int* __restrict__ blk_rep,
+static __global__ void k_rb_bin(const Replica* __restrict__ reps, const int* __restrict__ blk_rep,
                          const int* __restrict__ rebuild, Dyn d, int* __restrict__ pcell,
                          int* __restrict__ cell_cnt, const int* __restrict__ blist = nullptr) {
   const int bid_ = blist ? blist[blockIdx.x] : (int)blockIdx.x;  // block of the packed layout
@@ -951,14 +951,14 @@ __device__ __forceinline__ int seg_cell(const CellSeg* __restrict__ segs, int ns
   return segs[lo].cell_off + (v - segs[lo].vbase);
 }
 
-__global__ void k_seg_zero(const CellSeg* __restrict__ segs, int nseg, int n, int* __restrict__ a, int* __restrict__ b) {
+static __global__ void k_seg_zero(const CellSeg* __restrict__ segs, int nseg, int n, int* __restrict__ a, int* __restrict__ b) {
   for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) {
     const int g = seg_cell(segs, nseg, v);
     a[g] = 0; b[g] = 0;
   }
 }
 
-__global__ void k_scan_a(const int* __restrict__ in, int n, const CellSeg* __restrict__ segs, int nseg,
+static __global__ void k_scan_a(const int* __restrict__ in, int n, const CellSeg* __restrict__ segs, int nseg,
                          int* __restrict__ bsum) {
   __shared__ int sh[SCAN_T / 32];
   const int base = blockIdx.x * SCAN_TILE;
@@ -1002,7 +1002,7 @@ __device__ __forceinline__ int block_excl_scan(int v, int* sh_warp, int& total) 
   return wp + x - v;
 }
 
-__global__ void k_scan_b(int* bsum, int nb) {
+static __global__ void k_scan_b(int* bsum, int nb) {
   __shared__ int shw[32];
   int carry = 0;
   for (int base = 0; base < nb; base += SCAN_T) {
@@ -1016,7 +1016,7 @@ __global__ void k_scan_b(int* bsum, int nb) {
   }
 }
 
-__global__ void k_scan_c(const int* __restrict__ in, int n, const CellSeg* __restrict__ segs, int nseg,
+static __global__ void k_scan_c(const int* __restrict__ in, int n, const CellSeg* __restrict__ segs, int nseg,
                          const int* __restrict__ bsum, int* __restrict__ out) {
   __shared__ int shw[32];
   const int base = blockIdx.x * SCAN_TILE;
@@ -1040,7 +1040,7 @@ __global__ void k_scan_c(const int* __restrict__ in, int n, const CellSeg* __res
 }
 
 // unordered placement into the cell segments
-__global__ void k_rb_scatter(const Replica* __restrict__ reps, const int* __restrict__ blk_rep,
+static __global__ void k_rb_scatter(const Replica* __restrict__ reps, const int* __restrict__ blk_rep,
                              const int* __restrict__ rebuild, const int* __restrict__ pcell,
                              const int* __restrict__ cstart, int* __restrict__ cfill, int* __restrict__ tmp, const int* __restrict__ blist = nullptr) {
   const int bid_ = blist ? blist[blockIdx.x] : (int)blockIdx.x;  // block of the packed layout
@@ -1061,7 +1061,7 @@ __global__ void k_rb_scatter(const Replica* __restrict__ reps, const int* __rest
 __device__ __forceinline__ double pack_id_slot(int id, int slot) {
   return __longlong_as_double((long long)(((unsigned long long)(unsigned)id << 32) | (unsigned)slot));
 }
-__global__ void k_rb_rank(const Replica* __restrict__ reps, const int* __restrict__ blk_rep,
+static __global__ void k_rb_rank(const Replica* __restrict__ reps, const int* __restrict__ blk_rep,
                           const int* __restrict__ rebuild, const int* __restrict__ pcell,
                           const int* __restrict__ cstart, const int* __restrict__ ccnt,
                           const int* __restrict__ tmp, const int* __restrict__ id, int* __restrict__ perm,
@@ -1084,7 +1084,7 @@ __global__ void k_rb_rank(const Replica* __restrict__ reps, const int* __restric
 }
 
 // gather all particle arrays into the permuted order (dst = src[perm])
-__global__ void k_rb_gather(const Replica* __restrict__ reps, const int* __restrict__ blk_rep,
+static __global__ void k_rb_gather(const Replica* __restrict__ reps, const int* __restrict__ blk_rep,
                             const int* __restrict__ rebuild, const int* __restrict__ perm,
                             Dyn src, Dyn dst, Stat ssrc, Stat sdst, const int* __restrict__ blist = nullptr) {
   const int bid_ = blist ? blist[blockIdx.x] : (int)blockIdx.x;  // block of the packed layout
@@ -1102,7 +1102,7 @@ __global__ void k_rb_gather(const Replica* __restrict__ reps, const int* __restr
 }
 
 // copy back (dst -> src) for the rebuilt replicas
-__global__ void k_rb_copyback(const Replica* __restrict__ reps, const int* __restrict__ blk_rep,
+static __global__ void k_rb_copyback(const Replica* __restrict__ reps, const int* __restrict__ blk_rep,
                               const int* __restrict__ rebuild, Dyn tmpd, Dyn d, Stat tmps, Stat st, const int* __restrict__ blist = nullptr) {
   const int bid_ = blist ? blist[blockIdx.x] : (int)blockIdx.x;  // block of the packed layout
   const int r = blk_rep[bid_];
@@ -1346,7 +1346,7 @@ __device__ __forceinline__ void build_particle_packed(const Replica& R, int k, D
   nl.ox[k] = x; nl.oy[k] = y; nl.oz[k] = z;
 }
 
-__global__ void k_rb_build(const Replica* __restrict__ reps, const int* __restrict__ blk_rep,
+static __global__ void k_rb_build(const Replica* __restrict__ reps, const int* __restrict__ blk_rep,
                            const int* __restrict__ rebuild, Dyn d, Stat st, NbList nl,
                            const D4* __restrict__ cand, const int* __restrict__ cstart,
                            const int* __restrict__ ccnt, int* __restrict__ status, int* __restrict__ maxnb, const int* __restrict__ blist = nullptr) {
@@ -1382,7 +1382,7 @@ constexpr int TEAM_PARTS = 32;  // particles per block of TEAM * TEAM_PARTS thre
 constexpr int TEAM_SUB = BLOCK / TEAM_PARTS;  // blocks per packed block
 constexpr int NB_TEAM = 16;     // finds staged per lane and side
 
-__global__ void __launch_bounds__(TEAM * TEAM_PARTS)
+static __global__ void __launch_bounds__(TEAM * TEAM_PARTS)
 k_rb_build_team(const Replica* __restrict__ reps, const int* __restrict__ blk_rep, const int* __restrict__ rebuild,
                 Dyn d, Stat st, NbList nl, const int* __restrict__ cslot, const int* __restrict__ cstart,
                 const int* __restrict__ ccnt, int* __restrict__ status, int* __restrict__ maxnb,
@@ -1488,7 +1488,7 @@ __host__ __device__ constexpr bool tile_eligible(int use_cell, int cnx, int cny,
   return use_cell && cnx >= 3 && cny >= 3 && cnz == TILE_CZ;
 }
 
-__global__ void __launch_bounds__(BLOCK)
+static __global__ void __launch_bounds__(BLOCK)
 k_rb_build_tile(const Replica* __restrict__ reps, const TileRef* __restrict__ tiles, const int* __restrict__ rebuild,
                 Dyn d, Stat st, NbList nl, const int* __restrict__ cslot, const int* __restrict__ cstart,
                 const int* __restrict__ ccnt, int* __restrict__ status, int* __restrict__ maxnb) {
