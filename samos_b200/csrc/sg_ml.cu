@@ -34,50 +34,158 @@ constexpr int NP_W1A = 0, NP_B1A = 256, NP_W1B = 320, NP_B1B = 4416, NP_WPQ = 44
 constexpr int EDGE_WARPS = 8;  // warps per block in the edge kernels
 constexpr int EDGE_BLOCKS = 148 * 8;
 
-__device__ __forceinline__ float bf(const __nv_bfloat16 v) { return __bfloat162float(v); }
+// ---- edge passes ---------------------------------------------------------------
+// A warp takes EDGE_P consecutive slots and EDGE_Q list entries of each at a
+// time.  First each lane works out the geometry of one entry (FP64 minimum
+// image, square root, quotients) and leaves it in shared memory; then the warp
+// walks every slot's edges in list order with one feature pair (f, f + 32) per
+// lane.  With the geometry inside the feature loop every lane repeated the FP64
+// of every edge, and the passes were bound by the FP64 pipe (64 packings of
+// 4,096 particles: 187, 412, 550 and 286 us for the four passes).  The
+// feature arithmetic is packed FP32 (fma.rn.f32x2): one instruction for the
+// pair, rounded as the two scalar ones.
+constexpr int EDGE_P = 4, EDGE_Q = 8;
 
-__device__ __forceinline__ bool edge_vec(const sg_view& V, const double* box, int i, int j, double rc, float* e,
-                                         float& ux, float& uy, float ai) {
-  const double Lx = box[2 * i], Ly = box[2 * i + 1];
-  double dx = V.x_device[j] - V.x_device[i], dy = V.y_device[j] - V.y_device[i];
-  if (dx > 0.5 * Lx) dx -= Lx; else if (dx < -0.5 * Lx) dx += Lx;
-  if (dy > 0.5 * Ly) dy -= Ly; else if (dy < -0.5 * Ly) dy += Ly;
-  const double r = sqrt(dx * dx + dy * dy);
-  if (!(r < rc) || r == 0.0) return false;
-  const float aj = (float)V.radius_device[j];
-  e[0] = (float)r; e[1] = ai; e[2] = aj; e[3] = ai + aj - (float)r;
-  ux = (float)(dx / r); uy = (float)(dy / r);
-  return true;
+typedef unsigned long long f2_t;  // two FP32 values: features f and f + 32
+__device__ __forceinline__ f2_t f2_pack(float lo, float hi) {
+  f2_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ float f2_lo(f2_t a) { return __uint_as_float((uint32_t)a); }
+__device__ __forceinline__ float f2_hi(f2_t a) { return __uint_as_float((uint32_t)(a >> 32)); }
+__device__ __forceinline__ f2_t f2_fma(f2_t a, f2_t b, f2_t c) {
+  f2_t d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+__device__ __forceinline__ f2_t f2_add(f2_t a, f2_t b) {
+  f2_t d;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ f2_t f2_mul(f2_t a, f2_t b) {
+  f2_t d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ f2_t f2_relu(f2_t a) { return f2_pack(fmaxf(f2_lo(a), 0.f), fmaxf(f2_hi(a), 0.f)); }
+
+// one warp's staged edges: features as packed pairs (e, e), the unit vector
+struct EdgeStage {
+  ulonglong2 e01[32], e23[32];
+  float2 u[32];
+};
+
+// a lane's slot in the group of EDGE_P slots from i0: its particle and entry
+struct EdgeLane {
+  int i, cnt;
+  double x, y, Lx, Ly;
+  float a;
+};
+__device__ __forceinline__ EdgeLane edge_lane(const sg_view& V, const double* __restrict__ box, int i0, int lane) {
+  EdgeLane L;
+  L.i = i0 + lane / EDGE_Q;
+  L.cnt = 0;
+  L.x = L.y = 0.0; L.a = 0.f; L.Lx = L.Ly = 0.0;
+  if (L.i < V.slots) {
+    L.Lx = box[2 * (size_t)L.i]; L.Ly = box[2 * (size_t)L.i + 1];
+    if (L.Lx > 0.0) {
+      L.cnt = V.nb_cnt_device[L.i];
+      L.x = V.x_device[L.i]; L.y = V.y_device[L.i];
+      L.a = (float)V.radius_device[L.i];
+    }
+  }
+  return L;
+}
+
+// Stages entry q of the lane's slot; returns the mask of the warp's entries
+// that are edges (r < rc), *j the lane's neighbour (its own slot without an edge).
+__device__ __forceinline__ unsigned stage_edge(const sg_view& V, const EdgeLane& L, int q, double rc, int lane,
+                                               EdgeStage& S, int* j_out, float2* u_out) {
+  bool edge = false;
+  int j = L.i;
+  float2 u = make_float2(0.f, 0.f);
+  if (q < L.cnt) {
+    j = V.nb_device[(size_t)q * V.nb_stride + L.i];
+    double dx = V.x_device[j] - L.x, dy = V.y_device[j] - L.y;
+    if (dx > 0.5 * L.Lx) dx -= L.Lx; else if (dx < -0.5 * L.Lx) dx += L.Lx;
+    if (dy > 0.5 * L.Ly) dy -= L.Ly; else if (dy < -0.5 * L.Ly) dy += L.Ly;
+    const double r = sqrt(dx * dx + dy * dy);
+    edge = r < rc && r != 0.0;
+    if (edge) {
+      const float aj = (float)V.radius_device[j], rf = (float)r, g = L.a + aj - rf;
+      u = make_float2((float)(dx / r), (float)(dy / r));
+      S.e01[lane] = make_ulonglong2(f2_pack(rf, rf), f2_pack(L.a, L.a));
+      S.e23[lane] = make_ulonglong2(f2_pack(aj, aj), f2_pack(g, g));
+    }
+  }
+  S.u[lane] = u;
+  *j_out = j;
+  *u_out = u;
+  return __ballot_sync(0xffffffffu, edge);
+}
+
+// feature pairs (lane, lane + 32) of a [64 x 4] weight and a [64] vector
+struct EdgeWeights { f2_t w[4], b; };
+__device__ __forceinline__ EdgeWeights edge_weights(const float* __restrict__ W, const float* __restrict__ b, int lane) {
+  EdgeWeights E;
+#pragma unroll
+  for (int d = 0; d < 4; d++) E.w[d] = f2_pack(W[4 * lane + d], W[4 * (lane + 32) + d]);
+  E.b = f2_pack(b[lane], b[lane + 32]);
+  return E;
+}
+// W e + b, starting from `z`
+__device__ __forceinline__ f2_t edge_affine(const EdgeWeights& E, const ulonglong2& e01, const ulonglong2& e23, f2_t z) {
+  z = f2_fma(E.w[0], e01.x, z);
+  z = f2_fma(E.w[1], e01.y, z);
+  z = f2_fma(E.w[2], e23.x, z);
+  z = f2_fma(E.w[3], e23.y, z);
+  return f2_add(z, E.b);
+}
+__device__ __forceinline__ f2_t edge_layer1(const EdgeWeights& E, const ulonglong2& e01, const ulonglong2& e23) {
+  f2_t z = f2_mul(E.w[0], e01.x);
+  z = f2_fma(E.w[1], e01.y, z);
+  z = f2_fma(E.w[2], e23.x, z);
+  z = f2_fma(E.w[3], e23.y, z);
+  return f2_add(z, E.b);
 }
 
 // ---- layer 1 edges: s_i = sum_j relu(W1a e + b1a), stored BF16 ----------------
-__global__ void k_ml_l1(sg_view V, const double* __restrict__ box, double rc, const float* __restrict__ P,
-                        __nv_bfloat16* __restrict__ s16) {
-  const int lane = threadIdx.x & 31;
-  const int nw = gridDim.x * (blockDim.x >> 5);
-  float w[2][4], b[2];
-  for (int h = 0; h < 2; h++) {
-    const int f = lane + 32 * h;
-    for (int d = 0; d < 4; d++) w[h][d] = P[NP_W1A + 4 * f + d];
-    b[h] = P[NP_B1A + f];
-  }
-  for (int i = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); i < V.slots; i += nw) {
-    float acc[2] = {0.f, 0.f};
-    if (box[2 * i] > 0.0) {
-      const float ai = (float)V.radius_device[i];
-      const int cnt = V.nb_cnt_device[i];
-      for (int q = 0; q < cnt; q++) {
-        const int j = V.nb_device[(size_t)q * V.nb_stride + i];
-        float e[4], ux, uy;
-        if (!edge_vec(V, box, i, j, rc, e, ux, uy, ai)) continue;
-        for (int h = 0; h < 2; h++) {
-          const float z = w[h][0] * e[0] + w[h][1] * e[1] + w[h][2] * e[2] + w[h][3] * e[3] + b[h];
-          acc[h] += fmaxf(z, 0.f);
+__global__ void __launch_bounds__(32 * EDGE_WARPS)
+k_ml_l1(sg_view V, const double* __restrict__ box, double rc, const float* __restrict__ P,
+        __nv_bfloat16* __restrict__ s16) {
+  __shared__ EdgeStage stage[EDGE_WARPS];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  EdgeStage& S = stage[warp];
+  const int nw = gridDim.x * EDGE_WARPS;
+  const EdgeWeights E = edge_weights(P + NP_W1A, P + NP_B1A, lane);
+  for (int i0 = (blockIdx.x * EDGE_WARPS + warp) * EDGE_P; i0 < V.slots; i0 += nw * EDGE_P) {
+    const EdgeLane L = edge_lane(V, box, i0, lane);
+    const int most = __reduce_max_sync(0xffffffffu, L.cnt);
+    f2_t acc[EDGE_P];
+#pragma unroll
+    for (int p = 0; p < EDGE_P; p++) acc[p] = 0ull;
+    for (int q0 = 0; q0 < most; q0 += EDGE_Q) {
+      int j;
+      float2 u;
+      const unsigned mask = stage_edge(V, L, q0 + lane % EDGE_Q, rc, lane, S, &j, &u);
+      __syncwarp();
+#pragma unroll
+      for (int p = 0; p < EDGE_P; p++) {
+        for (unsigned m = mask & (0xffu << (p * EDGE_Q)); m; m &= m - 1) {
+          const int q = __ffs(m) - 1;
+          acc[p] = f2_add(acc[p], f2_relu(edge_layer1(E, S.e01[q], S.e23[q])));
         }
       }
+      __syncwarp();
     }
-    s16[(size_t)i * F + lane] = __float2bfloat16_rn(acc[0]);
-    s16[(size_t)i * F + lane + 32] = __float2bfloat16_rn(acc[1]);
+#pragma unroll
+    for (int p = 0; p < EDGE_P; p++)
+      if (i0 + p < V.slots) {
+        s16[(size_t)(i0 + p) * F + lane] = __float2bfloat16_rn(f2_lo(acc[p]));
+        s16[(size_t)(i0 + p) * F + lane + 32] = __float2bfloat16_rn(f2_hi(acc[p]));
+      }
   }
 }
 
@@ -313,7 +421,7 @@ template <int K, int N>
 __global__ void __launch_bounds__(128)
 k_ml_gemm_tc(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, int M,
              const float* __restrict__ bias, int relu, const double* __restrict__ box, float* __restrict__ C32,
-             __nv_bfloat16* __restrict__ C16, int* __restrict__ err) {
+             __nv_bfloat16* __restrict__ C16, const __nv_bfloat16* __restrict__ act, int* __restrict__ err) {
   static_assert((K == 64 || K == 128) && (N == 64 || N == 128), "K, N in {64, 128}");
   constexpr int KG = K / 64;                      // 128-B K groups
   constexpr int A_GROUP = 128 * 128, B_GROUP = N * 128;
@@ -404,6 +512,16 @@ k_ml_gemm_tc(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
       if (relu) t = fmaxf(t, 0.f);
       v[j] = valid ? t : 0.f;
     }
+    if (act) {  // backward through a relu: pass where its output was positive
+      const uint4* a = reinterpret_cast<const uint4*>(act + (size_t)row * N + q * 16);
+      const uint4 a0 = a[0], a1 = a[1];
+      const uint32_t w[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
+#pragma unroll
+      for (int j = 0; j < 16; j++) {
+        const uint32_t h = j & 1 ? w[j / 2] & 0xffff0000u : w[j / 2] << 16;
+        if (!(__uint_as_float(h) > 0.f)) v[j] = 0.f;
+      }
+    }
     if (C32) {
       float4* o = reinterpret_cast<float4*>(C32 + (size_t)row * N + q * 16);
 #pragma unroll
@@ -426,7 +544,7 @@ k_ml_gemm_tc(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CU
 
 template <int K, int N>
 int launch_gemm_tc(const void* A, const void* Bt, int M, const float* bias, int relu, const double* box, float* C32,
-                   void* C16, int* err, cudaStream_t st) {
+                   void* C16, const void* act, int* err, cudaStream_t st) {
   // at most 512 / N CTAs may share an SM's 512 tensor-memory columns: the
   // shared-memory request is padded so that no more fit (an allocation
   // beyond them would wait for another CTA's release)
@@ -441,117 +559,220 @@ int launch_gemm_tc(const void* A, const void* Bt, int M, const float* bias, int 
       return SG_ERR_CUDA;
     attr = true;
   }
-  k_ml_gemm_tc<K, N><<<(M + 127) / 128, 128, SMEM, st>>>(ma, mb, M, bias, relu, box, C32, (__nv_bfloat16*)C16, err);
+  k_ml_gemm_tc<K, N><<<(M + 127) / 128, 128, SMEM, st>>>(ma, mb, M, bias, relu, box, C32, (__nv_bfloat16*)C16,
+                                                               (const __nv_bfloat16*)act, err);
   return cudaGetLastError() == cudaSuccess ? SG_OK : SG_ERR_CUDA;
 }
 
-// out[i] += sum_b partial[b][i]   (fixed order)
-__global__ void k_ml_reduce(const float* __restrict__ partial, int nblk, int len, float* __restrict__ out) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= len) return;
+// out[i] += sum_b partial[b][i], in a fixed order: RED_Y threads sum strided
+// subsets of the partials of one output, then their sums in order.  (One thread
+// per output walked all partials in turn: 115 us for the five sums of a
+// training step, bound by the chain of loads.)
+constexpr int RED_X = 32, RED_Y = 32;
+__global__ void __launch_bounds__(RED_X * RED_Y)
+k_ml_reduce(const float* __restrict__ partial, int nblk, int len, float* __restrict__ out) {
+  __shared__ float sh[RED_Y][RED_X];
+  const int i = blockIdx.x * RED_X + threadIdx.x;
   float s = 0.f;
-  for (int b = 0; b < nblk; b++) s += partial[(size_t)b * len + i];
-  out[i] += s;
+  if (i < len)
+#pragma unroll 4
+    for (int b = threadIdx.y; b < nblk; b += RED_Y) s += partial[(size_t)b * len + i];
+  sh[threadIdx.y][threadIdx.x] = s;
+  __syncthreads();
+  if (threadIdx.y == 0 && i < len) {
+    float t = 0.f;
+    for (int y = 0; y < RED_Y; y++) t += sh[y][threadIdx.x];
+    out[i] += t;
+  }
+}
+static void reduce_into(const float* partial, int nblk, int len, float* out, cudaStream_t st) {
+  k_ml_reduce<<<(len + RED_X - 1) / RED_X, dim3(RED_X, RED_Y), 0, st>>>(partial, nblk, len, out);
 }
 
 // ---- layer 2 edges (forward): disp_i --------------------------------------------
-__global__ void k_ml_l2(sg_view V, const double* __restrict__ box, double rc, const float* __restrict__ P,
-                        const float* __restrict__ PQ, float* __restrict__ disp) {
-  const int lane = threadIdx.x & 31;
-  const int nw = gridDim.x * (blockDim.x >> 5);
-  float we[2][4], b2[2], w2[2];
-  for (int h = 0; h < 2; h++) {
-    const int f = lane + 32 * h;
-    for (int d = 0; d < 4; d++) we[h][d] = P[NP_W2E + 4 * f + d];
-    b2[h] = P[NP_B2 + f];
-    w2[h] = P[NP_W2 + f];
-  }
-  const float c = P[NP_C];
-  for (int i = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); i < V.slots; i += nw) {
-    float dx = 0.f, dy = 0.f;
-    if (box[2 * i] > 0.0) {
-      const float ai = (float)V.radius_device[i];
-      const float Pi0 = PQ[(size_t)i * 2 * F + lane], Pi1 = PQ[(size_t)i * 2 * F + lane + 32];
-      const int cnt = V.nb_cnt_device[i];
-      for (int q = 0; q < cnt; q++) {
-        const int j = V.nb_device[(size_t)q * V.nb_stride + i];
-        float e[4], ux, uy;
-        if (!edge_vec(V, box, i, j, rc, e, ux, uy, ai)) continue;
-        const float Qj0 = PQ[(size_t)j * 2 * F + F + lane], Qj1 = PQ[(size_t)j * 2 * F + F + lane + 32];
-        const float z0 = Pi0 + Qj0 + we[0][0] * e[0] + we[0][1] * e[1] + we[0][2] * e[2] + we[0][3] * e[3] + b2[0];
-        const float z1 = Pi1 + Qj1 + we[1][0] * e[0] + we[1][1] * e[1] + we[1][2] * e[2] + we[1][3] * e[3] + b2[1];
-        float part = fmaxf(z0, 0.f) * w2[0] + fmaxf(z1, 0.f) * w2[1];
-        for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
-        const float w = part + c;
-        dx += w * ux; dy += w * uy;
+// The 64-wide dot products of a slot's EDGE_Q edges are summed over the lanes
+// together: at offsets 16, 8 and 4 a lane passes on half of its edges' sums and
+// keeps the other half (7 + 2 shuffles for 8 edges instead of 40, the same
+// pairs added in the same order as in one sum after the other).
+__global__ void __launch_bounds__(32 * EDGE_WARPS)
+k_ml_l2(sg_view V, const double* __restrict__ box, double rc, const float* __restrict__ P,
+        const float* __restrict__ PQ, float* __restrict__ disp) {
+  __shared__ EdgeStage stage[EDGE_WARPS];
+  __shared__ float wsh[EDGE_WARPS][32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  EdgeStage& S = stage[warp];
+  const int nw = gridDim.x * EDGE_WARPS;
+  const EdgeWeights E = edge_weights(P + NP_W2E, P + NP_B2, lane);
+  const float w2a = P[NP_W2 + lane], w2b = P[NP_W2 + lane + 32], c = P[NP_C];
+  for (int i0 = (blockIdx.x * EDGE_WARPS + warp) * EDGE_P; i0 < V.slots; i0 += nw * EDGE_P) {
+    const EdgeLane L = edge_lane(V, box, i0, lane);
+    const int most = __reduce_max_sync(0xffffffffu, L.cnt);
+    float dx = 0.f, dy = 0.f;  // lane p < EDGE_P: slot i0 + p
+    for (int q0 = 0; q0 < most; q0 += EDGE_Q) {
+      int j;
+      float2 u;
+      const unsigned mask = stage_edge(V, L, q0 + lane % EDGE_Q, rc, lane, S, &j, &u);
+      __syncwarp();
+#pragma unroll
+      for (int p = 0; p < EDGE_P; p++) {
+        const unsigned m = (mask >> (p * EDGE_Q)) & 0xffu;
+        if (!m) continue;
+        const float* Pi = PQ + (size_t)(i0 + p) * 2 * F;
+        const f2_t pi = f2_pack(Pi[lane], Pi[lane + 32]);
+        f2_t qj[EDGE_Q];
+#pragma unroll
+        for (int q = 0; q < EDGE_Q; q++) {
+          const int jq = __shfl_sync(0xffffffffu, j, p * EDGE_Q + q);
+          if (m >> q & 1) {
+            const float* Qj = PQ + (size_t)jq * 2 * F + F;
+            qj[q] = f2_pack(Qj[lane], Qj[lane + 32]);
+          }
+        }
+        float part[EDGE_Q];
+#pragma unroll
+        for (int q = 0; q < EDGE_Q; q++) {
+          part[q] = 0.f;
+          if (m >> q & 1) {
+            const f2_t z = edge_affine(E, S.e01[p * EDGE_Q + q], S.e23[p * EDGE_Q + q], f2_add(pi, qj[q]));
+            part[q] = fmaf(fmaxf(f2_hi(z), 0.f), w2b, fmaxf(f2_lo(z), 0.f) * w2a);
+          }
+        }
+        static_assert(EDGE_Q == 8, "three halving steps");
+#pragma unroll
+        for (int h = 4, o = 16; h > 0; h >>= 1, o >>= 1) {
+          const bool up = lane & o;
+#pragma unroll
+          for (int q = 0; q < h; q++) {
+            const float give = up ? part[q] : part[q + h], keep = up ? part[q + h] : part[q];
+            part[q] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+          }
+        }
+        part[0] += __shfl_xor_sync(0xffffffffu, part[0], 2);
+        part[0] += __shfl_xor_sync(0xffffffffu, part[0], 1);
+        if ((lane & 3) == 0) wsh[warp][p * EDGE_Q + (lane >> 2)] = part[0] + c;
       }
+      __syncwarp();
+      if (lane < EDGE_P)
+        for (unsigned m = mask & (0xffu << (lane * EDGE_Q)); m; m &= m - 1) {
+          const int q = __ffs(m) - 1;
+          dx = fmaf(wsh[warp][q], S.u[q].x, dx);
+          dy = fmaf(wsh[warp][q], S.u[q].y, dy);
+        }
+      __syncwarp();
     }
-    if (lane == 0) { disp[2 * i] = dx; disp[2 * i + 1] = dy; }
+    if (lane < EDGE_P && i0 + lane < V.slots)
+      reinterpret_cast<float2*>(disp)[i0 + lane] = make_float2(dx, dy);
   }
 }
 
 // ---- layer 2 edges (backward) -------------------------------------------------
-// gPQ must be zero on entry: the P half of row i is written by i's warp, the Q
-// half of row j receives atomic contributions from every i that has j as a
-// neighbour.  Per-block partials of (gW2e, gb2, gw2, gc) go to part[block].
-constexpr int L2_GRAD = 256 + 64 + 64 + 1;  // W2e, b2, w2, c
-__global__ void k_ml_l2_bwd(sg_view V, const double* __restrict__ box, double rc, const float* __restrict__ P,
-                            const float* __restrict__ PQ, const float* __restrict__ disp,
-                            const float* __restrict__ target, float inv_n, float* __restrict__ gPQ,
-                            float* __restrict__ part, float* __restrict__ loss_part) {
+// Row i of gPQ is written whole by i's warp, in BF16 as the GEMMs take it: the
+// lists are full, so beside edge (i, j), whose gz_ij goes to P_i and the weight
+// gradients, the warp works out edge (j, i), whose gz_ji goes to Q_i, from row
+// j.  That costs another 256-byte row per edge and replaces the atomic adds
+// into row j, the zeroing of gPQ in FP32 and its conversion (550 + 99 + 20 us).
+// Per-block partials of (gb2, gW2e, gw2, gc), in parameter order, go to
+// part[block].
+constexpr int L2_GRAD = 64 + 256 + 64 + 1;  // b2, W2e, w2, c: as from NP_B2 on
+__global__ void __launch_bounds__(32 * EDGE_WARPS)
+k_ml_l2_bwd(sg_view V, const double* __restrict__ box, double rc, const float* __restrict__ P,
+            const float* __restrict__ PQ, const float* __restrict__ disp, const float* __restrict__ target, float inv_n,
+            __nv_bfloat16* __restrict__ gPQ16, float* __restrict__ part, float* __restrict__ loss_part) {
+  __shared__ EdgeStage stage[EDGE_WARPS];
+  __shared__ float2 gsh[EDGE_WARPS][32];  // d loss / d w of edges (i, j) and (j, i)
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int nw = gridDim.x * (blockDim.x >> 5);
-  float we[2][4], b2[2], w2[2];
-  for (int h = 0; h < 2; h++) {
-    const int f = lane + 32 * h;
-    for (int d = 0; d < 4; d++) we[h][d] = P[NP_W2E + 4 * f + d];
-    b2[h] = P[NP_B2 + f];
-    w2[h] = P[NP_W2 + f];
-  }
-  float gWe[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}}, gb2[2] = {0.f, 0.f}, gw2[2] = {0.f, 0.f};
+  EdgeStage& S = stage[warp];
+  const int nw = gridDim.x * EDGE_WARPS;
+  const EdgeWeights E = edge_weights(P + NP_W2E, P + NP_B2, lane);
+  const f2_t w2 = f2_pack(P[NP_W2 + lane], P[NP_W2 + lane + 32]);
+  f2_t gWe[4] = {0ull, 0ull, 0ull, 0ull}, gb2 = 0ull, gw2 = 0ull;
   float gc = 0.f, lsum = 0.f;
-  for (int i = blockIdx.x * (blockDim.x >> 5) + warp; i < V.slots; i += nw) {
-    if (!(box[2 * i] > 0.0)) continue;
-    const float ddx = disp[2 * i] - target[2 * i], ddy = disp[2 * i + 1] - target[2 * i + 1];
-    if (lane == 0) lsum += ddx * ddx + ddy * ddy;
-    const float gdx = 2.f * ddx * inv_n, gdy = 2.f * ddy * inv_n;
-    const float ai = (float)V.radius_device[i];
-    const float Pi0 = PQ[(size_t)i * 2 * F + lane], Pi1 = PQ[(size_t)i * 2 * F + lane + 32];
-    float gP0 = 0.f, gP1 = 0.f;
-    const int cnt = V.nb_cnt_device[i];
-    for (int q = 0; q < cnt; q++) {
-      const int j = V.nb_device[(size_t)q * V.nb_stride + i];
-      float e[4], ux, uy;
-      if (!edge_vec(V, box, i, j, rc, e, ux, uy, ai)) continue;
-      const float Qj0 = PQ[(size_t)j * 2 * F + F + lane], Qj1 = PQ[(size_t)j * 2 * F + F + lane + 32];
-      const float z0 = Pi0 + Qj0 + we[0][0] * e[0] + we[0][1] * e[1] + we[0][2] * e[2] + we[0][3] * e[3] + b2[0];
-      const float z1 = Pi1 + Qj1 + we[1][0] * e[0] + we[1][1] * e[1] + we[1][2] * e[2] + we[1][3] * e[3] + b2[1];
-      const float a0 = fmaxf(z0, 0.f), a1 = fmaxf(z1, 0.f);
-      const float gw = gdx * ux + gdy * uy;  // d loss / d w_ij
-      gw2[0] += gw * a0; gw2[1] += gw * a1;
-      if (lane == 0) gc += gw;
-      const float gz0 = z0 > 0.f ? gw * w2[0] : 0.f, gz1 = z1 > 0.f ? gw * w2[1] : 0.f;
-      gb2[0] += gz0; gb2[1] += gz1;
-      for (int d = 0; d < 4; d++) { gWe[0][d] += gz0 * e[d]; gWe[1][d] += gz1 * e[d]; }
-      gP0 += gz0; gP1 += gz1;
-      atomicAdd(&gPQ[(size_t)j * 2 * F + F + lane], gz0);
-      atomicAdd(&gPQ[(size_t)j * 2 * F + F + lane + 32], gz1);
+  for (int i0 = (blockIdx.x * EDGE_WARPS + warp) * EDGE_P; i0 < V.slots; i0 += nw * EDGE_P) {
+    const EdgeLane L = edge_lane(V, box, i0, lane);
+    const int most = __reduce_max_sync(0xffffffffu, L.cnt);
+    float gdx = 0.f, gdy = 0.f;
+    if (L.Lx > 0.0) {
+      const float2 d = reinterpret_cast<const float2*>(disp)[L.i], t = reinterpret_cast<const float2*>(target)[L.i];
+      const float ex = d.x - t.x, ey = d.y - t.y;
+      if (lane % EDGE_Q == 0) lsum += ex * ex + ey * ey;
+      gdx = 2.f * ex * inv_n; gdy = 2.f * ey * inv_n;
     }
-    gPQ[(size_t)i * 2 * F + lane] = gP0;
-    gPQ[(size_t)i * 2 * F + lane + 32] = gP1;
+    f2_t gP[EDGE_P], gQ[EDGE_P];
+#pragma unroll
+    for (int p = 0; p < EDGE_P; p++) gP[p] = gQ[p] = 0ull;
+    for (int q0 = 0; q0 < most; q0 += EDGE_Q) {
+      int j;
+      float2 u;
+      const unsigned mask = stage_edge(V, L, q0 + lane % EDGE_Q, rc, lane, S, &j, &u);
+      if (mask >> lane & 1) {
+        const float2 d = reinterpret_cast<const float2*>(disp)[j], t = reinterpret_cast<const float2*>(target)[j];
+        const float gw = gdx * u.x + gdy * u.y;
+        // the vector from j to i is exactly the opposite
+        const float gr = -(2.f * (d.x - t.x) * inv_n * u.x + 2.f * (d.y - t.y) * inv_n * u.y);
+        gsh[warp][lane] = make_float2(gw, gr);
+        gc += gw;
+      }
+      __syncwarp();
+#pragma unroll
+      for (int p = 0; p < EDGE_P; p++) {
+        const unsigned m = (mask >> (p * EDGE_Q)) & 0xffu;
+        if (!m) continue;
+        const float* Ri = PQ + (size_t)(i0 + p) * 2 * F;
+        const f2_t pi = f2_pack(Ri[lane], Ri[lane + 32]), qi = f2_pack(Ri[F + lane], Ri[F + lane + 32]);
+#pragma unroll
+        for (int q = 0; q < EDGE_Q; q++) {
+          const int t = p * EDGE_Q + q;
+          const int jq = __shfl_sync(0xffffffffu, j, t);
+          if (m >> q & 1) {
+            const float* Rj = PQ + (size_t)jq * 2 * F;
+            const f2_t pj = f2_pack(Rj[lane], Rj[lane + 32]), qj = f2_pack(Rj[F + lane], Rj[F + lane + 32]);
+            const ulonglong2 e01 = S.e01[t], e23 = S.e23[t];
+            const float2 g = gsh[warp][t];
+            const f2_t gw = f2_pack(g.x, g.x), gr = f2_pack(g.y, g.y);
+            const f2_t z = edge_affine(E, e01, e23, f2_add(pi, qj));
+            // edge (j, i): the two radii change places
+            const f2_t y = edge_affine(E, make_ulonglong2(e01.x, e23.x), make_ulonglong2(e01.y, e23.y), f2_add(pj, qi));
+            const f2_t fz = f2_mul(gw, w2), fy = f2_mul(gr, w2);
+            const f2_t gz = f2_pack(f2_lo(z) > 0.f ? f2_lo(fz) : 0.f, f2_hi(z) > 0.f ? f2_hi(fz) : 0.f);
+            const f2_t gy = f2_pack(f2_lo(y) > 0.f ? f2_lo(fy) : 0.f, f2_hi(y) > 0.f ? f2_hi(fy) : 0.f);
+            gw2 = f2_fma(gw, f2_relu(z), gw2);
+            gWe[0] = f2_fma(gz, e01.x, gWe[0]);
+            gWe[2] = f2_fma(gz, e23.x, gWe[2]);
+            gWe[3] = f2_fma(gz, e23.y, gWe[3]);
+            gP[p] = f2_add(gP[p], gz);
+            gQ[p] = f2_add(gQ[p], gy);
+          }
+        }
+      }
+      __syncwarp();
+    }
+#pragma unroll
+    for (int p = 0; p < EDGE_P; p++) {
+      const float ai = __shfl_sync(0xffffffffu, L.a, p * EDGE_Q);
+      gWe[1] = f2_fma(gP[p], f2_pack(ai, ai), gWe[1]);  // its own radius: the same for all of a slot's edges
+      gb2 = f2_add(gb2, gP[p]);
+      if (i0 + p < V.slots) {
+        __nv_bfloat16* R = gPQ16 + (size_t)(i0 + p) * 2 * F;  // padding slots: zeros
+        R[lane] = __float2bfloat16_rn(f2_lo(gP[p])); R[lane + 32] = __float2bfloat16_rn(f2_hi(gP[p]));
+        R[F + lane] = __float2bfloat16_rn(f2_lo(gQ[p])); R[F + lane + 32] = __float2bfloat16_rn(f2_hi(gQ[p]));
+      }
+    }
   }
   // block reduction of the weight-gradient partials (fixed order over warps)
   __shared__ float sp[EDGE_WARPS][L2_GRAD];
-  for (int h = 0; h < 2; h++) {
-    const int f = lane + 32 * h;
-    for (int d = 0; d < 4; d++) sp[warp][4 * f + d] = gWe[h][d];
-    sp[warp][256 + f] = gb2[h];
-    sp[warp][320 + f] = gw2[h];
+#pragma unroll
+  for (int d = 0; d < 4; d++) {
+    sp[warp][64 + 4 * lane + d] = f2_lo(gWe[d]);
+    sp[warp][64 + 4 * (lane + 32) + d] = f2_hi(gWe[d]);
   }
-  for (int o = 16; o > 0; o >>= 1) lsum += __shfl_xor_sync(0xffffffffu, lsum, o);
-  if (lane == 0) sp[warp][384] = gc;
+  sp[warp][lane] = f2_lo(gb2); sp[warp][lane + 32] = f2_hi(gb2);
+  sp[warp][320 + lane] = f2_lo(gw2); sp[warp][320 + lane + 32] = f2_hi(gw2);
+  for (int o = 16; o > 0; o >>= 1) {
+    lsum += __shfl_xor_sync(0xffffffffu, lsum, o);
+    gc += __shfl_xor_sync(0xffffffffu, gc, o);
+  }
   __shared__ float sl[EDGE_WARPS];
-  if (lane == 0) sl[warp] = lsum;
+  if (lane == 0) { sp[warp][384] = gc; sl[warp] = lsum; }
   __syncthreads();
   for (int idx = threadIdx.x; idx < L2_GRAD; idx += blockDim.x) {
     float s = 0.f;
@@ -565,77 +786,102 @@ __global__ void k_ml_l2_bwd(sg_view V, const double* __restrict__ box, double rc
   }
 }
 
-// gpre = gh * (h > 0) (BF16) and per-block column partials of gpre (gb1b)
-__global__ void k_ml_relu_bwd(int M, const float* __restrict__ gh, const __nv_bfloat16* __restrict__ h16,
-                              __nv_bfloat16* __restrict__ gpre16, float* __restrict__ part) {
-  const int f = threadIdx.x & 63, rsub = threadIdx.x >> 6;  // 256 threads: 4 rows per pass
-  float acc = 0.f;
+// per-block column partials of a BF16 [M x 64] array (gb1b of gpre): a thread
+// takes 8 columns (16 bytes) of every 32nd row of its block's run
+constexpr int COLSUM_BLOCKS = 148 * 4;
+__global__ void __launch_bounds__(256)
+k_ml_colsum(int M, const __nv_bfloat16* __restrict__ a, float* __restrict__ part) {
+  const int c8 = threadIdx.x & 7, rsub = threadIdx.x >> 3;
+  float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
   const int rows_per_block = (M + gridDim.x - 1) / gridDim.x;
   const int m0 = blockIdx.x * rows_per_block, m1 = min(M, m0 + rows_per_block);
-  for (int m = m0 + rsub; m < m1; m += 4) {
-    const float g = bf(h16[(size_t)m * F + f]) > 0.f ? gh[(size_t)m * F + f] : 0.f;
-    const __nv_bfloat16 gb = __float2bfloat16_rn(g);
-    gpre16[(size_t)m * F + f] = gb;
-    acc += bf(gb);
+#pragma unroll 4
+  for (int m = m0 + rsub; m < m1; m += 32) {
+    const uint4 v = *reinterpret_cast<const uint4*>(a + (size_t)m * F + c8 * 8);
+    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      acc[2 * k] += __uint_as_float(w[k] << 16);
+      acc[2 * k + 1] += __uint_as_float(w[k] & 0xffff0000u);
+    }
   }
-  __shared__ float s[4][64];
-  s[rsub][f] = acc;
+  __shared__ float s[32][F + 1];
+#pragma unroll
+  for (int k = 0; k < 8; k++) s[rsub][c8 * 8 + k] = acc[k];
   __syncthreads();
-  if (threadIdx.x < 64) part[(size_t)blockIdx.x * 64 + threadIdx.x] = s[0][f] + s[1][f] + s[2][f] + s[3][f];
+  if (threadIdx.x < F) {
+    float t = 0.f;
+    for (int y = 0; y < 32; y++) t += s[y][threadIdx.x];
+    part[(size_t)blockIdx.x * F + threadIdx.x] = t;
+  }
 }
 
-// ---- layer 1 edges (backward): gW1a, gb1a partials ------------------------------
+// ---- layer 1 edges (backward): gW1a, gb1a partials, in parameter order -----------
+// The gradient gs_i of s_i is the same for all edges of slot i, so a slot first
+// sums the features of its active edges (z > 0) and multiplies by gs_i once.
 constexpr int L1_GRAD = 256 + 64;
-__global__ void k_ml_l1_bwd(sg_view V, const double* __restrict__ box, double rc, const float* __restrict__ P,
-                            const float* __restrict__ gs, float* __restrict__ part) {
+__global__ void __launch_bounds__(32 * EDGE_WARPS)
+k_ml_l1_bwd(sg_view V, const double* __restrict__ box, double rc, const float* __restrict__ P,
+            const float* __restrict__ gs, float* __restrict__ part) {
+  __shared__ EdgeStage stage[EDGE_WARPS];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int nw = gridDim.x * (blockDim.x >> 5);
-  float w[2][4], b[2];
-  for (int h = 0; h < 2; h++) {
-    const int f = lane + 32 * h;
-    for (int d = 0; d < 4; d++) w[h][d] = P[NP_W1A + 4 * f + d];
-    b[h] = P[NP_B1A + f];
-  }
-  float gW[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}}, gb[2] = {0.f, 0.f};
-  for (int i = blockIdx.x * (blockDim.x >> 5) + warp; i < V.slots; i += nw) {
-    if (!(box[2 * i] > 0.0)) continue;
-    const float ai = (float)V.radius_device[i];
-    const float gs0 = gs[(size_t)i * F + lane], gs1 = gs[(size_t)i * F + lane + 32];
-    const int cnt = V.nb_cnt_device[i];
-    for (int q = 0; q < cnt; q++) {
-      const int j = V.nb_device[(size_t)q * V.nb_stride + i];
-      float e[4], ux, uy;
-      if (!edge_vec(V, box, i, j, rc, e, ux, uy, ai)) continue;
-      const float z0 = w[0][0] * e[0] + w[0][1] * e[1] + w[0][2] * e[2] + w[0][3] * e[3] + b[0];
-      const float z1 = w[1][0] * e[0] + w[1][1] * e[1] + w[1][2] * e[2] + w[1][3] * e[3] + b[1];
-      const float g0 = z0 > 0.f ? gs0 : 0.f, g1 = z1 > 0.f ? gs1 : 0.f;
-      gb[0] += g0; gb[1] += g1;
-      for (int d = 0; d < 4; d++) { gW[0][d] += g0 * e[d]; gW[1][d] += g1 * e[d]; }
+  EdgeStage& S = stage[warp];
+  const int nw = gridDim.x * EDGE_WARPS;
+  const EdgeWeights E = edge_weights(P + NP_W1A, P + NP_B1A, lane);
+  f2_t gW[4] = {0ull, 0ull, 0ull, 0ull}, gb = 0ull;
+  for (int i0 = (blockIdx.x * EDGE_WARPS + warp) * EDGE_P; i0 < V.slots; i0 += nw * EDGE_P) {
+    const EdgeLane L = edge_lane(V, box, i0, lane);
+    const int most = __reduce_max_sync(0xffffffffu, L.cnt);
+    f2_t s0[EDGE_P], s2[EDGE_P], s3[EDGE_P], sn[EDGE_P], g[EDGE_P];
+#pragma unroll
+    for (int p = 0; p < EDGE_P; p++) {
+      s0[p] = s2[p] = s3[p] = sn[p] = 0ull;
+      const size_t row = (size_t)min(i0 + p, V.slots - 1) * F;
+      g[p] = f2_pack(gs[row + lane], gs[row + lane + 32]);
+    }
+    for (int q0 = 0; q0 < most; q0 += EDGE_Q) {
+      int j;
+      float2 u;
+      const unsigned mask = stage_edge(V, L, q0 + lane % EDGE_Q, rc, lane, S, &j, &u);
+      __syncwarp();
+#pragma unroll
+      for (int p = 0; p < EDGE_P; p++)
+        for (unsigned m = mask & (0xffu << (p * EDGE_Q)); m; m &= m - 1) {
+          const int q = __ffs(m) - 1;
+          const ulonglong2 e01 = S.e01[q], e23 = S.e23[q];
+          const f2_t z = edge_layer1(E, e01, e23);
+          const f2_t on = f2_pack(f2_lo(z) > 0.f ? 1.f : 0.f, f2_hi(z) > 0.f ? 1.f : 0.f);
+          s0[p] = f2_fma(on, e01.x, s0[p]);
+          s2[p] = f2_fma(on, e23.x, s2[p]);
+          s3[p] = f2_fma(on, e23.y, s3[p]);
+          sn[p] = f2_add(sn[p], on);
+        }
+      __syncwarp();
+    }
+#pragma unroll
+    for (int p = 0; p < EDGE_P; p++) {
+      const float ai = __shfl_sync(0xffffffffu, L.a, p * EDGE_Q);
+      const f2_t gn = f2_mul(g[p], sn[p]);  // slots without edges: zero
+      gW[0] = f2_fma(g[p], s0[p], gW[0]);
+      gW[1] = f2_fma(gn, f2_pack(ai, ai), gW[1]);
+      gW[2] = f2_fma(g[p], s2[p], gW[2]);
+      gW[3] = f2_fma(g[p], s3[p], gW[3]);
+      gb = f2_add(gb, gn);
     }
   }
   __shared__ float sp[EDGE_WARPS][L1_GRAD];
-  for (int h = 0; h < 2; h++) {
-    const int f = lane + 32 * h;
-    for (int d = 0; d < 4; d++) sp[warp][4 * f + d] = gW[h][d];
-    sp[warp][256 + f] = gb[h];
+#pragma unroll
+  for (int d = 0; d < 4; d++) {
+    sp[warp][4 * lane + d] = f2_lo(gW[d]);
+    sp[warp][4 * (lane + 32) + d] = f2_hi(gW[d]);
   }
+  sp[warp][256 + lane] = f2_lo(gb); sp[warp][256 + lane + 32] = f2_hi(gb);
   __syncthreads();
   for (int idx = threadIdx.x; idx < L1_GRAD; idx += blockDim.x) {
     float s = 0.f;
     for (int ww = 0; ww < EDGE_WARPS; ww++) s += sp[ww][idx];
     part[(size_t)blockIdx.x * L1_GRAD + idx] = s;
   }
-}
-
-// add the reduced small-gradient vectors into the flat gradient buffer
-__global__ void k_ml_place(const float* __restrict__ src, int len, float* __restrict__ dst, int off_d) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < len) dst[off_d + i] += src[i];
-}
-
-__global__ void k_ml_to_bf16(const float* __restrict__ a, __nv_bfloat16* __restrict__ b, size_t n) {
-  const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) b[i] = __float2bfloat16_rn(a[i]);
 }
 
 __global__ void k_ml_adam(float* __restrict__ p, const float* __restrict__ g, float* __restrict__ m,
@@ -691,9 +937,9 @@ int sg_mlp_forward(const sg_view* V, const double* box, double rc, const float* 
   int* gerr = nullptr;
   if (cudaGetSymbolAddress((void**)&gerr, g_ml_tc_err) != cudaSuccess) return SG_ERR_CUDA;
   cudaMemsetAsync(gerr, 0, sizeof(int), st);
-  int grc = launch_gemm_tc<F, F>(s16, W1bT16, M, params + NP_B1B, 1, box, nullptr, h16, gerr, st);
+  int grc = launch_gemm_tc<F, F>(s16, W1bT16, M, params + NP_B1B, 1, box, nullptr, h16, nullptr, gerr, st);
   if (grc) return grc;
-  grc = launch_gemm_tc<F, 2 * F>(h16, WpqT16, M, nullptr, 0, box, PQ, nullptr, gerr, st);
+  grc = launch_gemm_tc<F, 2 * F>(h16, WpqT16, M, nullptr, 0, box, PQ, nullptr, nullptr, gerr, st);
   if (grc) return grc;
   k_ml_l2<<<EDGE_BLOCKS, 32 * EDGE_WARPS, 0, st>>>(*V, box, rc, params, PQ, disp);
   if (cudaGetLastError() != cudaSuccess) return SG_ERR_CUDA;
@@ -704,10 +950,9 @@ int sg_mlp_forward(const sg_view* V, const double* box, double rc, const float* 
   return timed_out ? SG_ERR_TIMEOUT : SG_OK;
 }
 
-// Gradients are ADDED to grad[NP_TOTAL] (zero it first).  work: gPQ [M x 128]
-// fp32, gPQ16 [M x 128] bf16, gh [M x 64] fp32, gpre16 [M x 64] bf16, gs
-// [M x 64] fp32, part >= sg_mlp_part_floats() floats, red >= 512 floats,
-// loss_part >= sg_mlp_edge_blocks() floats (per-block partial sums of
+// Gradients are ADDED to grad[NP_TOTAL] (zero it first).  work: gPQ16 [M x 128]
+// bf16, gpre16 [M x 64] bf16, gs [M x 64] fp32, part >= sg_mlp_part_floats()
+// floats (gPQ, gh and red are not used), loss_part >= sg_mlp_edge_blocks() floats (per-block partial sums of
 // |disp - target|^2).
 int sg_mlp_backward(const sg_view* V, const double* box, double rc, const float* params, const void* W1b16,
                     const void* Wpq16, const void* s16, const void* h16, const float* PQ, const float* disp,
@@ -716,47 +961,32 @@ int sg_mlp_backward(const sg_view* V, const double* box, double rc, const float*
   if (!V || !box || !params || !grad) return SG_ERR_ARG;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const int M = V->slots;
-  cudaMemsetAsync(gPQ, 0, sizeof(float) * (size_t)M * 2 * F, st);
-  // layer 2 edges
-  k_ml_l2_bwd<<<EDGE_BLOCKS, 32 * EDGE_WARPS, 0, st>>>(*V, box, rc, params, PQ, disp, target, inv_n, gPQ, part,
-                                                       loss_part);
-  cudaMemsetAsync(red, 0, sizeof(float) * L2_GRAD, st);
-  k_ml_reduce<<<(L2_GRAD + 255) / 256, 256, 0, st>>>(part, EDGE_BLOCKS, L2_GRAD, red);
-  k_ml_place<<<1, 256, 0, st>>>(red, 256, grad, NP_W2E);
-  k_ml_place<<<1, 64, 0, st>>>(red + 256, 64, grad, NP_B2);
-  k_ml_place<<<1, 64, 0, st>>>(red + 320, 64, grad, NP_W2);
-  k_ml_place<<<1, 1, 0, st>>>(red + 384, 1, grad, NP_C);
-  // gPQ -> bf16 for the GEMMs
-  {
-    const size_t len = (size_t)M * 2 * F;
-    k_ml_to_bf16<<<(unsigned)((len + 255) / 256), 256, 0, st>>>(gPQ, (__nv_bfloat16*)gPQ16, len);
-  }
-  // gWpq = h^T gPQ (tensor cores, one CTA per SM)
-  constexpr int WG_BLOCKS = 148;
   int* werr = nullptr;
   if (cudaGetSymbolAddress((void**)&werr, g_ml_tc_err) != cudaSuccess) return SG_ERR_CUDA;
   cudaMemsetAsync(werr, 0, sizeof(int), st);
+  // layer 2 edges
+  k_ml_l2_bwd<<<EDGE_BLOCKS, 32 * EDGE_WARPS, 0, st>>>(*V, box, rc, params, PQ, disp, target, inv_n,
+                                                       (__nv_bfloat16*)gPQ16, part, loss_part);
+  reduce_into(part, EDGE_BLOCKS, L2_GRAD, grad + NP_B2, st);
+  // gWpq = h^T gPQ (tensor cores, one CTA per SM)
+  constexpr int WG_BLOCKS = 148;
   int wrc = launch_wgrad_tc<2 * F>(h16, gPQ16, M, WG_BLOCKS, part, werr, st);
   if (wrc) return wrc;
-  k_ml_reduce<<<(F * 2 * F + 255) / 256, 256, 0, st>>>(part, WG_BLOCKS, F * 2 * F, grad + NP_WPQ);
-  // gh = gPQ Wpq^T
-  wrc = launch_gemm_tc<2 * F, F>(gPQ16, Wpq16, M, nullptr, 0, box, gh, nullptr, werr, st);
+  reduce_into(part, WG_BLOCKS, F * 2 * F, grad + NP_WPQ, st);
+  // gh = gPQ Wpq^T, through relu(s W1b + b1b): gpre, and its column sums
+  wrc = launch_gemm_tc<2 * F, F>(gPQ16, Wpq16, M, nullptr, 0, box, nullptr, gpre16, h16, werr, st);
   if (wrc) return wrc;
-  // through relu(s W1b + b1b)
-  k_ml_relu_bwd<<<WG_BLOCKS, 256, 0, st>>>(M, gh, (const __nv_bfloat16*)h16, (__nv_bfloat16*)gpre16, part);
-  k_ml_reduce<<<1, 64, 0, st>>>(part, WG_BLOCKS, F, grad + NP_B1B);
+  k_ml_colsum<<<COLSUM_BLOCKS, 256, 0, st>>>(M, (const __nv_bfloat16*)gpre16, part);
+  reduce_into(part, COLSUM_BLOCKS, F, grad + NP_B1B, st);
   wrc = launch_wgrad_tc<F>(s16, gpre16, M, WG_BLOCKS, part, werr, st);
   if (wrc) return wrc;
-  k_ml_reduce<<<(F * F + 255) / 256, 256, 0, st>>>(part, WG_BLOCKS, F * F, grad + NP_W1B);
+  reduce_into(part, WG_BLOCKS, F * F, grad + NP_W1B, st);
   // gs = gpre W1b^T
-  wrc = launch_gemm_tc<F, F>(gpre16, W1b16, M, nullptr, 0, box, gs, nullptr, werr, st);
+  wrc = launch_gemm_tc<F, F>(gpre16, W1b16, M, nullptr, 0, box, gs, nullptr, nullptr, werr, st);
   if (wrc) return wrc;
   // layer 1 edges
   k_ml_l1_bwd<<<EDGE_BLOCKS, 32 * EDGE_WARPS, 0, st>>>(*V, box, rc, params, gs, part);
-  cudaMemsetAsync(red, 0, sizeof(float) * L1_GRAD, st);
-  k_ml_reduce<<<(L1_GRAD + 255) / 256, 256, 0, st>>>(part, EDGE_BLOCKS, L1_GRAD, red);
-  k_ml_place<<<1, 256, 0, st>>>(red, 256, grad, NP_W1A);
-  k_ml_place<<<1, 64, 0, st>>>(red + 256, 64, grad, NP_B1A);
+  reduce_into(part, EDGE_BLOCKS, L1_GRAD, grad + NP_W1A, st);
   if (cudaGetLastError() != cudaSuccess) return SG_ERR_CUDA;
   int timed_out = 0;
   if (cudaMemcpyAsync(&timed_out, werr, sizeof(int), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
