@@ -35,16 +35,20 @@ constexpr int EDGE_WARPS = 8;  // warps per block in the edge kernels
 constexpr int EDGE_BLOCKS = 148 * 8;
 
 // ---- edge passes ---------------------------------------------------------------
-// A warp takes EDGE_P consecutive slots and EDGE_Q list entries of each at a
-// time.  First each lane works out the geometry of one entry (FP64 minimum
-// image, square root, quotients) and leaves it in shared memory; then the warp
-// walks every slot's edges in list order with one feature pair (f, f + 32) per
-// lane.  With the geometry inside the feature loop every lane repeated the FP64
-// of every edge, and the passes were bound by the FP64 pipe (64 packings of
-// 4,096 particles: 187, 412, 550 and 286 us for the four passes).  The
-// feature arithmetic is packed FP32 (fma.rn.f32x2): one instruction for the
-// pair, rounded as the two scalar ones.
-constexpr int EDGE_P = 4, EDGE_Q = 8;
+// A warp takes EDGE_P consecutive slots.  Their list entries form one flat run;
+// EDGE_CAP of them at a time are worked out with one entry per lane (FP64
+// minimum image, square root, quotients) and the edges among them (r < rc) put
+// in shared memory without gaps, in list order.  Then the warp walks the edges
+// with one feature pair (f, f + 32) per lane.  With the geometry inside the
+// feature loop every lane repeated the FP64 of every edge, and the passes were
+// bound by the FP64 pipe; now they wait for memory (entry, neighbour's position,
+// neighbour's row), so the next slots' data and the rows of EDGE_L edges are
+// requested together.  The feature arithmetic is packed FP32 (fma.rn.f32x2):
+// one instruction for the pair, rounded as the two scalar ones.  64 packings of
+// 4,096 particles, before and now: layer 1 forward 187 and 68 us, backward 286
+// and 97; layer 2 forward 412 and 134, backward 550 (and 120 for what it left to
+// convert and clear) and 213.
+constexpr int EDGE_P = 8, EDGE_CAP = 64, EDGE_L = 4;
 
 typedef unsigned long long f2_t;  // two FP32 values: features f and f + 32
 __device__ __forceinline__ f2_t f2_pack(float lo, float hi) {
@@ -71,59 +75,100 @@ __device__ __forceinline__ f2_t f2_mul(f2_t a, f2_t b) {
 }
 __device__ __forceinline__ f2_t f2_relu(f2_t a) { return f2_pack(fmaxf(f2_lo(a), 0.f), fmaxf(f2_hi(a), 0.f)); }
 
-// one warp's staged edges: features as packed pairs (e, e), the unit vector
+// one warp's slots and staged edges: features as packed pairs (e, e), the unit
+// vector, the neighbour's slot, the slot's number in the group
 struct EdgeStage {
-  ulonglong2 e01[32], e23[32];
-  float2 u[32];
+  ulonglong2 e01[EDGE_CAP], e23[EDGE_CAP];
+  float2 u[EDGE_CAP];
+  int j[EDGE_CAP], p[EDGE_CAP];
+  double x[EDGE_P], y[EDGE_P], Lx[EDGE_P], Ly[EDGE_P];
+  float a[EDGE_P];
+  int off[EDGE_P + 1];    // first flat entry of each slot
+  int first[EDGE_P + 1];  // first staged edge of each slot, of the current EDGE_CAP entries
 };
 
-// a lane's slot in the group of EDGE_P slots from i0: its particle and entry
-struct EdgeLane {
-  int i, cnt;
+// lane p < EDGE_P: slot i0 + p (no entries for padding and slots outside the batch)
+struct EdgeSlot {
+  int cnt;
   double x, y, Lx, Ly;
   float a;
 };
-__device__ __forceinline__ EdgeLane edge_lane(const sg_view& V, const double* __restrict__ box, int i0, int lane) {
-  EdgeLane L;
-  L.i = i0 + lane / EDGE_Q;
-  L.cnt = 0;
-  L.x = L.y = 0.0; L.a = 0.f; L.Lx = L.Ly = 0.0;
-  if (L.i < V.slots) {
-    L.Lx = box[2 * (size_t)L.i]; L.Ly = box[2 * (size_t)L.i + 1];
-    if (L.Lx > 0.0) {
-      L.cnt = V.nb_cnt_device[L.i];
-      L.x = V.x_device[L.i]; L.y = V.y_device[L.i];
-      L.a = (float)V.radius_device[L.i];
-    }
+__device__ __forceinline__ EdgeSlot edge_slot(const sg_view& V, const double* __restrict__ box, int i0, int lane) {
+  EdgeSlot L{0, 0.0, 0.0, 0.0, 0.0, 0.f};
+  const int i = i0 + lane;
+  if (lane < EDGE_P && i < V.slots) {
+    const double2 b = reinterpret_cast<const double2*>(box)[i];
+    L.Lx = b.x; L.Ly = b.y;
+    const int c = V.nb_cnt_device[i];
+    L.x = V.x_device[i]; L.y = V.y_device[i];
+    L.a = (float)V.radius_device[i];
+    L.cnt = b.x > 0.0 ? c : 0;
   }
   return L;
 }
 
-// Stages entry q of the lane's slot; returns the mask of the warp's entries
-// that are edges (r < rc), *j the lane's neighbour (its own slot without an edge).
-__device__ __forceinline__ unsigned stage_edge(const sg_view& V, const EdgeLane& L, int q, double rc, int lane,
-                                               EdgeStage& S, int* j_out, float2* u_out) {
-  bool edge = false;
-  int j = L.i;
-  float2 u = make_float2(0.f, 0.f);
-  if (q < L.cnt) {
-    j = V.nb_device[(size_t)q * V.nb_stride + L.i];
-    double dx = V.x_device[j] - L.x, dy = V.y_device[j] - L.y;
-    if (dx > 0.5 * L.Lx) dx -= L.Lx; else if (dx < -0.5 * L.Lx) dx += L.Lx;
-    if (dy > 0.5 * L.Ly) dy -= L.Ly; else if (dy < -0.5 * L.Ly) dy += L.Ly;
-    const double r = sqrt(dx * dx + dy * dy);
-    edge = r < rc && r != 0.0;
-    if (edge) {
-      const float aj = (float)V.radius_device[j], rf = (float)r, g = L.a + aj - rf;
-      u = make_float2((float)(dx / r), (float)(dy / r));
-      S.e01[lane] = make_ulonglong2(f2_pack(rf, rf), f2_pack(L.a, L.a));
-      S.e23[lane] = make_ulonglong2(f2_pack(aj, aj), f2_pack(g, g));
-    }
+// Puts the group's slots in place; returns the number of its list entries.
+__device__ __forceinline__ int stage_slots(const EdgeSlot& L, int lane, EdgeStage& S) {
+  int inc = L.cnt;
+#pragma unroll
+  for (int o = 1; o < EDGE_P; o <<= 1) {
+    const int v = __shfl_up_sync(0xffffffffu, inc, o);
+    if (lane >= o) inc += v;
   }
-  S.u[lane] = u;
-  *j_out = j;
-  *u_out = u;
-  return __ballot_sync(0xffffffffu, edge);
+  if (lane < EDGE_P) {
+    S.x[lane] = L.x; S.y[lane] = L.y; S.Lx[lane] = L.Lx; S.Ly[lane] = L.Ly; S.a[lane] = L.a;
+    S.off[lane + 1] = inc;
+  }
+  if (lane == 0) S.off[0] = 0;
+  __syncwarp();
+  return S.off[EDGE_P];
+}
+
+// Stages the edges among entries [t0, t0 + EDGE_CAP); returns their number.
+__device__ __forceinline__ int stage_edges(const sg_view& V, int i0, int t0, int total, double rc, int lane,
+                                           EdgeStage& S) {
+  int n = 0, first = 0;
+  const int bound = lane <= EDGE_P ? S.off[lane] : 0;  // lane p: where slot p's entries begin
+#pragma unroll
+  for (int w = 0; w < EDGE_CAP; w += 32) {
+    if (t0 + w >= total) break;  // the same for the whole warp
+    const int t = t0 + w + lane;
+    bool edge = false;
+    int j = 0, p = 0;
+    float2 u = make_float2(0.f, 0.f);
+    float rf = 0.f, ai = 0.f, aj = 0.f, g = 0.f;
+    if (t < total) {
+#pragma unroll
+      for (int k = 1; k < EDGE_P; k++) p += t >= S.off[k] ? 1 : 0;
+      j = V.nb_device[(size_t)(t - S.off[p]) * V.nb_stride + i0 + p];
+      double dx = V.x_device[j] - S.x[p], dy = V.y_device[j] - S.y[p];
+      const double Lx = S.Lx[p], Ly = S.Ly[p];
+      if (dx > 0.5 * Lx) dx -= Lx; else if (dx < -0.5 * Lx) dx += Lx;
+      if (dy > 0.5 * Ly) dy -= Ly; else if (dy < -0.5 * Ly) dy += Ly;
+      const double r = sqrt(dx * dx + dy * dy);
+      edge = r < rc && r != 0.0;
+      if (edge) {
+        ai = S.a[p]; aj = (float)V.radius_device[j];
+        rf = (float)r; g = ai + aj - rf;
+        u = make_float2((float)(dx / r), (float)(dy / r));
+      }
+    }
+    const unsigned m = __ballot_sync(0xffffffffu, edge);
+    if (edge) {
+      const int at = n + __popc(m & ((1u << lane) - 1u));
+      S.e01[at] = make_ulonglong2(f2_pack(rf, rf), f2_pack(ai, ai));
+      S.e23[at] = make_ulonglong2(f2_pack(aj, aj), f2_pack(g, g));
+      S.u[at] = u;
+      S.j[at] = j;
+      S.p[at] = p;
+    }
+    const int below = bound - (t0 + w);  // edges of this round before the bound
+    first += below <= 0 ? 0 : below >= 32 ? __popc(m) : __popc(m & ((1u << below) - 1u));
+    n += __popc(m);
+  }
+  if (lane <= EDGE_P) S.first[lane] = first;
+  __syncwarp();
+  return n;
 }
 
 // feature pairs (lane, lane + 32) of a [64 x 4] weight and a [64] vector
@@ -152,40 +197,35 @@ __device__ __forceinline__ f2_t edge_layer1(const EdgeWeights& E, const ulonglon
 }
 
 // ---- layer 1 edges: s_i = sum_j relu(W1a e + b1a), stored BF16 ----------------
-__global__ void __launch_bounds__(32 * EDGE_WARPS)
+__global__ void __launch_bounds__(32 * EDGE_WARPS, 4)
 k_ml_l1(sg_view V, const double* __restrict__ box, double rc, const float* __restrict__ P,
         __nv_bfloat16* __restrict__ s16) {
   __shared__ EdgeStage stage[EDGE_WARPS];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   EdgeStage& S = stage[warp];
-  const int nw = gridDim.x * EDGE_WARPS;
+  const int step = gridDim.x * EDGE_WARPS * EDGE_P;
   const EdgeWeights E = edge_weights(P + NP_W1A, P + NP_B1A, lane);
-  for (int i0 = (blockIdx.x * EDGE_WARPS + warp) * EDGE_P; i0 < V.slots; i0 += nw * EDGE_P) {
-    const EdgeLane L = edge_lane(V, box, i0, lane);
-    const int most = __reduce_max_sync(0xffffffffu, L.cnt);
-    f2_t acc[EDGE_P];
-#pragma unroll
-    for (int p = 0; p < EDGE_P; p++) acc[p] = 0ull;
-    for (int q0 = 0; q0 < most; q0 += EDGE_Q) {
-      int j;
-      float2 u;
-      const unsigned mask = stage_edge(V, L, q0 + lane % EDGE_Q, rc, lane, S, &j, &u);
-      __syncwarp();
-#pragma unroll
-      for (int p = 0; p < EDGE_P; p++) {
-        for (unsigned m = mask & (0xffu << (p * EDGE_Q)); m; m &= m - 1) {
-          const int q = __ffs(m) - 1;
-          acc[p] = f2_add(acc[p], f2_relu(edge_layer1(E, S.e01[q], S.e23[q])));
+  int i0 = (blockIdx.x * EDGE_WARPS + warp) * EDGE_P;
+  EdgeSlot next = edge_slot(V, box, i0, lane);
+  for (; i0 < V.slots; i0 += step) {
+    const int total = stage_slots(next, lane, S);
+    next = edge_slot(V, box, i0 + step, lane);
+    int p = 0;
+    f2_t acc = 0ull;
+    for (int t0 = 0; p < EDGE_P; t0 += EDGE_CAP) {
+      stage_edges(V, i0, t0, total, rc, lane, S);
+      for (; p < EDGE_P; p++) {  // a slot whose entries go on beyond these keeps its sum
+        const int e1 = S.first[p + 1];
+        for (int e = S.first[p]; e < e1; e++) acc = f2_add(acc, f2_relu(edge_layer1(E, S.e01[e], S.e23[e])));
+        if (S.off[p + 1] > t0 + EDGE_CAP) break;
+        if (i0 + p < V.slots) {
+          s16[(size_t)(i0 + p) * F + lane] = __float2bfloat16_rn(f2_lo(acc));
+          s16[(size_t)(i0 + p) * F + lane + 32] = __float2bfloat16_rn(f2_hi(acc));
         }
+        acc = 0ull;
       }
       __syncwarp();
     }
-#pragma unroll
-    for (int p = 0; p < EDGE_P; p++)
-      if (i0 + p < V.slots) {
-        s16[(size_t)(i0 + p) * F + lane] = __float2bfloat16_rn(f2_lo(acc[p]));
-        s16[(size_t)(i0 + p) * F + lane + 32] = __float2bfloat16_rn(f2_hi(acc[p]));
-      }
   }
 }
 
@@ -590,54 +630,45 @@ static void reduce_into(const float* partial, int nblk, int len, float* out, cud
 }
 
 // ---- layer 2 edges (forward): disp_i --------------------------------------------
-// The 64-wide dot products of a slot's EDGE_Q edges are summed over the lanes
-// together: at offsets 16, 8 and 4 a lane passes on half of its edges' sums and
-// keeps the other half (7 + 2 shuffles for 8 edges instead of 40, the same
-// pairs added in the same order as in one sum after the other).
-__global__ void __launch_bounds__(32 * EDGE_WARPS)
+// The 64-wide dot products of EDGE_B edges are summed over the lanes together:
+// at offsets 16, 8 and 4 a lane passes on half of its edges' sums and keeps the
+// other half (7 + 2 shuffles for 8 edges instead of 40; the same pairs are added
+// in the same order as in one sum after the other).
+constexpr int EDGE_B = 8;
+__global__ void __launch_bounds__(32 * EDGE_WARPS, 4)
 k_ml_l2(sg_view V, const double* __restrict__ box, double rc, const float* __restrict__ P,
         const float* __restrict__ PQ, float* __restrict__ disp) {
   __shared__ EdgeStage stage[EDGE_WARPS];
-  __shared__ float wsh[EDGE_WARPS][32];
+  __shared__ float wsh[EDGE_WARPS][EDGE_CAP];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   EdgeStage& S = stage[warp];
-  const int nw = gridDim.x * EDGE_WARPS;
+  const int step = gridDim.x * EDGE_WARPS * EDGE_P;
   const EdgeWeights E = edge_weights(P + NP_W2E, P + NP_B2, lane);
   const float w2a = P[NP_W2 + lane], w2b = P[NP_W2 + lane + 32], c = P[NP_C];
-  for (int i0 = (blockIdx.x * EDGE_WARPS + warp) * EDGE_P; i0 < V.slots; i0 += nw * EDGE_P) {
-    const EdgeLane L = edge_lane(V, box, i0, lane);
-    const int most = __reduce_max_sync(0xffffffffu, L.cnt);
+  int i0 = (blockIdx.x * EDGE_WARPS + warp) * EDGE_P;
+  EdgeSlot next = edge_slot(V, box, i0, lane);
+  for (; i0 < V.slots; i0 += step) {
+    const int total = stage_slots(next, lane, S);
+    next = edge_slot(V, box, i0 + step, lane);
     float dx = 0.f, dy = 0.f;  // lane p < EDGE_P: slot i0 + p
-    for (int q0 = 0; q0 < most; q0 += EDGE_Q) {
-      int j;
-      float2 u;
-      const unsigned mask = stage_edge(V, L, q0 + lane % EDGE_Q, rc, lane, S, &j, &u);
-      __syncwarp();
+    for (int t0 = 0; t0 < total; t0 += EDGE_CAP) {
+      const int n = stage_edges(V, i0, t0, total, rc, lane, S);
+      for (int e0 = 0; e0 < n; e0 += EDGE_B) {
+        f2_t z[EDGE_B];
 #pragma unroll
-      for (int p = 0; p < EDGE_P; p++) {
-        const unsigned m = (mask >> (p * EDGE_Q)) & 0xffu;
-        if (!m) continue;
-        const float* Pi = PQ + (size_t)(i0 + p) * 2 * F;
-        const f2_t pi = f2_pack(Pi[lane], Pi[lane + 32]);
-        f2_t qj[EDGE_Q];
-#pragma unroll
-        for (int q = 0; q < EDGE_Q; q++) {
-          const int jq = __shfl_sync(0xffffffffu, j, p * EDGE_Q + q);
-          if (m >> q & 1) {
-            const float* Qj = PQ + (size_t)jq * 2 * F + F;
-            qj[q] = f2_pack(Qj[lane], Qj[lane + 32]);
-          }
+        for (int v = 0; v < EDGE_B; v++) {
+          const int e = min(e0 + v, n - 1);  // past the end: the last edge again, its sum unused
+          const float *Pi = PQ + (size_t)(i0 + S.p[e]) * 2 * F, *Qj = PQ + (size_t)S.j[e] * 2 * F + F;
+          z[v] = f2_add(f2_pack(Pi[lane], Pi[lane + 32]), f2_pack(Qj[lane], Qj[lane + 32]));
         }
-        float part[EDGE_Q];
+        float part[EDGE_B];
 #pragma unroll
-        for (int q = 0; q < EDGE_Q; q++) {
-          part[q] = 0.f;
-          if (m >> q & 1) {
-            const f2_t z = edge_affine(E, S.e01[p * EDGE_Q + q], S.e23[p * EDGE_Q + q], f2_add(pi, qj[q]));
-            part[q] = fmaf(fmaxf(f2_hi(z), 0.f), w2b, fmaxf(f2_lo(z), 0.f) * w2a);
-          }
+        for (int v = 0; v < EDGE_B; v++) {
+          const int e = min(e0 + v, n - 1);
+          z[v] = edge_affine(E, S.e01[e], S.e23[e], z[v]);
+          part[v] = fmaf(fmaxf(f2_hi(z[v]), 0.f), w2b, fmaxf(f2_lo(z[v]), 0.f) * w2a);
         }
-        static_assert(EDGE_Q == 8, "three halving steps");
+        static_assert(EDGE_B == 8, "three halving steps");
 #pragma unroll
         for (int h = 4, o = 16; h > 0; h >>= 1, o >>= 1) {
           const bool up = lane & o;
@@ -649,14 +680,13 @@ k_ml_l2(sg_view V, const double* __restrict__ box, double rc, const float* __res
         }
         part[0] += __shfl_xor_sync(0xffffffffu, part[0], 2);
         part[0] += __shfl_xor_sync(0xffffffffu, part[0], 1);
-        if ((lane & 3) == 0) wsh[warp][p * EDGE_Q + (lane >> 2)] = part[0] + c;
+        if ((lane & 3) == 0) wsh[warp][e0 + (lane >> 2)] = part[0] + c;
       }
       __syncwarp();
       if (lane < EDGE_P)
-        for (unsigned m = mask & (0xffu << (lane * EDGE_Q)); m; m &= m - 1) {
-          const int q = __ffs(m) - 1;
-          dx = fmaf(wsh[warp][q], S.u[q].x, dx);
-          dy = fmaf(wsh[warp][q], S.u[q].y, dy);
+        for (int e = S.first[lane]; e < S.first[lane + 1]; e++) {
+          dx = fmaf(wsh[warp][e], S.u[e].x, dx);
+          dy = fmaf(wsh[warp][e], S.u[e].y, dy);
         }
       __syncwarp();
     }
@@ -670,92 +700,98 @@ k_ml_l2(sg_view V, const double* __restrict__ box, double rc, const float* __res
 // lists are full, so beside edge (i, j), whose gz_ij goes to P_i and the weight
 // gradients, the warp works out edge (j, i), whose gz_ji goes to Q_i, from row
 // j.  That costs another 256-byte row per edge and replaces the atomic adds
-// into row j, the zeroing of gPQ in FP32 and its conversion (550 + 99 + 20 us).
+// into row j, the zeroing of gPQ in FP32 and its conversion.
 // Per-block partials of (gb2, gW2e, gw2, gc), in parameter order, go to
 // part[block].
 constexpr int L2_GRAD = 64 + 256 + 64 + 1;  // b2, W2e, w2, c: as from NP_B2 on
-__global__ void __launch_bounds__(32 * EDGE_WARPS)
+__global__ void __launch_bounds__(32 * EDGE_WARPS, 4)
 k_ml_l2_bwd(sg_view V, const double* __restrict__ box, double rc, const float* __restrict__ P,
             const float* __restrict__ PQ, const float* __restrict__ disp, const float* __restrict__ target, float inv_n,
             __nv_bfloat16* __restrict__ gPQ16, float* __restrict__ part, float* __restrict__ loss_part) {
   __shared__ EdgeStage stage[EDGE_WARPS];
-  __shared__ float2 gsh[EDGE_WARPS][32];  // d loss / d w of edges (i, j) and (j, i)
+  __shared__ float2 gsh[EDGE_WARPS][EDGE_CAP];  // d loss / d w of edges (i, j) and (j, i)
+  __shared__ float2 dsh[EDGE_WARPS][EDGE_P];    // d loss / d disp_i
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   EdgeStage& S = stage[warp];
-  const int nw = gridDim.x * EDGE_WARPS;
+  const int step = gridDim.x * EDGE_WARPS * EDGE_P;
   const EdgeWeights E = edge_weights(P + NP_W2E, P + NP_B2, lane);
   const f2_t w2 = f2_pack(P[NP_W2 + lane], P[NP_W2 + lane + 32]);
   f2_t gWe[4] = {0ull, 0ull, 0ull, 0ull}, gb2 = 0ull, gw2 = 0ull;
   float gc = 0.f, lsum = 0.f;
-  for (int i0 = (blockIdx.x * EDGE_WARPS + warp) * EDGE_P; i0 < V.slots; i0 += nw * EDGE_P) {
-    const EdgeLane L = edge_lane(V, box, i0, lane);
-    const int most = __reduce_max_sync(0xffffffffu, L.cnt);
-    float gdx = 0.f, gdy = 0.f;
-    if (L.Lx > 0.0) {
-      const float2 d = reinterpret_cast<const float2*>(disp)[L.i], t = reinterpret_cast<const float2*>(target)[L.i];
+  int i0 = (blockIdx.x * EDGE_WARPS + warp) * EDGE_P;
+  EdgeSlot next = edge_slot(V, box, i0, lane);
+  for (; i0 < V.slots; i0 += step) {
+    if (lane < EDGE_P && next.Lx > 0.0) {
+      const float2 d = reinterpret_cast<const float2*>(disp)[i0 + lane],
+                   t = reinterpret_cast<const float2*>(target)[i0 + lane];
       const float ex = d.x - t.x, ey = d.y - t.y;
-      if (lane % EDGE_Q == 0) lsum += ex * ex + ey * ey;
-      gdx = 2.f * ex * inv_n; gdy = 2.f * ey * inv_n;
+      lsum += ex * ex + ey * ey;
+      dsh[warp][lane] = make_float2(2.f * ex * inv_n, 2.f * ey * inv_n);
     }
-    f2_t gP[EDGE_P], gQ[EDGE_P];
-#pragma unroll
-    for (int p = 0; p < EDGE_P; p++) gP[p] = gQ[p] = 0ull;
-    for (int q0 = 0; q0 < most; q0 += EDGE_Q) {
-      int j;
-      float2 u;
-      const unsigned mask = stage_edge(V, L, q0 + lane % EDGE_Q, rc, lane, S, &j, &u);
-      if (mask >> lane & 1) {
+    const int total = stage_slots(next, lane, S);
+    next = edge_slot(V, box, i0 + step, lane);
+    int p = 0;
+    f2_t gP = 0ull, gQ = 0ull;
+    for (int t0 = 0; p < EDGE_P; t0 += EDGE_CAP) {
+      const int n = stage_edges(V, i0, t0, total, rc, lane, S);
+      for (int e = lane; e < n; e += 32) {
+        const int j = S.j[e];
         const float2 d = reinterpret_cast<const float2*>(disp)[j], t = reinterpret_cast<const float2*>(target)[j];
-        const float gw = gdx * u.x + gdy * u.y;
+        const float2 gi = dsh[warp][S.p[e]], u = S.u[e];
+        const float gw = gi.x * u.x + gi.y * u.y;
         // the vector from j to i is exactly the opposite
-        const float gr = -(2.f * (d.x - t.x) * inv_n * u.x + 2.f * (d.y - t.y) * inv_n * u.y);
-        gsh[warp][lane] = make_float2(gw, gr);
+        gsh[warp][e] = make_float2(gw, -(2.f * (d.x - t.x) * inv_n * u.x + 2.f * (d.y - t.y) * inv_n * u.y));
         gc += gw;
       }
       __syncwarp();
+      for (; p < EDGE_P; p++) {
+        const int e1 = S.first[p + 1];
+        if (S.first[p] < e1) {
+          const float* Ri = PQ + (size_t)(i0 + p) * 2 * F;
+          const f2_t pi = f2_pack(Ri[lane], Ri[lane + 32]), qi = f2_pack(Ri[F + lane], Ri[F + lane + 32]);
+          for (int e0 = S.first[p]; e0 < e1; e0 += EDGE_L) {
+            f2_t pj[EDGE_L], qj[EDGE_L];
 #pragma unroll
-      for (int p = 0; p < EDGE_P; p++) {
-        const unsigned m = (mask >> (p * EDGE_Q)) & 0xffu;
-        if (!m) continue;
-        const float* Ri = PQ + (size_t)(i0 + p) * 2 * F;
-        const f2_t pi = f2_pack(Ri[lane], Ri[lane + 32]), qi = f2_pack(Ri[F + lane], Ri[F + lane + 32]);
+            for (int v = 0; v < EDGE_L; v++) {
+              const float* Rj = PQ + (size_t)S.j[min(e0 + v, e1 - 1)] * 2 * F;
+              pj[v] = f2_pack(Rj[lane], Rj[lane + 32]);
+              qj[v] = f2_pack(Rj[F + lane], Rj[F + lane + 32]);
+            }
 #pragma unroll
-        for (int q = 0; q < EDGE_Q; q++) {
-          const int t = p * EDGE_Q + q;
-          const int jq = __shfl_sync(0xffffffffu, j, t);
-          if (m >> q & 1) {
-            const float* Rj = PQ + (size_t)jq * 2 * F;
-            const f2_t pj = f2_pack(Rj[lane], Rj[lane + 32]), qj = f2_pack(Rj[F + lane], Rj[F + lane + 32]);
-            const ulonglong2 e01 = S.e01[t], e23 = S.e23[t];
-            const float2 g = gsh[warp][t];
-            const f2_t gw = f2_pack(g.x, g.x), gr = f2_pack(g.y, g.y);
-            const f2_t z = edge_affine(E, e01, e23, f2_add(pi, qj));
-            // edge (j, i): the two radii change places
-            const f2_t y = edge_affine(E, make_ulonglong2(e01.x, e23.x), make_ulonglong2(e01.y, e23.y), f2_add(pj, qi));
-            const f2_t fz = f2_mul(gw, w2), fy = f2_mul(gr, w2);
-            const f2_t gz = f2_pack(f2_lo(z) > 0.f ? f2_lo(fz) : 0.f, f2_hi(z) > 0.f ? f2_hi(fz) : 0.f);
-            const f2_t gy = f2_pack(f2_lo(y) > 0.f ? f2_lo(fy) : 0.f, f2_hi(y) > 0.f ? f2_hi(fy) : 0.f);
-            gw2 = f2_fma(gw, f2_relu(z), gw2);
-            gWe[0] = f2_fma(gz, e01.x, gWe[0]);
-            gWe[2] = f2_fma(gz, e23.x, gWe[2]);
-            gWe[3] = f2_fma(gz, e23.y, gWe[3]);
-            gP[p] = f2_add(gP[p], gz);
-            gQ[p] = f2_add(gQ[p], gy);
+            for (int v = 0; v < EDGE_L; v++) {
+              const int e = e0 + v;
+              if (e >= e1) break;
+              const ulonglong2 e01 = S.e01[e], e23 = S.e23[e];
+              const float2 g = gsh[warp][e];
+              const f2_t gw = f2_pack(g.x, g.x), gr = f2_pack(g.y, g.y);
+              const f2_t z = edge_affine(E, e01, e23, f2_add(pi, qj[v]));
+              // edge (j, i): the two radii change places
+              const f2_t y = edge_affine(E, make_ulonglong2(e01.x, e23.x), make_ulonglong2(e01.y, e23.y),
+                                         f2_add(pj[v], qi));
+              const f2_t fz = f2_mul(gw, w2), fy = f2_mul(gr, w2);
+              const f2_t gz = f2_pack(f2_lo(z) > 0.f ? f2_lo(fz) : 0.f, f2_hi(z) > 0.f ? f2_hi(fz) : 0.f);
+              const f2_t gy = f2_pack(f2_lo(y) > 0.f ? f2_lo(fy) : 0.f, f2_hi(y) > 0.f ? f2_hi(fy) : 0.f);
+              gw2 = f2_fma(gw, f2_relu(z), gw2);
+              gWe[0] = f2_fma(gz, e01.x, gWe[0]);
+              gWe[2] = f2_fma(gz, e23.x, gWe[2]);
+              gWe[3] = f2_fma(gz, e23.y, gWe[3]);
+              gP = f2_add(gP, gz);
+              gQ = f2_add(gQ, gy);
+            }
           }
         }
+        if (S.off[p + 1] > t0 + EDGE_CAP) break;  // its entries go on: the sums are kept
+        const float ai = S.a[p];
+        gWe[1] = f2_fma(gP, f2_pack(ai, ai), gWe[1]);  // its own radius: the same for all of a slot's edges
+        gb2 = f2_add(gb2, gP);
+        if (i0 + p < V.slots) {
+          __nv_bfloat16* R = gPQ16 + (size_t)(i0 + p) * 2 * F;  // padding slots: zeros
+          R[lane] = __float2bfloat16_rn(f2_lo(gP)); R[lane + 32] = __float2bfloat16_rn(f2_hi(gP));
+          R[F + lane] = __float2bfloat16_rn(f2_lo(gQ)); R[F + lane + 32] = __float2bfloat16_rn(f2_hi(gQ));
+        }
+        gP = gQ = 0ull;
       }
       __syncwarp();
-    }
-#pragma unroll
-    for (int p = 0; p < EDGE_P; p++) {
-      const float ai = __shfl_sync(0xffffffffu, L.a, p * EDGE_Q);
-      gWe[1] = f2_fma(gP[p], f2_pack(ai, ai), gWe[1]);  // its own radius: the same for all of a slot's edges
-      gb2 = f2_add(gb2, gP[p]);
-      if (i0 + p < V.slots) {
-        __nv_bfloat16* R = gPQ16 + (size_t)(i0 + p) * 2 * F;  // padding slots: zeros
-        R[lane] = __float2bfloat16_rn(f2_lo(gP[p])); R[lane + 32] = __float2bfloat16_rn(f2_hi(gP[p]));
-        R[F + lane] = __float2bfloat16_rn(f2_lo(gQ[p])); R[F + lane + 32] = __float2bfloat16_rn(f2_hi(gQ[p]));
-      }
     }
   }
   // block reduction of the weight-gradient partials (fixed order over warps)
@@ -820,53 +856,48 @@ k_ml_colsum(int M, const __nv_bfloat16* __restrict__ a, float* __restrict__ part
 // The gradient gs_i of s_i is the same for all edges of slot i, so a slot first
 // sums the features of its active edges (z > 0) and multiplies by gs_i once.
 constexpr int L1_GRAD = 256 + 64;
-__global__ void __launch_bounds__(32 * EDGE_WARPS)
+__global__ void __launch_bounds__(32 * EDGE_WARPS, 4)
 k_ml_l1_bwd(sg_view V, const double* __restrict__ box, double rc, const float* __restrict__ P,
             const float* __restrict__ gs, float* __restrict__ part) {
   __shared__ EdgeStage stage[EDGE_WARPS];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   EdgeStage& S = stage[warp];
-  const int nw = gridDim.x * EDGE_WARPS;
+  const int step = gridDim.x * EDGE_WARPS * EDGE_P;
   const EdgeWeights E = edge_weights(P + NP_W1A, P + NP_B1A, lane);
   f2_t gW[4] = {0ull, 0ull, 0ull, 0ull}, gb = 0ull;
-  for (int i0 = (blockIdx.x * EDGE_WARPS + warp) * EDGE_P; i0 < V.slots; i0 += nw * EDGE_P) {
-    const EdgeLane L = edge_lane(V, box, i0, lane);
-    const int most = __reduce_max_sync(0xffffffffu, L.cnt);
-    f2_t s0[EDGE_P], s2[EDGE_P], s3[EDGE_P], sn[EDGE_P], g[EDGE_P];
-#pragma unroll
-    for (int p = 0; p < EDGE_P; p++) {
-      s0[p] = s2[p] = s3[p] = sn[p] = 0ull;
-      const size_t row = (size_t)min(i0 + p, V.slots - 1) * F;
-      g[p] = f2_pack(gs[row + lane], gs[row + lane + 32]);
-    }
-    for (int q0 = 0; q0 < most; q0 += EDGE_Q) {
-      int j;
-      float2 u;
-      const unsigned mask = stage_edge(V, L, q0 + lane % EDGE_Q, rc, lane, S, &j, &u);
-      __syncwarp();
-#pragma unroll
-      for (int p = 0; p < EDGE_P; p++)
-        for (unsigned m = mask & (0xffu << (p * EDGE_Q)); m; m &= m - 1) {
-          const int q = __ffs(m) - 1;
-          const ulonglong2 e01 = S.e01[q], e23 = S.e23[q];
+  int i0 = (blockIdx.x * EDGE_WARPS + warp) * EDGE_P;
+  EdgeSlot next = edge_slot(V, box, i0, lane);
+  for (; i0 < V.slots; i0 += step) {
+    const int total = stage_slots(next, lane, S);
+    next = edge_slot(V, box, i0 + step, lane);
+    int p = 0;
+    f2_t s0 = 0ull, s2 = 0ull, s3 = 0ull, sn = 0ull;
+    for (int t0 = 0; p < EDGE_P; t0 += EDGE_CAP) {
+      stage_edges(V, i0, t0, total, rc, lane, S);
+      for (; p < EDGE_P; p++) {
+        const int e1 = S.first[p + 1];
+        const size_t row = (size_t)min(i0 + p, V.slots - 1) * F;
+        const f2_t g = f2_pack(gs[row + lane], gs[row + lane + 32]);
+        for (int e = S.first[p]; e < e1; e++) {
+          const ulonglong2 e01 = S.e01[e], e23 = S.e23[e];
           const f2_t z = edge_layer1(E, e01, e23);
           const f2_t on = f2_pack(f2_lo(z) > 0.f ? 1.f : 0.f, f2_hi(z) > 0.f ? 1.f : 0.f);
-          s0[p] = f2_fma(on, e01.x, s0[p]);
-          s2[p] = f2_fma(on, e23.x, s2[p]);
-          s3[p] = f2_fma(on, e23.y, s3[p]);
-          sn[p] = f2_add(sn[p], on);
+          s0 = f2_fma(on, e01.x, s0);
+          s2 = f2_fma(on, e23.x, s2);
+          s3 = f2_fma(on, e23.y, s3);
+          sn = f2_add(sn, on);
         }
+        if (S.off[p + 1] > t0 + EDGE_CAP) break;  // its entries go on: the sums are kept
+        const float ai = S.a[p];
+        const f2_t gn = f2_mul(g, sn);
+        gW[0] = f2_fma(g, s0, gW[0]);
+        gW[1] = f2_fma(gn, f2_pack(ai, ai), gW[1]);
+        gW[2] = f2_fma(g, s2, gW[2]);
+        gW[3] = f2_fma(g, s3, gW[3]);
+        gb = f2_add(gb, gn);
+        s0 = s2 = s3 = sn = 0ull;
+      }
       __syncwarp();
-    }
-#pragma unroll
-    for (int p = 0; p < EDGE_P; p++) {
-      const float ai = __shfl_sync(0xffffffffu, L.a, p * EDGE_Q);
-      const f2_t gn = f2_mul(g[p], sn[p]);  // slots without edges: zero
-      gW[0] = f2_fma(g[p], s0[p], gW[0]);
-      gW[1] = f2_fma(gn, f2_pack(ai, ai), gW[1]);
-      gW[2] = f2_fma(g[p], s2[p], gW[2]);
-      gW[3] = f2_fma(g[p], s3[p], gW[3]);
-      gb = f2_add(gb, gn);
     }
   }
   __shared__ float sp[EDGE_WARPS][L1_GRAD];

@@ -1,0 +1,68 @@
+"""The network's edge passes at the sizes where their staging turns over: slots
+without an edge, eight slots with more entries than are staged at a time, one
+slot with more than that by itself, and a batch that leaves replicas out.  The
+tolerances are those of BF16 operands (2^-9 each) over a few layers, as for the
+ordinary packings."""
+import numpy as np
+import pytest
+
+from oracle import warmstart_ref as W
+
+pytestmark = pytest.mark.gpu
+
+
+def two_clumps(n, seed):
+    """A particle between two clumps of 40 that do not see each other (at most
+    48 lower-id neighbours are allowed), among n - 81 sparse ones."""
+    from samos_b200.ensemble import quench_disks
+    parts, L = quench_disks(n, 0.05, seed)
+    rng = np.random.default_rng(seed)
+    far = np.hypot(parts["x"], parts["y"]) < 12.0
+    parts["x"][far] = L / 2 - 8.0 + rng.uniform(-6.0, 6.0, far.sum())
+    parts["x"][:81] = np.repeat([-2.6, 0.0, 2.6], [40, 1, 40]) + rng.uniform(-0.2, 0.2, 81)
+    parts["y"][:81] = rng.uniform(-0.2, 0.2, 81)
+    return parts, L
+
+
+@pytest.mark.parametrize("n,phi", [(200, 0.02), (300, 2.5), (400, None)])
+def test_forward_and_gradient_match_the_reference_network(n, phi):
+    from samos_b200.ensemble import plane_fire_ensemble, quench_disks
+    from samos_b200.warmstart import OFF, WarmStartNet
+
+    make = (lambda m, seed: quench_disks(m, phi, seed)) if phi else two_clumps
+    insts = [make(n, 31), quench_disks(129, 0.86, 32), make(n + 1, 33)]
+    eng = plane_fire_ensemble(insts)
+    eng.build_nlist()
+    counts = np.bincount(np.concatenate(eng.pairs(2)), minlength=n + 1)
+    assert {0.02: (counts == 0).any(), 2.5: counts.mean() > 8, None: counts.max() > 64}[phi]
+    net = WarmStartNet(seed=3)
+    rng = np.random.default_rng(4)
+    p = net.get_params()
+    p[OFF["w2"][0]:OFF["w2"][0] + 64] = rng.normal(0.0, 0.3, 64)
+    p[OFF["c"][0]] = 0.05
+    net.set_params(p)
+    targets = [rng.normal(0.0, 0.3, (len(pp["x"]), 2)) for pp, _ in insts]
+    chosen = (0, 2)  # the middle replica's slots are not part of the batch
+    box, tgt = net.box_array(eng, chosen), net.slot_targets(eng, targets)
+    n_valid = sum(len(insts[r][0]["x"]) for r in chosen)
+    loss = net.loss_and_grad(eng, box, tgt, n_valid)
+    got = net.grad.cpu().numpy().astype(np.float64)
+    disp = net.forward(eng, box).cpu().numpy().reshape(-1, 2).astype(np.float64)
+    ids = net.slot_ids(eng)
+    want, total = np.zeros(W.NPARAM), 0.0
+    for r in chosen:
+        parts, L = insts[r]
+        I, J, e, u = W.edges(eng.download("x", r), eng.download("y", r), parts["radius"], L, 2.8)
+        one, d, g = W.Net(p.astype(np.float64)).loss_and_grad(len(parts["x"]), I, J, e, u, targets[r], 1.0 / n_valid)
+        total, want = total + one, want + g
+        off, m = eng.replica_slots(r)
+        by_id = np.zeros((m, 2))
+        by_id[ids[off:off + m]] = disp[off:off + m]
+        assert np.linalg.norm(by_id - d) < 5e-3 * np.linalg.norm(d), r
+    off, m = eng.replica_slots(1)
+    assert not disp[off:off + m].any()
+    assert loss == pytest.approx(total, rel=5e-3)
+    for name, (o, s) in OFF.items():
+        size = int(np.prod(s))
+        assert np.linalg.norm(got[o:o + size] - want[o:o + size]) < 2e-2 * max(np.linalg.norm(want[o:o + size]), 1e-12), name
+    eng.close()
