@@ -81,19 +81,16 @@ constexpr int ABP_NTUNED = (int)(sizeof(ABP_TUNED) / sizeof(ABP_TUNED[0]));
 // similar list lengths and the warp's sweep is not set by one long list.
 // Padding slots go last.  Each particle's own arithmetic is unchanged.
 constexpr int LO_KEYS = 128;  // distinct sort keys the counting sort handles (list lengths 0..126 + padding)
-static_assert(BLOCK == LO_KEYS, "k_lane_order scans one key per thread");
+static_assert(BLOCK == LO_KEYS, "lane_order_block scans one key per thread");
 
-static __global__ void __launch_bounds__(BLOCK)
-k_lane_order(const Replica* __restrict__ reps, const int* __restrict__ blk_rep, NbList nl,
-             uint8_t* __restrict__ order, const int* __restrict__ blist = nullptr) {
+// `c`: this thread's list length, -1 for a padding slot; all of the block's threads call.
+__device__ __forceinline__ void lane_order_block(int c, int cap, uint8_t* order) {
   constexpr int NW = BLOCK / 32;
   __shared__ int hist[NW][LO_KEYS];  // per warp: lanes holding each key
   __shared__ int wsum[NW];
   __shared__ int sc[BLOCK];
-  const int b = blist ? blist[blockIdx.x] : (int)blockIdx.x, t = threadIdx.x, k = b * BLOCK + t;
-  const Replica& R = reps[blk_rep[b]];
-  const int c = (k - R.off < R.n) ? nl.cnt[k] : -1;
-  if (nl.cap + 2 > LO_KEYS) {  // long lists (same branch for the whole grid): rank by comparison
+  const int t = threadIdx.x;
+  if (cap + 2 > LO_KEYS) {  // long lists (same branch for the whole grid): rank by comparison
     sc[t] = c;
     __syncthreads();
     int rank = 0;
@@ -101,7 +98,7 @@ k_lane_order(const Replica* __restrict__ reps, const int* __restrict__ blk_rep, 
       const int cu = sc[u];
       rank += (cu > c || (cu == c && u < t)) ? 1 : 0;
     }
-    order[(size_t)b * BLOCK + rank] = (uint8_t)t;
+    order[rank] = (uint8_t)t;
     return;
   }
   // stable counting sort on key = count + 1 (padding 0), largest key first
@@ -128,7 +125,15 @@ k_lane_order(const Replica* __restrict__ reps, const int* __restrict__ blk_rep, 
   __syncthreads();
   int rank = sc[key] + below;
   for (int u = 0; u < w; u++) rank += hist[u][key];
-  order[(size_t)b * BLOCK + rank] = (uint8_t)t;
+  order[rank] = (uint8_t)t;
+}
+
+static __global__ void __launch_bounds__(BLOCK)
+k_lane_order(const Replica* __restrict__ reps, const int* __restrict__ blk_rep, NbList nl,
+             uint8_t* __restrict__ order, const int* __restrict__ blist = nullptr) {
+  const int b = blist ? blist[blockIdx.x] : (int)blockIdx.x, k = b * BLOCK + threadIdx.x;
+  const Replica& R = reps[blk_rep[b]];
+  lane_order_block((k - R.off < R.n) ? nl.cnt[k] : -1, nl.cap, order + (size_t)b * BLOCK);
 }
 
 // One neighbour's pair term of the specialised program: soft repulsion
@@ -193,32 +198,26 @@ __device__ __forceinline__ void abp_pair_term(const AbpParams& S, double x, doub
     }
 }
 
-// Integration tail of the specialised program: self-propulsion, the
-// Brownian update (integrator_brownian.cpp:57-121), enforce, torque
-// projection, rotation, skin test (neighbour_list.cpp:278-302), the next
-// step's enforce, and the stores.
+// Integration of the specialised program, in registers: self-propulsion, the
+// Brownian update (integrator_brownian.cpp:57-121), enforce, torque projection,
+// rotation, skin test (neighbour_list.cpp:278-302), the next step's enforce.
+// In: p's position, director, force and torque; g_*: the step's Gaussian draws,
+// flip: its nematic flip.  Out: p moved on (force and torque as integrated),
+// image flag changes; true when the particle has left its skin.
 template <int SHAPE, bool SP>
-__device__ __forceinline__ void abp_finish(const AbpParams& S, int r, int k, double x, double y, double z, double nx,
-                                           double ny, double nz, double ri, double fx, double fy, double fz, double tx,
-                                           double ty, double tz, double g_rot, double g_x, double g_y, double g_z,
-                                           double T, uint64_t gid, uint64_t s_base, double ox, double oy, double oz,
-                                           double age0, D4* __restrict__ Gout, D4* __restrict__ Hout, Dyn& d,
-                                           int* __restrict__ rebuild, int* __restrict__ status, int apply_e1,
-                                           int last) {
+__device__ __forceinline__ bool abp_advance(const AbpParams& S, Hp& p, double g_rot, double g_x, double g_y, double g_z,
+                                            double T, bool flip, double ox, double oy, double oz, int apply_e1,
+                                            int& dix, int& diy, bool& finite) {
   constexpr bool PLANE = SHAPE == HOT_PLANE;
-  if (SP) { fx += S.alpha * nx; fy += S.alpha * ny; if (!PLANE) fz += S.alpha * nz; }
+  if (SP) { p.fx += S.alpha * p.nx; p.fy += S.alpha * p.ny; if (!PLANE) p.fz += S.alpha * p.nz; }
 
   // ---- IntegratorBrownian::integrate (integrator_brownian.cpp:57-121) ----
-  Hp p;
-  p.x = x; p.y = y; p.z = z; p.nx = nx; p.ny = ny; p.nz = nz;
   p.vx = 0.0; p.vy = 0.0; p.vz = 0.0;
-  if (S.nematic) {
-    // the velocity flip of velocity_align is overwritten below (v = fd)
-    if (noise_uniform(S.seed, s_base + gid) < S.flip) { p.nx = -p.nx; p.ny = -p.ny; p.nz = -p.nz; }
-  }
-  double fd_x = S.v0 * p.nx + S.mu * fx;
-  double fd_y = S.v0 * p.ny + S.mu * fy;
-  double fd_z = S.v0 * p.nz + S.mu * fz;
+  // the velocity flip of velocity_align is overwritten below (v = fd)
+  if (flip) { p.nx = -p.nx; p.ny = -p.ny; p.nz = -p.nz; }
+  double fd_x = S.v0 * p.nx + S.mu * p.fx;
+  double fd_y = S.v0 * p.ny + S.mu * p.fy;
+  double fd_z = S.v0 * p.nz + S.mu * p.fz;
   p.vx = fd_x; p.vy = fd_y; p.vz = fd_z;
   p.x += S.dt * fd_x; p.y += S.dt * fd_y;
   if (!PLANE) p.z += S.dt * fd_z;
@@ -229,31 +228,47 @@ __device__ __forceinline__ void abp_finish(const AbpParams& S, int r, int k, dou
     p.x += sqrt_dt * fr_x; p.y += sqrt_dt * fr_y;
     if (!PLANE) { const double fr_z = B * g_z; p.vz += fr_z; p.z += sqrt_dt * fr_z; }
   }
-  int dix = 0, diy = 0;
+  dix = 0; diy = 0;
   const ShapeGeom Rb{S.xlo, S.xhi, S.Lx, S.ylo, S.yhi, S.Ly, S.Rs};
   hot_enforce<SHAPE>(Rb, p, dix, diy);
   if (PLANE) p.vz = 0.0;
-  p.tx = tx; p.ty = ty; p.tz = tz;
   p.omega = S.mur * hot_project_torque<SHAPE>(Rb, p);
   const double dtheta = S.dt * p.omega + S.stoch * g_rot;
   hot_rotate<SHAPE>(Rb, p, dtheta, S.velocity != 0);
-  const double age = age0 + S.dt;
 
   // ---- skin test, NeighbourList::need_update (neighbour_list.cpp:278-302)
-  {
-    double ddx = ox - p.x, ddy = oy - p.y, ddz = PLANE ? 0.0 : oz - p.z;
-    if (S.periodic) {
-      if (ddx > S.xhi) ddx -= S.Lx; else if (ddx < S.xlo) ddx += S.Lx;
-      if (ddy > S.yhi) ddy -= S.Ly; else if (ddy < S.ylo) ddy += S.Ly;
-      if (!PLANE) { if (ddz > S.zhi) ddz -= S.Lz; else if (ddz < S.zlo) ddz += S.Lz; }
-    }
-    const double d2 = PLANE ? ddx * ddx + ddy * ddy : ddx * ddx + ddy * ddy + ddz * ddz;
-    if (!(d2 < S.pad2q)) {
-      if (rebuild[r] == 0) atomicOr(&rebuild[r], 1);
-    }
+  double ddx = ox - p.x, ddy = oy - p.y, ddz = PLANE ? 0.0 : oz - p.z;
+  if (S.periodic) {
+    if (ddx > S.xhi) ddx -= S.Lx; else if (ddx < S.xlo) ddx += S.Lx;
+    if (ddy > S.yhi) ddy -= S.Ly; else if (ddy < S.ylo) ddy += S.Ly;
+    if (!PLANE) { if (ddz > S.zhi) ddz -= S.Lz; else if (ddz < S.zlo) ddz += S.Lz; }
   }
-  if (!(isfinite(p.x) && isfinite(p.y) && isfinite(p.z))) atomicOr(status, ST_NONFINITE);
+  const double d2 = PLANE ? ddx * ddx + ddy * ddy : ddx * ddx + ddy * ddy + ddz * ddz;
+  finite = isfinite(p.x) && isfinite(p.y) && isfinite(p.z);
   if (apply_e1) hot_enforce<SHAPE>(Rb, p, dix, diy);
+  return !(d2 < S.pad2q);
+}
+
+// abp_advance with the stores of a step kernel.
+template <int SHAPE, bool SP>
+__device__ __forceinline__ void abp_finish(const AbpParams& S, int r, int k, double x, double y, double z, double nx,
+                                           double ny, double nz, double ri, double fx, double fy, double fz, double tx,
+                                           double ty, double tz, double g_rot, double g_x, double g_y, double g_z,
+                                           double T, uint64_t gid, uint64_t s_base, double ox, double oy, double oz,
+                                           double age0, D4* __restrict__ Gout, D4* __restrict__ Hout, Dyn& d,
+                                           int* __restrict__ rebuild, int* __restrict__ status, int apply_e1,
+                                           int last) {
+  constexpr bool PLANE = SHAPE == HOT_PLANE;
+  Hp p;
+  p.x = x; p.y = y; p.z = z; p.nx = nx; p.ny = ny; p.nz = nz;
+  p.fx = fx; p.fy = fy; p.fz = fz; p.tx = tx; p.ty = ty; p.tz = tz;
+  const bool flip = S.nematic && noise_uniform(S.seed, s_base + gid) < S.flip;
+  int dix, diy;
+  bool finite;
+  if (abp_advance<SHAPE, SP>(S, p, g_rot, g_x, g_y, g_z, T, flip, ox, oy, oz, apply_e1, dix, diy, finite))
+    if (rebuild[r] == 0) atomicOr(&rebuild[r], 1);
+  if (!finite) atomicOr(status, ST_NONFINITE);
+  const double age = age0 + S.dt;
 
   // ---- stores ---------------------------------------------------------------
   if (PLANE) {
@@ -269,7 +284,7 @@ __device__ __forceinline__ void abp_finish(const AbpParams& S, int r, int k, dou
   if (diy) d.iy[k] += diy;
   if (last) {
     d.omega[k] = p.omega;
-    d.fx[k] = fx; d.fy[k] = fy; d.fz[k] = PLANE ? 0.0 : fz;
+    d.fx[k] = p.fx; d.fy[k] = p.fy; d.fz[k] = PLANE ? 0.0 : p.fz;
     d.tx[k] = tx; d.ty[k] = ty; d.tz[k] = tz;
   }
 }

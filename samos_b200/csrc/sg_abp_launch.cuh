@@ -2,6 +2,7 @@
 // one shape and aligner, instantiated by the sg_abp_*.cu units.
 #pragma once
 #include "sg_abp_launch.h"
+#include "sg_abp_run.cuh"
 
 namespace sg {
 
@@ -102,6 +103,24 @@ template <int SHAPE, int ALIGN>
 static void launch_abp_unit(const AbpLaunch& L) {
   if (L.self_propulsion) launch_abp3<SHAPE, ALIGN, true>(L);
   else launch_abp3<SHAPE, ALIGN, false>(L);
+}
+
+template <int SHAPE, int ALIGN, bool SP, bool BYVAL>
+static cudaError_t launch_abp_run(const AbpRunLaunch* L, int* blocks_per_sm) {
+  const void* f = (const void*)k_abp_run<SHAPE, ALIGN, SP, BYVAL>;
+  if (!L) return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, f, BLOCK, 0);
+  AbpRunLaunch A = *L;
+  void* args[] = {&A.abp, &A.abp0, &A.blk_rep, &A.G0, &A.G1, &A.H0, &A.H1, &A.rb, &A.word, &A.nsteps, &A.sort_every};
+  return cudaLaunchCooperativeKernel(f, dim3(A.nblocks), dim3(BLOCK), args, 0, A.stream);
+}
+template <int SHAPE, int ALIGN>
+static cudaError_t launch_abp_run_unit(const AbpRunLaunch* L, int* blocks_per_sm) {
+  if (!L) return launch_abp_run<SHAPE, ALIGN, true, false>(L, blocks_per_sm);
+  if (L->nrep == 1)
+    return L->self_propulsion ? launch_abp_run<SHAPE, ALIGN, true, true>(L, nullptr)
+                              : launch_abp_run<SHAPE, ALIGN, false, true>(L, nullptr);
+  return L->self_propulsion ? launch_abp_run<SHAPE, ALIGN, true, false>(L, nullptr)
+                            : launch_abp_run<SHAPE, ALIGN, false, false>(L, nullptr);
 }
 
 }  // namespace sg

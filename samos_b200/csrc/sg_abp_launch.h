@@ -2,7 +2,7 @@
 // kernels.  Each shape / aligner pair is compiled in a unit of its own
 // (sg_abp_*.cu), so the kernel variants build side by side.
 #pragma once
-#include "sg_abp.cuh"
+#include "sg_rebuild.cuh"
 
 namespace sg {
 
@@ -34,5 +34,25 @@ void launch_abp_plane_nematic(const AbpLaunch& L);
 void launch_abp_sphere_none(const AbpLaunch& L);
 void launch_abp_sphere_polar(const AbpLaunch& L);
 void launch_abp_sphere_nematic(const AbpLaunch& L);
+
+// Many steps in one cooperative launch (k_abp_run).
+struct AbpRunLaunch {
+  const AbpParams* abp;
+  AbpParams abp0;
+  const int* blk_rep;
+  D4 *G0, *G1, *H0, *H1;  // state in G0 / H0
+  RebuildArgs rb;
+  unsigned long long* word;  // step barrier, two words, 0 between launches
+  int nsteps, sort_every, nblocks, nrep;
+  bool self_propulsion;
+  cudaStream_t stream;
+};
+// *blocks_per_sm set, nothing launched, when L is null
+cudaError_t launch_abp_run_plane_none(const AbpRunLaunch* L, int* blocks_per_sm);
+cudaError_t launch_abp_run_plane_polar(const AbpRunLaunch* L, int* blocks_per_sm);
+cudaError_t launch_abp_run_plane_nematic(const AbpRunLaunch* L, int* blocks_per_sm);
+cudaError_t launch_abp_run_sphere_none(const AbpRunLaunch* L, int* blocks_per_sm);
+cudaError_t launch_abp_run_sphere_polar(const AbpRunLaunch* L, int* blocks_per_sm);
+cudaError_t launch_abp_run_sphere_nematic(const AbpRunLaunch* L, int* blocks_per_sm);
 
 }  // namespace sg

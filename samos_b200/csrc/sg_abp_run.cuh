@@ -1,0 +1,230 @@
+// sg_abp_run.cuh -- many steps of the specialised active-Brownian program in
+// one cooperative launch, for systems whose blocks are all resident at once.
+//
+// A small system's step is latency: at 2,000 disks the step kernel runs 16
+// blocks for 6.5 us and the launch, the tail and the gaps around them cost
+// another 10.  Here each block keeps its 128 particles for the whole launch:
+// state in registers, list entries and neighbour radii in shared memory, only
+// the packed records go through L2, and a step ends in one grid barrier, with
+// the next step's noise drawn while the block waits.  A rebuild runs inside the
+// launch (rebuild_phases).  The terms are abp_pair_term and abp_advance, in the
+// step kernels' order: same bits.
+#pragma once
+#include "sg_abp_launch.h"
+
+namespace sg {
+
+// blocks per SM that the registers are bounded for: with 4 (128 registers) all
+// of a step's neighbour records are in flight at once
+constexpr int ABP_RUN_MINB = 4;
+// entries per particle kept in shared memory; longer lists read the rest from
+// the list itself
+constexpr int RUN_NB = 16;
+
+// Arrival of one block at the step barrier: a word for even and one for odd
+// steps, arrivals in the low half and blocks that ask for a rebuild in the high
+// half.  A block that is one step ahead writes the other word, so every block
+// of a step reads the same requests.
+__device__ __forceinline__ unsigned long long ld_acquire64(const unsigned long long* p) {
+  unsigned long long v;
+  asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+  return v;
+}
+
+template <int SHAPE, int ALIGN, bool SP, bool BYVAL>
+__global__ void __launch_bounds__(BLOCK, ABP_RUN_MINB)
+k_abp_run(const AbpParams* __restrict__ prm, const __grid_constant__ AbpParams pv, const int* __restrict__ blk_rep,
+          D4* G0, D4* G1, D4* H0, D4* H1, RebuildArgs A, unsigned long long* word, int nsteps, int sort_every) {
+  constexpr bool PLANE = SHAPE == HOT_PLANE;
+  constexpr int CH = PLANE ? 8 : 4;  // neighbour records requested together
+  __shared__ RebuildList L;
+  __shared__ AbpParams S_sh;
+  __shared__ int nbs[RUN_NB][BLOCK];
+  __shared__ double rbs[PLANE ? RUN_NB : 1][BLOCK];
+  __shared__ uint8_t order[BLOCK];
+  __shared__ unsigned long long seen;
+  __shared__ uint64_t s_ctr;
+  const int t = threadIdx.x;
+  const int r = BYVAL ? 0 : blk_rep[blockIdx.x];
+  if (!BYVAL) {
+    constexpr int NW = (int)(sizeof(AbpParams) / 8);
+    if (t < NW)
+      reinterpret_cast<unsigned long long*>(&S_sh)[t] = reinterpret_cast<const unsigned long long*>(prm + r)[t];
+  }
+  if (t == 0) s_ctr = A.clk[r].ctr[0];
+  __syncthreads();
+  const AbpParams& S = abp_params<BYVAL>(pv, S_sh);
+  const double T = S.temp.min_val;  // a constant temperature (checked by the host)
+  const int D = T > 0.0 ? 4 : 1;
+  const uint64_t draws = (uint64_t)S.n * (uint64_t)((S.nematic ? 1 : 0) + D);
+  uint64_t base = s_ctr;
+
+  GridBar bar{A.bar, 0u, A.status};
+  unsigned long long asked[2] = {0ull, 0ull};
+  unsigned target[2] = {0u, 0u};
+
+  // this thread's particle: slot k, its constants between rebuilds, its state
+  int k = 0, cnt = 0, lo = 0, dix_sum = 0, diy_sum = 0;
+  bool mine = false;
+  uint64_t gid = 0;
+  double ri = 1.0, ox = 0.0, oy = 0.0, oz = 0.0, age = 0.0;
+  Hp p;
+  p.x = p.y = p.z = p.nx = p.ny = p.nz = p.vx = p.vy = p.vz = 0.0;
+  double g_rot = 0.0, g_x = 0.0, g_y = 0.0, g_z = 0.0;
+  bool flip = false;
+  D4 *Gin = G0, *Gout = G1, *Hin = H0, *Hout = H1;
+
+  auto draw = [&]() {  // the noise of the step whose counters start at `base`
+    const uint64_t c0 = base + (S.nematic ? (uint64_t)S.n : 0ull) + gid * (uint64_t)D;
+    g_rot = noise_gauss(S.seed, c0 + (uint64_t)(D - 1));
+    if (T > 0.0) {
+      g_x = noise_gauss(S.seed, c0 + 0);
+      g_y = noise_gauss(S.seed, c0 + 1);
+      if (!PLANE) g_z = noise_gauss(S.seed, c0 + 2);
+    }
+    flip = S.nematic && noise_uniform(S.seed, base + gid) < S.flip;
+  };
+  auto load = [&](bool state) {  // particle, lists (and state) from memory
+    const int k0 = blockIdx.x * BLOCK;
+    const bool in = k0 + t - S.off < S.n;
+    lane_order_block(in ? A.nl.cnt[k0 + t] : -1, A.nl.cap, order);
+    __syncthreads();
+    k = k0 + order[t];
+    mine = k - S.off < S.n;
+    cnt = 0;
+    if (mine) {
+      cnt = A.nl.cnt[k]; lo = A.nl.lo[k];
+      gid = (uint64_t)A.st.id[k];
+      ri = A.st.r[k];
+      ox = A.nl.ox[k]; oy = A.nl.oy[k]; oz = PLANE ? 0.0 : A.nl.oz[k];
+      for (int q = 0; q < min(cnt, RUN_NB); q++) {
+        const int j = A.nl.nb[(size_t)q * A.nl.stride + k];
+        nbs[q][t] = j;
+        if (PLANE) rbs[q][t] = S.use_radii ? A.st.r[j] : 1.0;
+      }
+      if (state) {
+        const D4 g = ld4(Gin + k);
+        p.x = g.x; p.y = g.y;
+        if (PLANE) { p.z = 0.0; p.nx = g.z; p.ny = g.w; p.nz = 0.0; }
+        else { const D4 h = ld4(Hin + k); p.z = g.z; p.nx = h.x; p.ny = h.y; p.nz = h.z; }
+        age = A.cur.age[k];
+        dix_sum = 0; diy_sum = 0;
+        p.vx = A.cur.vx[k]; p.vy = A.cur.vy[k]; p.vz = A.cur.vz[k];
+      }
+    }
+  };
+  auto store = [&]() {  // what the packed records do not hold
+    if (!mine) return;
+    A.cur.vx[k] = p.vx; A.cur.vy[k] = p.vy;
+    if (!PLANE) A.cur.vz[k] = p.vz;
+    A.cur.age[k] = age;
+    if (dix_sum) A.cur.ix[k] += dix_sum;
+    if (diy_sum) A.cur.iy[k] += diy_sum;
+  };
+
+  load(true);
+  if (mine) draw();
+  int done = 0;
+  bool over = false;
+  for (int step = 0; step < nsteps; step++) {
+    // ---- forces and torques ------------------------------------------------
+    double fx = 0.0, fy = 0.0, fz = 0.0, tx = 0.0, ty = 0.0, tz = 0.0, e0 = 0.0, e1 = 0.0;
+    for (int q0 = 0; q0 < cnt; q0 += CH) {
+      D4 gg[CH], hh[CH];
+      double rr[CH];
+      int jj[CH];
+#pragma unroll
+      for (int u = 0; u < CH; u++) {
+        const int q = q0 + u;
+        jj[u] = k;
+        if (q < cnt) jj[u] = q < RUN_NB ? nbs[q][t] : A.nl.nb[(size_t)q * A.nl.stride + k];
+        if (PLANE && q < cnt) rr[u] = q < RUN_NB ? rbs[q][t] : (S.use_radii ? A.st.r[jj[u]] : 1.0);
+      }
+#pragma unroll
+      for (int u = 0; u < CH; u++)
+        if (q0 + u < cnt) {
+          gg[u] = ld4(Gin + jj[u]);
+          if (!PLANE && ALIGN != ABP_ALIGN_NONE) hh[u] = ld4(Hin + jj[u]);
+        }
+#pragma unroll
+      for (int u = 0; u < CH; u++)
+        if (q0 + u < cnt)
+          abp_pair_term<SHAPE, ALIGN, false>(S, p.x, p.y, p.z, p.nx, p.ny, p.nz, ri, gg[u], hh[u],
+                                             PLANE ? rr[u] : gg[u].w, false, fx, fy, fz, tx, ty, tz, e0, e1);
+    }
+    bool ask = false;
+    if (mine) {
+      p.fx = fx; p.fy = fy; p.fz = fz; p.tx = tx; p.ty = ty; p.tz = tz;
+      int dix, diy;
+      bool finite;
+      if (abp_advance<SHAPE, SP>(S, p, g_rot, g_x, g_y, g_z, T, flip, ox, oy, oz, 1, dix, diy, finite)) ask = true;
+      if (!finite) atomicOr(A.status, ST_NONFINITE);
+      age = age + S.dt;
+      dix_sum += dix; diy_sum += diy;
+      if (PLANE) stg4(Gout + k, D4{p.x, p.y, p.nx, p.ny});
+      else {
+        stg4(Gout + k, D4{p.x, p.y, p.z, ri});
+        stg4(Hout + k, D4{p.nx, p.ny, p.nz, 0.0});
+      }
+    }
+    base += draws;
+    // ---- step barrier: arrive, draw the next step's noise, wait ----------------
+    const int w = step & 1;
+    const bool block_asks = __syncthreads_or(ask) != 0;
+    target[w] += gridDim.x;
+    if (t == 0) {
+      if (block_asks) atomicOr(&A.rebuild[r], 1);
+      __threadfence();
+      atomicAdd(word + w, 1ull + (block_asks ? 1ull << 32 : 0ull));
+    }
+    if (mine && step + 1 < nsteps) draw();
+    int ok = 1;
+    if (t == 0) {
+      unsigned long long v = ld_acquire64(word + w);
+      for (unsigned it = 0; (unsigned)v < target[w]; v = ld_acquire64(word + w))
+        if (++it >= GRID_SPIN_LIMIT) { atomicOr(A.status, ST_TIMEOUT); ok = 0; break; }
+      __threadfence();
+      seen = v;
+    }
+    if (!__syncthreads_and(ok)) return;
+    { D4* x = Gin; Gin = Gout; Gout = x; x = Hin; Hin = Hout; Hout = x; }
+    done = step + 1;
+    if ((unsigned)(seen >> 32) != (unsigned)asked[w]) {  // the same for every block
+      asked[w] = seen >> 32;
+      const unsigned long long t0 = global_ns();
+      store();
+      RebuildArgs B = A;
+      B.G = Gin; B.H = Hin;
+      if (!grid_wait(bar)) return;  // the stores before a re-sort reads them
+      rebuild_list(B, sort_every, L);
+      if (!rebuild_phases<SHAPE>(B, L, bar)) return;
+      if (blockIdx.x == 0)  // every block has read the flags and counts
+        for (int s = t; s < L.n; s += BLOCK) { A.rebuild[L.rep[s]] = 0; A.builds[L.rep[s]]++; }
+      if (!grid_wait(bar)) return;
+      over = (__ldcg(A.bstatus) & ST_OVERFLOW) != 0;
+      if (blockIdx.x == 0 && t == 0) { A.stats->builds++; A.stats->ns += global_ns() - t0; }
+      if (over) break;
+      load(true);
+      if (mine && step + 1 < nsteps) draw();  // a re-sort has changed the thread's particle
+    }
+  }
+  if (!over) store();
+  if (grid_last(bar)) {
+    if (t == 0) { word[0] = 0ull; word[1] = 0ull; *A.executed = done; }
+    for (int q = t; q < A.nrep; q += BLOCK) {
+      Clock& C = A.clk[q];
+      const AbpParams& Q = prm[q];
+      C.ctr[0] += (uint64_t)done * ((uint64_t)Q.n * (uint64_t)((Q.nematic ? 1 : 0) + (Q.temp.min_val > 0.0 ? 4 : 1)));
+      C.run_step += done;
+      C.time_step += done;
+      if (over) C.halt = 1;
+    }
+    if (over) {  // the lists did not fit: the host grows them and rebuilds these
+      __syncthreads();
+      for (int s = t; s < L.n; s += BLOCK) { A.rebuild[L.rep[s]] = 1; A.builds[L.rep[s]]--; }
+      if (t == 0) A.stats->builds--;
+    }
+  }
+}
+
+}  // namespace sg

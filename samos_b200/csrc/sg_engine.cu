@@ -3,6 +3,7 @@
 // once per configuration and reused by every step.
 #include "samos_gpu.h"
 #include "sg_abp_launch.h"
+#include "sg_rebuild.cuh"
 
 #include <algorithm>
 #include <cmath>
@@ -42,13 +43,26 @@ const int kNumDynDouble = 17;
 }  // namespace
 
 struct sg_system {
-  int device = 0;
+  int device = 0, sms = 0;
   int nrep = 0, ntypes = 1;
   std::vector<int> n, off;
   int slots = 0, nblocks = 0;
   int* blk_rep = nullptr;
   std::vector<int> blk_rep_h, rep_blk0_h, rep_nblk_h;
-  std::vector<int64_t> rep_builds;  // neighbour-list builds per replica
+  // neighbour-list builds per replica (every kSortEvery-th re-sorts): counted
+  // by whoever rebuilds, the host or the device; the other's copy is brought
+  // up to date when it is needed
+  std::vector<int> rep_builds;
+  int* rep_builds_d = nullptr;
+  bool builds_host_new = true, builds_dev_new = false;
+  // rebuilds enqueued with the steps (k_tail_rebuild)
+  RebuildStats* rb_stats = nullptr;
+  unsigned* rb_bar = nullptr;
+  int* rb_bsum = nullptr;
+  unsigned long long* run_word = nullptr;  // step barrier of the resident run
+  int run_per_sm = 0, run_kind = -1;       // its blocks per SM, and for which kernel
+  int rb_grid[3] = {0, 0, 0};  // blocks that fit the device at once, per shape
+  bool rb_used = false;        // in the current run
   int *rep_blk0 = nullptr, *rep_nblk = nullptr;
   std::vector<Replica> reps_h;
   Replica* reps = nullptr;
@@ -151,7 +165,7 @@ struct sg_system {
   int gen_n[2] = {0, 0};
   // autotuner: every variant yields the same bits, so candidates are timed on
   // the run's own first steps (CUDA events around the step kernel)
-  bool tuned = false;
+  bool tuned = false, pinned = false;
   int tune_trial = 0;
   double tune_ms[ABP_NVARIANT] = {0};
   int tune_n[ABP_NVARIANT] = {0};
@@ -249,6 +263,7 @@ int sg_create(int n_replicas, const int32_t* n_particles, int ntypes, sg_system*
   if (cudaGetDeviceCount(&dev_count) != cudaSuccess || dev_count == 0) return SG_ERR_CUDA;
   sg_system* s = new sg_system();
   cudaGetDevice(&s->device);
+  cudaDeviceGetAttribute(&s->sms, cudaDevAttrMultiProcessorCount, s->device);
   s->nrep = n_replicas;
   s->ntypes = ntypes;
   s->n.assign(n_particles, n_particles + n_replicas);
@@ -737,8 +752,17 @@ static int prepare_tiles(sg_system* s) {
   return SG_OK;
 }
 
+static int builds_to_host(sg_system* s) {
+  if (!s->builds_dev_new) return SG_OK;
+  CU(s, cudaMemcpyAsync(s->rep_builds.data(), s->rep_builds_d, sizeof(int) * s->nrep, cudaMemcpyDeviceToHost, s->stream));
+  CU(s, cudaStreamSynchronize(s->stream));
+  s->builds_dev_new = false;
+  return SG_OK;
+}
+
 static int rebuild_flagged(sg_system* s, bool* sorted, bool blist_ready = false) {
   s->forces_fresh = false;
+  if (int rcb = builds_to_host(s)) return rcb;
   bool any_sort = false;
   for (int r = 0; r < s->nrep; r++) {
     if (!s->rebuild_h[r]) continue;
@@ -851,6 +875,7 @@ static int rebuild_flagged(sg_system* s, bool* sorted, bool blist_ready = false)
       s->maxnb_seen = std::max(s->maxnb_seen, mx);
       for (int r = 0; r < s->nrep; r++)
         if (s->rebuild_h[r]) s->rep_builds[r]++;
+      s->builds_host_new = true;
       return SG_OK;
     }
     if (any_sort) {  // arrays are now sorted: retry as list-only rebuilds of the same replicas
@@ -1838,6 +1863,78 @@ static int rebuild_pending(sg_system* s, int shape, bool last, double* rebuild_m
   return SG_OK;
 }
 
+// Rebuilds enqueued with the steps: taken up to kDevRebuildSlots slots.  Above
+// that a step outlasts the host's round trip by far, and the separate kernels
+// of rebuild_flagged run each phase at its own occupancy.
+static constexpr int kDevRebuildSlots = 5 << 20;
+
+static bool dev_rebuild(const sg_system* s) {
+  return s->has_nlist && s->nrep <= RB_MAX_REP && s->slots <= kDevRebuildSlots && s->build_mode <= 1 && !s->profile &&
+         !(s->abp_on && s->abp_variant == 8);
+}
+
+static int dev_rebuild_ready(sg_system* s) {
+  if (!s->rb_bar) {
+    s->rep_builds_d = s->mem.alloc<int>(s->nrep);
+    s->rb_stats = s->mem.alloc<RebuildStats>(1);
+    s->rb_bar = s->mem.alloc<unsigned>(2);
+    s->run_word = s->mem.alloc<unsigned long long>(2);
+    s->rb_bsum = s->mem.alloc<int>(148 * 16);
+    if (s->mem.err != cudaSuccess) { s->mem.err = cudaSuccess; return fail(s, SG_ERR_NOMEM, "rebuild state"); }
+    const void* k[3] = {(const void*)k_tail_rebuild<HOT_NONE>, (const void*)k_tail_rebuild<HOT_PLANE>,
+                        (const void*)k_tail_rebuild<HOT_SPHERE>};
+    for (int i = 0; i < 3; i++) {
+      int per = 0;
+      CU(s, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k[i], BLOCK, 0));
+      s->rb_grid[i] = std::min(148 * 16, std::max(1, per) * s->sms);
+    }
+  }
+  if (s->builds_host_new) {
+    CU(s, cudaMemcpyAsync(s->rep_builds_d, s->rep_builds.data(), sizeof(int) * s->nrep, cudaMemcpyHostToDevice, s->stream));
+    s->builds_host_new = false;
+  }
+  if (!s->rb_used) {
+    CU(s, cudaMemsetAsync(s->rb_stats, 0, sizeof(RebuildStats), s->stream));
+    s->rb_used = true;
+  }
+  s->builds_dev_new = true;
+  return SG_OK;
+}
+
+static RebuildArgs rebuild_args(sg_system* s, int shape) {
+  RebuildArgs A{};
+  A.reps = s->reps; A.rep_blk0 = s->rep_blk0; A.rep_nblk = s->rep_nblk; A.nrep = s->nrep;
+  A.clk = s->clk; A.rebuild = s->rebuild; A.builds = s->rep_builds_d;
+  A.cur = s->cur; A.alt = s->alt; A.st = s->st; A.st_alt = s->st_alt; A.nl = s->nl;
+  A.G = shape == HOT_NONE ? nullptr : s->G[s->hot_buf];
+  A.H = shape == HOT_NONE ? nullptr : s->H[s->hot_buf];
+  A.pcell = s->pcell; A.cell_cnt = s->cell_cnt; A.cell_start = s->cell_start; A.cell_fill = s->cell_fill;
+  A.tmp = s->tmp; A.perm = s->perm; A.bsum = s->rb_bsum; A.cand = s->cand;
+  A.lane_order = s->order_valid ? s->lane_order : nullptr;
+  A.bstatus = s->bstatus; A.stats = s->rb_stats; A.bar = s->rb_bar; A.status = s->status; A.executed = s->exec_cnt;
+  return A;
+}
+
+// a grid barrier's bounded wait ran out: its words are put back, the run fails
+static int grid_timeout(sg_system* s) {
+  cudaMemsetAsync(s->rb_bar, 0, 2 * sizeof(unsigned), s->stream);
+  cudaMemsetAsync(s->run_word, 0, 2 * sizeof(unsigned long long), s->stream);
+  return fail(s, SG_ERR_TIMEOUT, "a grid barrier gave up");
+}
+
+// the end of the step just enqueued: counters, and the lists that it flagged
+static int tail_rebuild(sg_system* s, int shape) {
+  RebuildArgs A = rebuild_args(s, shape);
+  int every = kSortEvery;
+  void* args[] = {&s->prog, &A, &every};
+  const void* k = shape == HOT_NONE ? (const void*)k_tail_rebuild<HOT_NONE>
+                  : shape == HOT_PLANE ? (const void*)k_tail_rebuild<HOT_PLANE> : (const void*)k_tail_rebuild<HOT_SPHERE>;
+  CU(s, cudaLaunchCooperativeKernel(k, dim3(std::min(s->rb_grid[shape], std::max(1, s->nblocks))), dim3(BLOCK), args, 0,
+                                    s->stream));
+  s->launches++;
+  return SG_OK;
+}
+
 // K non-final steps on the packed path, enqueued without waiting (the caller
 // keeps K at or below half the last gap between rebuilds, since a longer
 // batch would mostly enqueue halted launches, and steps one at a time when
@@ -1846,16 +1943,23 @@ static int rebuild_pending(sg_system* s, int shape, bool last, double* rebuild_m
 // rebuild (Clock::halt, set by k_tail_batch), so the host learns after the
 // batch how many steps ran, puts the double-buffer index right, rebuilds and
 // goes on from there.  Results are those of stepping one at a time.
-static constexpr int64_t kBatch = 32;
+static constexpr int64_t kBatch = 32, kBatchDev = 512, kResidentSteps = 2048;
 
 static int run_batch(sg_system* s, int shape, int64_t K, bool needs_nl, int64_t* executed, double* rebuild_ms) {
   const int b0 = s->hot_buf;
   CU(s, cudaMemsetAsync(s->exec_cnt, 0, sizeof(int), s->stream));
+  const bool dev = needs_nl && dev_rebuild(s);
+  if (dev)
+    if (int rcd = dev_rebuild_ready(s)) return rcd;
   for (int64_t i = 0; i < K; i++) {
     int rc = step_hot(s, shape, true, false, false);
     if (rc) return rc;
-    k_tail_batch<<<1, 256, 0, s->stream>>>(s->prog, s->reps, s->clk, s->nrep, s->rebuild, s->exec_cnt);
-    LAUNCH_CHECK(s);
+    if (dev) {
+      if ((rc = tail_rebuild(s, shape))) return rc;
+    } else {
+      k_tail_batch<<<1, 256, 0, s->stream>>>(s->prog, s->reps, s->clk, s->nrep, s->rebuild, s->exec_cnt);
+      LAUNCH_CHECK(s);
+    }
   }
   int ex = 0;
   CU(s, cudaMemcpyAsync(&ex, s->exec_cnt, sizeof(int), cudaMemcpyDeviceToHost, s->stream));
@@ -1876,6 +1980,63 @@ static int run_batch(sg_system* s, int shape, int64_t K, bool needs_nl, int64_t*
   return rebuild_pending(s, shape, false, rebuild_ms);
 }
 
+// Resident runs (k_abp_run): the whole system on the device at once, steps and
+// rebuilds in one launch.  For every specialised program whose temperatures are
+// constant (the noise counters then advance by a fixed number a step), unless a
+// step kernel was pinned.
+static cudaError_t abp_run(const sg_system* s, int shape, const AbpRunLaunch* L, int* per_sm) {
+  const Program& P = s->prog;
+  const int al = P.nalign == 0 ? ABP_ALIGN_NONE : P.align[0].kind;
+  if (shape == HOT_PLANE)
+    return al == ABP_ALIGN_NONE ? launch_abp_run_plane_none(L, per_sm)
+           : al == ALIGN_POLAR  ? launch_abp_run_plane_polar(L, per_sm) : launch_abp_run_plane_nematic(L, per_sm);
+  return al == ABP_ALIGN_NONE ? launch_abp_run_sphere_none(L, per_sm)
+         : al == ALIGN_POLAR  ? launch_abp_run_sphere_polar(L, per_sm) : launch_abp_run_sphere_nematic(L, per_sm);
+}
+
+static bool resident_run(sg_system* s, int shape) {
+  if (!s->abp_on || !s->tuned || s->pinned || !dev_rebuild(s) || s->prog.integ[0].temp.kind != 0) return false;
+  const int kind = shape * 8 + (s->prog.nalign ? 1 + s->prog.align[0].kind : 0);
+  if (s->run_kind != kind) {
+    int per = 0;
+    if (abp_run(s, shape, nullptr, &per) != cudaSuccess) { cudaGetLastError(); per = 0; }
+    s->run_per_sm = per;
+    s->run_kind = kind;
+  }
+  return s->nblocks <= s->run_per_sm * s->sms;
+}
+
+static int run_resident(sg_system* s, int shape, int64_t K, int64_t* executed, double* rebuild_ms) {
+  int rc = dev_rebuild_ready(s);
+  if (rc) return rc;
+  const int b = s->hot_buf;
+  AbpRunLaunch L{};
+  L.abp = s->abp; L.abp0 = s->abp0_h; L.blk_rep = s->blk_rep;
+  L.G0 = s->G[b]; L.G1 = s->G[1 - b]; L.H0 = s->H[b]; L.H1 = s->H[1 - b];
+  L.rb = rebuild_args(s, shape);
+  L.word = s->run_word; L.nsteps = (int)K; L.sort_every = kSortEvery;
+  L.nblocks = s->nblocks; L.nrep = s->nrep; L.self_propulsion = s->prog.next == 1; L.stream = s->stream;
+  CU(s, abp_run(s, shape, &L, nullptr));
+  s->launches++;
+  int ex = 0, st = 0;
+  CU(s, cudaMemcpyAsync(&ex, s->exec_cnt, sizeof(int), cudaMemcpyDeviceToHost, s->stream));
+  CU(s, cudaMemcpyAsync(&st, s->status, sizeof(int), cudaMemcpyDeviceToHost, s->stream));
+  CU(s, cudaMemcpyAsync(s->rebuild_h, s->rebuild, sizeof(int) * s->nrep, cudaMemcpyDeviceToHost, s->stream));
+  CU(s, cudaStreamSynchronize(s->stream));
+  if (st & ST_TIMEOUT) return grid_timeout(s);
+  if (ex < 1 || ex > K) return fail(s, SG_ERR_CUDA, "resident run: inconsistent step count");
+  s->hot_buf = b ^ (int)(ex & 1);
+  s->e1_applied = true;
+  *executed = ex;
+  s->since_rebuild += ex;
+  bool any = false;
+  for (int r = 0; r < s->nrep; r++) any = any || s->rebuild_h[r];
+  if (!any) return SG_OK;
+  k_set_halt<<<(s->nrep + 127) / 128, 128, 0, s->stream>>>(s->clk, s->nrep, 0);
+  LAUNCH_CHECK(s);
+  return rebuild_pending(s, shape, false, rebuild_ms);
+}
+
 // The generic fused step (k_step_brownian), K steps enqueued without a host
 // round trip like run_batch: the halted steps' kernels return at once and
 // write nothing, so the buffer holding the state is the one after the
@@ -1883,6 +2044,9 @@ static int run_batch(sg_system* s, int shape, int64_t K, bool needs_nl, int64_t*
 // the swaps of the halted ones.
 static int run_batch_generic(sg_system* s, int64_t K, bool needs_nl, int64_t* executed, double* rebuild_ms) {
   CU(s, cudaMemsetAsync(s->exec_cnt, 0, sizeof(int), s->stream));
+  const bool dev = needs_nl && dev_rebuild(s);
+  if (dev)
+    if (int rcd = dev_rebuild_ready(s)) return rcd;
   if (!s->e1_applied) {  // the first step's start-of-step enforce (samos.cpp:887-888)
     k_enforce<<<s->nblocks, BLOCK, 0, s->stream>>>(s->prog, s->reps, s->blk_rep, s->cur, s->st, nullptr);
     LAUNCH_CHECK(s);
@@ -1890,8 +2054,12 @@ static int run_batch_generic(sg_system* s, int64_t K, bool needs_nl, int64_t* ex
   for (int64_t i = 0; i < K; i++) {
     int rc = step_fused(s, true, false);
     if (rc) return rc;
-    k_tail_batch<<<1, 256, 0, s->stream>>>(s->prog, s->reps, s->clk, s->nrep, s->rebuild, s->exec_cnt);
-    LAUNCH_CHECK(s);
+    if (dev) {
+      if ((rc = tail_rebuild(s, HOT_NONE))) return rc;
+    } else {
+      k_tail_batch<<<1, 256, 0, s->stream>>>(s->prog, s->reps, s->clk, s->nrep, s->rebuild, s->exec_cnt);
+      LAUNCH_CHECK(s);
+    }
   }
   int ex = 0;
   CU(s, cudaMemcpyAsync(&ex, s->exec_cnt, sizeof(int), cudaMemcpyDeviceToHost, s->stream));
@@ -2024,6 +2192,7 @@ static int run_impl(sg_system* s, int64_t steps, sg_run_stats* stats, bool drive
   double kernel_ms = 0.0, rebuild_ms = 0.0;
   int64_t kernels_timed = 0;
   s->b_pending = false;
+  s->rb_used = false;
   CU(s, cudaEventRecord(s->ev_run0, s->stream));
   CU(s, cudaMemsetAsync(s->status, 0, sizeof(int), s->stream));
   // run-step counters restart with every `run` (samos.cpp:881); a
@@ -2061,7 +2230,15 @@ static int run_impl(sg_system* s, int64_t steps, sg_run_stats* stats, bool drive
     }
     // batched stepping: steps enqueued kBatch at a time with no host round
     // trip, the first step that flags a rebuild halting the rest (same bits)
-    const int64_t K = std::min<int64_t>(needs_nl ? std::min<int64_t>(kBatch, s->last_gap / 2) : kBatch, steps - t);
+    // (with the rebuilds enqueued too, nothing halts them)
+    const bool dev = needs_nl && !driver && !resc && fused && dev_rebuild(s);
+    const int64_t K = std::min<int64_t>(dev ? kBatchDev : needs_nl ? std::min<int64_t>(kBatch, s->last_gap / 2) : kBatch,
+                                        steps - t);
+    if (shape != HOT_NONE && t == 0) {
+      if (!s->e1_applied) rc = hot_pack_enforce(s, shape);
+      else rc = hot_pack(s, shape);
+      if (rc) return rc;
+    }
     if (driver && t > 0 && !last && K > 1 && !s->profile && !resc) {
       int64_t ex = 0;
       bool all = false;
@@ -2071,7 +2248,15 @@ static int run_impl(sg_system* s, int64_t steps, sg_run_stats* stats, bool drive
       if (all) break;
       continue;
     }
-    if (shape != HOT_NONE && t > 0 && !last && K > 1 && !driver && !s->profile && (!s->abp_on || s->tuned)) {
+    if (dev && shape != HOT_NONE && !last && resident_run(s, shape)) {
+      int64_t ex = 0;
+      if ((rc = run_resident(s, shape, std::min<int64_t>(kResidentSteps, steps - t), &ex, &rebuild_ms))) return rc;
+      done += ex;
+      t += ex - 1;
+      continue;
+    }
+    if (shape != HOT_NONE && (t > 0 || dev) && !last && K > (dev ? 0 : 1) && !driver && !s->profile &&
+        (!s->abp_on || s->tuned)) {
       int64_t ex = 0;
       if ((rc = run_batch(s, shape, K, needs_nl, &ex, &rebuild_ms))) return rc;
       done += ex;
@@ -2085,7 +2270,8 @@ static int run_impl(sg_system* s, int64_t steps, sg_run_stats* stats, bool drive
       t += ex - 1;
       continue;
     }
-    if (shape == HOT_NONE && fused && !resc && t > 0 && !last && K > 1 && !s->profile && (s->gen_tuned || s->gen_pin)) {
+    if (shape == HOT_NONE && fused && !resc && (t > 0 || dev) && !last && K > (dev ? 0 : 1) && !s->profile &&
+        (s->gen_tuned || s->gen_pin)) {
       int64_t ex = 0;
       if ((rc = run_batch_generic(s, K, needs_nl, &ex, &rebuild_ms))) return rc;
       done += ex;
@@ -2093,11 +2279,6 @@ static int run_impl(sg_system* s, int64_t steps, sg_run_stats* stats, bool drive
       continue;
     }
     if (shape != HOT_NONE) {
-      if (t == 0) {
-        if (!s->e1_applied) rc = hot_pack_enforce(s, shape);
-        else rc = hot_pack(s, shape);
-        if (rc) return rc;
-      }
       rc = step_hot(s, shape, !last, last, last);
       s->e1_applied = !last;
     } else if (fused) {
@@ -2139,8 +2320,14 @@ static int run_impl(sg_system* s, int64_t steps, sg_run_stats* stats, bool drive
   }
   CU(s, cudaEventRecord(s->ev_run1, s->stream));
   int st = 0;
+  RebuildStats rbs{};
   CU(s, cudaMemcpyAsync(&st, s->status, sizeof(int), cudaMemcpyDeviceToHost, s->stream));
+  if (s->rb_used) CU(s, cudaMemcpyAsync(&rbs, s->rb_stats, sizeof(rbs), cudaMemcpyDeviceToHost, s->stream));
   CU(s, cudaStreamSynchronize(s->stream));
+  s->builds_run += rbs.builds;
+  s->maxnb_seen = std::max(s->maxnb_seen, rbs.maxnb);
+  rebuild_ms += 1e-6 * (double)rbs.ns;
+  if (st & ST_TIMEOUT) return grid_timeout(s);
   float run_ms = 0.f;
   CU(s, cudaEventElapsedTime(&run_ms, s->ev_run0, s->ev_run1));
   if (int rcb = flush_rebuild_time(s, &rebuild_ms)) return rcb;
@@ -2238,6 +2425,7 @@ int sg_positions_changed(sg_system* s) {
 
 int sg_set_variant(sg_system* s, int variant) {
   if (!s || variant < -1 || variant >= ABP_NVARIANT) return SG_ERR_ARG;
+  s->pinned = variant >= 0;
   if (variant < 0) {  // re-tune on the next run
     s->tuned = false; s->tune_trial = 0;
     for (int v = 0; v < ABP_NVARIANT; v++) { s->tune_ms[v] = 0.0; s->tune_n[v] = 0; }

@@ -1232,15 +1232,25 @@ __device__ __forceinline__ void build_particle(const Replica& R, int mode, int k
 // each candidate is one 32-byte record read straight from its cell's range
 // (position, id, slot) instead of a slot index followed by four loads from
 // the particle arrays.  Same candidates, order and arithmetic: same lists.
-__device__ __forceinline__ void build_particle_packed(const Replica& R, int k, Dyn d, Stat st, NbList nl,
-                                                     const D4* __restrict__ cand, const int* __restrict__ cstart,
-                                                     const int* __restrict__ ccnt, int* __restrict__ status,
-                                                     int* __restrict__ maxnb) {
-  const double x = d.x[k], y = d.y[k], z = d.z[k];
-  const int myid = st.id[k];
+// COH: the records and cell arrays were written by this kernel (before a grid
+// barrier), so they are read with plain loads.
+template <bool COH>
+__device__ __forceinline__ int ld_int(const int* p) {
+  if constexpr (COH) return *p;
+  else return __ldg(p);
+}
+template <bool COH>
+__device__ __forceinline__ D4 ld_rec(const D4* p) {
+  if constexpr (COH) return ld4(p);
+  else return ldg4(p);
+}
+template <bool COH>
+__device__ __forceinline__ void build_particle_packed(const Replica& R, int k, double x, double y, double z, int myid,
+                                                      const NbList& nl, const D4* cand, const int* cstart,
+                                                      const int* ccnt, int* status, int* maxnb) {
   int a, b, c;
   cell_of(R, x, y, z, a, b, c);
-  const int base0 = cstart[R.cell_off];
+  const int base0 = ld_int<COH>(cstart + R.cell_off);
   // the stencil's cells in visiting order as runs of consecutive candidate
   // records: runs that meet in the record array merge, empty ones drop out.
   // Away from the z faces the three z-cells of one (x, y) column are
@@ -1255,7 +1265,8 @@ __device__ __forceinline__ void build_particle_packed(const Replica& R, int k, D
         int ib = b + oy;
         if (ib < 0) ib = R.cny - 1; else if (ib == R.cny) ib = 0;
         const int f = R.cell_off + R.cny * R.cnz * ia + R.cnz * ib + (c - 1);
-        const int s0 = R.off + cstart[f] - base0, n = cstart[f + 2] + ccnt[f + 2] - cstart[f];
+        const int first = ld_int<COH>(cstart + f);
+        const int s0 = R.off + first - base0, n = ld_int<COH>(cstart + f + 2) + ld_int<COH>(ccnt + f + 2) - first;
         if (n == 0) continue;
         if (nr > 0 && rs[nr - 1] + rn[nr - 1] == s0) rn[nr - 1] += n;
         else { rs[nr] = s0; rn[nr] = n; nr++; }
@@ -1266,7 +1277,7 @@ __device__ __forceinline__ void build_particle_packed(const Replica& R, int k, D
     const int ncells = build_stencil(R, a, b, c, cells);
     for (int m = 0; m < ncells; m++) {
       const int cg = R.cell_off + cells[m];
-      const int s0 = R.off + cstart[cg] - base0, n = ccnt[cg];
+      const int s0 = R.off + ld_int<COH>(cstart + cg) - base0, n = ld_int<COH>(ccnt + cg);
       if (n == 0) continue;
       if (nr > 0 && rs[nr - 1] + rn[nr - 1] == s0) rn[nr - 1] += n;
       else { rs[nr] = s0; rn[nr] = n; nr++; }
@@ -1280,12 +1291,12 @@ __device__ __forceinline__ void build_particle_packed(const Replica& R, int k, D
   // one flat sweep over the runs' records (lanes of a warp stay together
   // across cell boundaries); each record requested one candidate ahead
   int ri = 0, pos = nr > 0 ? rs[0] : 0, end = nr > 0 ? rs[0] + rn[0] : 0;
-  D4 nxt = total > 0 ? ldg4(cand + pos) : D4{0.0, 0.0, 0.0, 0.0};
+  D4 nxt = total > 0 ? ld_rec<COH>(cand + pos) : D4{0.0, 0.0, 0.0, 0.0};
   for (int t = 0; t < total; t++) {
     const D4 cr = nxt;
     if (t + 1 < total) {
       if (++pos == end) { ri++; pos = rs[ri]; end = pos + rn[ri]; }
-      nxt = ldg4(cand + pos);
+      nxt = ld_rec<COH>(cand + pos);
     }
     {
       const unsigned long long key = (unsigned long long)__double_as_longlong(cr.w);
@@ -1333,7 +1344,7 @@ __device__ __forceinline__ void build_particle_packed(const Replica& R, int k, D
       int w = nlo;
       for (int i = 0; i < nr; i++)
         for (int q = rs[i]; q < rs[i] + rn[i]; q++) {
-          const D4 cr = ldg4(cand + q);
+          const D4 cr = ld_rec<COH>(cand + q);
           const unsigned long long key = (unsigned long long)__double_as_longlong(cr.w);
           if ((int)(unsigned)(key >> 32) <= myid) continue;
           double dx = x - cr.x, dy = y - cr.y, dz = z - cr.z;
@@ -1357,7 +1368,7 @@ static __global__ void k_rb_build(const Replica* __restrict__ reps, const int* _
   const Replica& R = reps[r];
   const int k = bid_ * BLOCK + threadIdx.x;
   if (k - R.off >= R.n) return;
-  build_particle_packed(R, k, d, st, nl, cand, cstart, ccnt, status, maxnb);
+  build_particle_packed<false>(R, k, d.x[k], d.y[k], d.z[k], st.id[k], nl, cand, cstart, ccnt, status, maxnb);
 }
 
 // Cell m (0..26) of the 27-cell stencil of (a, b, c), in the visiting order

@@ -1,0 +1,382 @@
+// sg_rebuild.cuh -- the neighbour-list rebuild as phases of one cooperative
+// kernel (sm_100a), so that steps and rebuilds are enqueued without a host
+// round trip.
+//
+// The host-driven rebuild (rebuild_flagged) costs eight launches, three small
+// uploads, a read-back and a wait, and halts every step enqueued after the one
+// that flagged it.  A system of many replicas rebuilds some of them after
+// nearly every step.  Here the blocks of one cooperative launch pass through
+// the same phases with a grid barrier between them; when no replica is flagged
+// they return after reading the flags.  Same cells, order and arithmetic: same
+// lists.
+#pragma once
+#include "sg_abp.cuh"
+
+namespace sg {
+
+// ---------------------------------------------------------------------------
+// grid barrier of a cooperative launch: every block adds 1 to bar[0] and waits
+// until all have.  Bounded: a wait that runs out records ST_TIMEOUT and the
+// block leaves the kernel (the others then run out too).
+// ---------------------------------------------------------------------------
+constexpr unsigned GRID_SPIN_LIMIT = 1u << 24;
+
+__device__ __forceinline__ unsigned ld_acquire(const unsigned* p) {
+  unsigned v;
+  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+
+struct GridBar {
+  unsigned* cnt;    // [0] arrivals, [1] blocks done: both 0 between launches
+  unsigned passed;  // barriers passed by this block
+  int* status;
+};
+
+__device__ __forceinline__ bool grid_wait(GridBar& g) {
+  g.passed++;
+  __syncthreads();
+  int ok = 1;
+  if (threadIdx.x == 0) {
+    const unsigned target = g.passed * gridDim.x;
+    __threadfence();
+    atomicAdd(g.cnt, 1u);
+    unsigned it = 0;
+    while (ld_acquire(g.cnt) < target && ++it < GRID_SPIN_LIMIT) {}
+    if (it >= GRID_SPIN_LIMIT) { atomicOr(g.status, ST_TIMEOUT); ok = 0; }
+    __threadfence();
+  }
+  return __syncthreads_and(ok) != 0;
+}
+
+// True on every thread of the block that finishes last; that block has put the
+// barrier back to its start.
+__device__ __forceinline__ bool grid_last(GridBar& g) {
+  __shared__ int last;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    last = atomicAdd(g.cnt + 1, 1u) == gridDim.x - 1;
+    if (last) { g.cnt[0] = 0; g.cnt[1] = 0; }
+    __threadfence();
+  }
+  __syncthreads();
+  return last != 0;
+}
+
+// ---------------------------------------------------------------------------
+constexpr int RB_MAX_REP = 512;  // replicas whose flags a block keeps in shared memory
+
+struct RebuildStats { unsigned long long ns; int builds; int maxnb; };
+
+struct RebuildArgs {
+  const Replica* reps;
+  const int *rep_blk0, *rep_nblk;
+  int nrep;
+  Clock* clk;
+  int* rebuild;     // flags set by the step's skin test
+  int* builds;      // list builds per replica: every SORT_EVERY-th re-sorts
+  Dyn cur, alt;
+  Stat st, st_alt;
+  NbList nl;
+  D4 *G, *H;        // packed records (HOT_PLANE / HOT_SPHERE)
+  int *pcell, *cell_cnt, *cell_start, *cell_fill, *tmp, *perm, *bsum;
+  D4* cand;
+  uint8_t* lane_order;  // null: not kept
+  int* bstatus;
+  RebuildStats* stats;
+  unsigned* bar;
+  int* status;
+  int* executed;
+};
+
+// the flagged replicas of this launch, as each block holds them
+struct RebuildList {
+  int n, nblk, ncell, any_sort;
+  int rep[RB_MAX_REP], mode[RB_MAX_REP];
+  int blk[RB_MAX_REP + 1], cell[RB_MAX_REP + 1];  // first virtual block / cell of each
+};
+
+// Reads the flags; false when no replica is flagged.
+__device__ __forceinline__ bool rebuild_list(const RebuildArgs& A, int sort_every, RebuildList& L) {
+  __shared__ int any;
+  if (threadIdx.x == 0) any = 0;
+  __syncthreads();
+  for (int r = threadIdx.x; r < A.nrep; r += blockDim.x)
+    if (__ldcg(A.rebuild + r)) any = 1;
+  __syncthreads();
+  if (!any) return false;
+  if (threadIdx.x < 32) {  // one warp puts the flagged replicas in order
+    int n = 0, nb = 0, nc = 0, srt = 0;
+    for (int r0 = 0; r0 < A.nrep; r0 += 32) {
+      const int r = r0 + threadIdx.x;
+      const bool f = r < A.nrep && __ldcg(A.rebuild + r) != 0;
+      const unsigned m = __ballot_sync(0xffffffffu, f);
+      int b = f ? A.rep_nblk[r] : 0, c = f ? A.reps[r].ncell : 0;
+      const int b_own = b, c_own = c;
+      for (int o = 1; o < 32; o <<= 1) {
+        const int vb = __shfl_up_sync(0xffffffffu, b, o), vc = __shfl_up_sync(0xffffffffu, c, o);
+        if ((int)threadIdx.x >= o) { b += vb; c += vc; }
+      }
+      if (f) {
+        const int at = n + __popc(m & ((1u << threadIdx.x) - 1u));
+        const int mode = (__ldcg(A.builds + r) % sort_every) == 0 ? 2 : 1;
+        L.rep[at] = r; L.mode[at] = mode;
+        L.blk[at] = nb + b - b_own; L.cell[at] = nc + c - c_own;
+        if (mode == 2) srt = 1;
+      }
+      n += __popc(m);
+      nb += __shfl_sync(0xffffffffu, b, 31);
+      nc += __shfl_sync(0xffffffffu, c, 31);
+    }
+    srt = __any_sync(0xffffffffu, srt);
+    if (threadIdx.x == 0) { L.n = n; L.nblk = nb; L.ncell = nc; L.any_sort = srt; L.blk[n] = nb; L.cell[n] = nc; }
+  }
+  __syncthreads();
+  return true;
+}
+
+__device__ __forceinline__ int list_find(const int* first, int n, int v) {  // last entry with first <= v
+  int lo = 0, hi = n - 1;
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) >> 1;
+    if (first[mid] <= v) lo = mid; else hi = mid - 1;
+  }
+  return lo;
+}
+
+// position of slot k as the list build sees it
+template <int SHAPE>
+__device__ __forceinline__ void rb_position(const RebuildArgs& A, int k, double& x, double& y, double& z) {
+  if (SHAPE == HOT_NONE) { x = A.cur.x[k]; y = A.cur.y[k]; z = A.cur.z[k]; }
+  else {
+    const D4 g = ld4(A.G + k);
+    x = g.x; y = g.y;
+    z = SHAPE == HOT_PLANE ? A.cur.z[k] : g.z;
+  }
+}
+template <int SHAPE>
+__device__ __forceinline__ void rb_store_position(const RebuildArgs& A, int k, double x, double y, double z) {
+  if (SHAPE == HOT_NONE) { A.cur.x[k] = x; A.cur.y[k] = y; A.cur.z[k] = z; }
+  else {
+    D4 g = ld4(A.G + k);
+    g.x = x; g.y = y;
+    if (SHAPE == HOT_SPHERE) g.z = z; else A.cur.z[k] = z;
+    stg4(A.G + k, g);
+  }
+}
+
+// All phases for the replicas in L (every block of the launch takes part).
+// False: a barrier's wait ran out.
+template <int SHAPE>
+__device__ bool rebuild_phases(const RebuildArgs& A, RebuildList& L, GridBar& bar) {
+  const int t = threadIdx.x, nthr = gridDim.x * blockDim.x, gid = blockIdx.x * blockDim.x + t;
+  __shared__ int shw[32];
+  for (int v = gid; v < L.ncell; v += nthr) {  // (k_seg_zero)
+    const int s = list_find(L.cell, L.n, v);
+    const int c = A.reps[L.rep[s]].cell_off + v - L.cell[s];
+    A.cell_cnt[c] = 0; A.cell_fill[c] = 0;
+  }
+  if (gid == 0) *A.bstatus = 0;
+  if (!grid_wait(bar)) return false;
+
+  for (int v = blockIdx.x; v < L.nblk; v += gridDim.x) {  // (k_rb_bin)
+    const int s = list_find(L.blk, L.n, v);
+    const Replica& R = A.reps[L.rep[s]];
+    const int k = R.off + (v - L.blk[s]) * BLOCK + t;
+    if (k - R.off >= R.n) continue;
+    double x, y, z;
+    rb_position<SHAPE>(A, k, x, y, z);
+    if (R.periodic) {
+      bool ch = false;
+      if (x < R.xlo) { x += R.Lx; ch = true; } else if (x > R.xhi) { x -= R.Lx; ch = true; }
+      if (y < R.ylo) { y += R.Ly; ch = true; } else if (y > R.yhi) { y -= R.Ly; ch = true; }
+      if (z < R.zlo) { z += R.Lz; ch = true; } else if (z > R.zhi) { z -= R.Lz; ch = true; }
+      if (ch) rb_store_position<SHAPE>(A, k, x, y, z);
+    }
+    int a, b, c;
+    const int cl = cell_of(R, x, y, z, a, b, c);
+    A.pcell[k] = cl;
+    atomicAdd(&A.cell_cnt[R.cell_off + cl], 1);
+  }
+  if (!grid_wait(bar)) return false;
+
+  // exclusive scan of the flagged cells' counts: a run of tiles per block
+  const int tiles = (L.ncell + BLOCK * 4 - 1) / (BLOCK * 4);
+  const int per = (tiles + gridDim.x - 1) / gridDim.x;
+  const int tile0 = min((int)blockIdx.x * per, tiles), tile1 = min(tile0 + per, tiles);
+  auto cell_at = [&](int v) {
+    const int s = list_find(L.cell, L.n, v);
+    return A.reps[L.rep[s]].cell_off + v - L.cell[s];
+  };
+  {
+    int sum = 0;
+    for (int v = tile0 * BLOCK * 4 + t; v < min(tile1 * BLOCK * 4, L.ncell); v += BLOCK) sum += A.cell_cnt[cell_at(v)];
+    for (int o = 16; o > 0; o >>= 1) sum += __shfl_down_sync(0xffffffffu, sum, o);
+    if ((t & 31) == 0) shw[t >> 5] = sum;
+    __syncthreads();
+    if (t == 0) {
+      int x = 0;
+      for (int w = 0; w < BLOCK / 32; w++) x += shw[w];
+      A.bsum[blockIdx.x] = x;
+    }
+  }
+  if (!grid_wait(bar)) return false;
+  {
+    int before = 0;
+    for (int b = t; b < (int)blockIdx.x; b += BLOCK) before += A.bsum[b];
+    for (int o = 16; o > 0; o >>= 1) before += __shfl_down_sync(0xffffffffu, before, o);
+    __syncthreads();
+    if ((t & 31) == 0) shw[t >> 5] = before;
+    __syncthreads();
+    before = 0;
+    for (int w = 0; w < BLOCK / 32; w++) before += shw[w];
+    __syncthreads();
+    for (int tile = tile0; tile < tile1; tile++) {
+      int c[4], n[4], s = 0;
+#pragma unroll
+      for (int i = 0; i < 4; i++) {
+        const int v = (tile * BLOCK + t) * 4 + i;
+        c[i] = v < L.ncell ? cell_at(v) : -1;
+        n[i] = c[i] >= 0 ? A.cell_cnt[c[i]] : 0;
+        s += n[i];
+      }
+      int tot;
+      int ex = before + block_excl_scan(s, shw, tot);
+#pragma unroll
+      for (int i = 0; i < 4; i++) {
+        if (c[i] >= 0) A.cell_start[c[i]] = ex;
+        ex += n[i];
+      }
+      before += tot;
+    }
+  }
+  if (!grid_wait(bar)) return false;
+
+  for (int v = blockIdx.x; v < L.nblk; v += gridDim.x) {  // (k_rb_scatter)
+    const int s = list_find(L.blk, L.n, v);
+    const Replica& R = A.reps[L.rep[s]];
+    const int k = R.off + (v - L.blk[s]) * BLOCK + t;
+    if (k - R.off >= R.n) continue;
+    const int cg = R.cell_off + A.pcell[k];
+    const int pos = A.cell_start[cg] - A.cell_start[R.cell_off] + atomicAdd(&A.cell_fill[cg], 1);
+    A.tmp[R.off + pos] = k;
+  }
+  if (!grid_wait(bar)) return false;
+
+  for (int v = blockIdx.x; v < L.nblk; v += gridDim.x) {  // (k_rb_rank)
+    const int s = list_find(L.blk, L.n, v);
+    const Replica& R = A.reps[L.rep[s]];
+    const int k = R.off + (v - L.blk[s]) * BLOCK + t;
+    if (k - R.off >= R.n) continue;
+    const int cg = R.cell_off + A.pcell[k];
+    const int s0 = R.off + A.cell_start[cg] - A.cell_start[R.cell_off], n = A.cell_cnt[cg];
+    const int myid = A.st.id[k];
+    int rank = 0;
+    for (int q = 0; q < n; q++) rank += A.st.id[A.tmp[s0 + q]] < myid ? 1 : 0;
+    A.perm[s0 + rank] = k;
+    double x, y, z;
+    rb_position<SHAPE>(A, k, x, y, z);
+    stg4(A.cand + s0 + rank, D4{x, y, z, pack_id_slot(myid, L.mode[s] == 2 ? s0 + rank : k)});
+  }
+  if (!grid_wait(bar)) return false;
+
+  for (int v = blockIdx.x; v < L.nblk; v += gridDim.x) {  // (k_rb_gather, k_rb_build, k_lane_order)
+    const int s = list_find(L.blk, L.n, v);
+    const Replica& R = A.reps[L.rep[s]];
+    const int k = R.off + (v - L.blk[s]) * BLOCK + t;
+    const bool valid = k - R.off < R.n;
+    if (valid) {
+      double x, y, z;
+      int myid;
+      if (L.mode[s] == 2) {
+        // slot k takes the k-th particle in cell order; its fields wait in the
+        // other store until every block has read the old order
+        const int o = A.perm[k];
+        Part p;
+        load_dyn(A.cur, o, p);
+        if (SHAPE != HOT_NONE) {
+          const D4 g = ld4(A.G + o);
+          p.x = g.x; p.y = g.y;
+          if (SHAPE == HOT_PLANE) { p.nx = g.z; p.ny = g.w; }
+          else { const D4 h = ld4(A.H + o); p.z = g.z; p.nx = h.x; p.ny = h.y; p.nz = h.z; }
+        }
+        store_dyn(A.alt, k, p);
+        A.st_alt.r[k] = A.st.r[o]; A.st_alt.mass[k] = A.st.mass[o];
+        A.st_alt.type[k] = A.st.type[o]; A.st_alt.id[k] = A.st.id[o];
+        x = p.x; y = p.y; z = p.z;
+        myid = A.st.id[o];
+      } else {
+        rb_position<SHAPE>(A, k, x, y, z);
+        myid = A.st.id[k];
+      }
+      build_particle_packed<true>(R, k, x, y, z, myid, A.nl, A.cand, A.cell_start, A.cell_cnt, A.bstatus,
+                                  &A.stats->maxnb);
+    }
+    if (A.lane_order) {
+      __syncthreads();
+      lane_order_block(valid ? A.nl.cnt[k] : -1, A.nl.cap, A.lane_order + (size_t)(k - t));
+      __syncthreads();
+    }
+  }
+  if (L.any_sort) {
+    if (!grid_wait(bar)) return false;
+    for (int v = blockIdx.x; v < L.nblk; v += gridDim.x) {  // (k_rb_copyback, k_hot_pack)
+      const int s = list_find(L.blk, L.n, v);
+      if (L.mode[s] != 2) continue;
+      const Replica& R = A.reps[L.rep[s]];
+      const int k = R.off + (v - L.blk[s]) * BLOCK + t;
+      if (k - R.off >= R.n) continue;
+      Part p;
+      load_dyn(A.alt, k, p);
+      store_dyn(A.cur, k, p);
+      A.st.r[k] = A.st_alt.r[k]; A.st.mass[k] = A.st_alt.mass[k];
+      A.st.type[k] = A.st_alt.type[k]; A.st.id[k] = A.st_alt.id[k];
+      if (SHAPE == HOT_PLANE) stg4(A.G + k, D4{p.x, p.y, p.nx, p.ny});
+      if (SHAPE == HOT_SPHERE) {
+        stg4(A.G + k, D4{p.x, p.y, p.z, A.st_alt.r[k]});
+        stg4(A.H + k, D4{p.nx, p.ny, p.nz, 0.0});
+      }
+    }
+  }
+  return true;
+}
+
+__device__ __forceinline__ unsigned long long global_ns() {
+  unsigned long long t;
+  asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+  return t;
+}
+
+// Bookkeeping of the block that finishes last: the flags are cleared and the
+// builds counted; lists that did not fit leave the flags set and halt the
+// steps enqueued after this one, for the host to grow the lists.
+__device__ __forceinline__ void rebuild_done(const RebuildArgs& A, const RebuildList& L, unsigned long long t0) {
+  const bool over = (__ldcg(A.bstatus) & ST_OVERFLOW) != 0;
+  if (over) {
+    for (int r = threadIdx.x; r < A.nrep; r += blockDim.x) A.clk[r].halt = 1;
+  } else {
+    for (int s = threadIdx.x; s < L.n; s += blockDim.x) { A.rebuild[L.rep[s]] = 0; A.builds[L.rep[s]]++; }
+    if (threadIdx.x == 0) { A.stats->builds++; A.stats->ns += global_ns() - t0; }
+  }
+}
+
+// End of a step enqueued without a host round trip: the step counters advance
+// (as k_tail_batch), and the flagged replicas' lists are rebuilt.
+template <int SHAPE>
+__global__ void __launch_bounds__(BLOCK)
+k_tail_rebuild(Program P, RebuildArgs A, int sort_every) {
+  __shared__ RebuildList L;
+  if (A.clk[0].halt) return;  // set between launches only: the same for every block
+  const unsigned long long t0 = global_ns();
+  if (blockIdx.x == 0) {
+    for (int r = threadIdx.x; r < A.nrep; r += blockDim.x) tail_one(P, A.reps[r], A.clk[r]);
+    if (threadIdx.x == 0) (*A.executed)++;
+  }
+  if (!rebuild_list(A, sort_every, L)) return;
+  GridBar bar{A.bar, 0u, A.status};
+  if (!rebuild_phases<SHAPE>(A, L, bar)) return;
+  if (grid_last(bar)) rebuild_done(A, L, t0);
+}
+
+}  // namespace sg
