@@ -26,7 +26,7 @@ struct AbpParams {
   double J, rc2;          // aligner: effective J (nematic: 2J unless align_param), rcut*rcut
   double alpha;           // self_propulsion alpha
   double dt, v0, nu, mu, mur, stoch, flip;  // brownian; stoch = sqrt(nu*dt), flip = dt/tau
-  double Rs;              // sphere radius
+  double Rs, iRs;         // sphere radius, and RN(1 / Rs)
   Value temp;
   int off, n, periodic, use_radii, nematic, velocity;
   uint32_t seed, pad0;
@@ -229,7 +229,7 @@ __device__ __forceinline__ bool abp_advance(const AbpParams& S, Hp& p, double g_
     if (!PLANE) { const double fr_z = B * g_z; p.vz += fr_z; p.z += sqrt_dt * fr_z; }
   }
   dix = 0; diy = 0;
-  const ShapeGeom Rb{S.xlo, S.xhi, S.Lx, S.ylo, S.yhi, S.Ly, S.Rs};
+  const ShapeGeom Rb{S.xlo, S.xhi, S.Lx, S.ylo, S.yhi, S.Ly, S.Rs, S.iRs};
   hot_enforce<SHAPE>(Rb, p, dix, diy);
   if (PLANE) p.vz = 0.0;
   p.omega = S.mur * hot_project_torque<SHAPE>(Rb, p);
@@ -1070,7 +1070,7 @@ k_abp_flat(const AbpParams* __restrict__ prm, const int* __restrict__ blk_rep, c
       if (!PLANE) { const double fr_z = B * g_z; p.vz += fr_z; p.z += sqrt_dt * fr_z; }
     }
     int dix = 0, diy = 0;
-    const ShapeGeom Rb{S.xlo, S.xhi, S.Lx, S.ylo, S.yhi, S.Ly, S.Rs};
+    const ShapeGeom Rb{S.xlo, S.xhi, S.Lx, S.ylo, S.yhi, S.Ly, S.Rs, S.iRs};
     hot_enforce<SHAPE>(Rb, p, dix, diy);
     if (PLANE) p.vz = 0.0;
     p.tx = tx; p.ty = ty; p.tz = tz;

@@ -31,6 +31,10 @@ __device__ __forceinline__ unsigned long long ld_acquire64(const unsigned long l
   return v;
 }
 
+__device__ __forceinline__ void red_release64(unsigned long long* p, unsigned long long v) {
+  asm volatile("red.release.gpu.global.add.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+}
+
 template <int SHAPE, int ALIGN, bool SP, bool BYVAL>
 __global__ void __launch_bounds__(BLOCK, ABP_RUN_MINB)
 k_abp_run(const AbpParams* __restrict__ prm, const __grid_constant__ AbpParams pv, const int* __restrict__ blk_rep,
@@ -174,8 +178,7 @@ k_abp_run(const AbpParams* __restrict__ prm, const __grid_constant__ AbpParams p
     target[w] += gridDim.x;
     if (t == 0) {
       if (block_asks) atomicOr(&A.rebuild[r], 1);
-      __threadfence();
-      atomicAdd(word + w, 1ull + (block_asks ? 1ull << 32 : 0ull));
+      red_release64(word + w, 1ull + (block_asks ? 1ull << 32 : 0ull));
     }
     if (mine && step + 1 < nsteps) draw();
     int ok = 1;
@@ -183,7 +186,6 @@ k_abp_run(const AbpParams* __restrict__ prm, const __grid_constant__ AbpParams p
       unsigned long long v = ld_acquire64(word + w);
       for (unsigned it = 0; (unsigned)v < target[w]; v = ld_acquire64(word + w))
         if (++it >= GRID_SPIN_LIMIT) { atomicOr(A.status, ST_TIMEOUT); ok = 0; break; }
-      __threadfence();
       seen = v;
     }
     if (!__syncthreads_and(ok)) return;

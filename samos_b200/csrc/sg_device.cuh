@@ -301,6 +301,70 @@ __host__ __device__ __forceinline__ double noise_uniform(uint32_t seed, uint64_t
 }
 
 // ---------------------------------------------------------------------------
+// Correctly rounded square roots and quotients where the operands are known,
+// with a few additions and FMAs instead of a general sequence: the same bits as
+// sqrt() and '/', which every other operand still takes.
+//
+// Directors are renormalised several times a step, so their squared length s is
+// 1 but for rounding (or a step's tangential correction).  For e = s - 1,
+// |e| < 2^-27: sqrt(1 + e) = 1 + e/2 - e^2/8 + ..., the square term being below
+// a quarter of the spacing next to 1 and negative, so the nearest double is
+// 1 + e/2, rounded down where that falls half way.  For a length 1 + d, |d| <
+// 2^-27: 1/(1 + d) = 1 - d + d^2 - ..., so 1 - d, rounded up where half way.
+// A quotient a / (1 + d): a - a d is within an ulp of it, and Markstein's
+// correction (P. Markstein, IBM J. Res. Dev. 34, 1990: with the correctly
+// rounded reciprocal y and a quotient q off by less than an ulp, q + (a - b q) y
+// rounds correctly) finishes it.
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ bool near_one(double s) { return fabs(s - 1.0) < 0x1p-27; }
+__device__ __forceinline__ double sqrt_near_one(double s) { return __dadd_rd(1.0, 0.5 * (s - 1.0)); }
+__device__ __forceinline__ double rcp_near_one(double len) { return __dsub_ru(1.0, len - 1.0); }
+__device__ __forceinline__ double div_near_one(double a, double len, double y) {
+  const double q = __fma_rn(-a, len - 1.0, a);
+  return __fma_rn(__fma_rn(-q, len, a), y, q);
+}
+// far enough from zero that no remainder above underflows, and not a zero,
+// whose sign the correction would not keep
+__device__ __forceinline__ bool div_safe(double a) { return fabs(a) > 1e-200; }
+
+// 1 / sqrt(s) in the reference's two roundings
+__device__ __forceinline__ double inv_len(double s) {
+  if (near_one(s)) return rcp_near_one(sqrt_near_one(s));
+  return 1.0 / sqrt(s);
+}
+
+// (x, y[, z]) / |(x, y[, z])|
+__device__ __forceinline__ void set_unit(double x, double y, double& ux, double& uy) {
+  const double s = x * x + y * y;
+  if (near_one(s) && div_safe(x) && div_safe(y)) {
+    const double len = sqrt_near_one(s), inv = rcp_near_one(len);
+    ux = div_near_one(x, len, inv); uy = div_near_one(y, len, inv);
+  } else {
+    const double len = sqrt(s);
+    ux = x / len; uy = y / len;
+  }
+}
+__device__ __forceinline__ void set_unit(double x, double y, double z, double& ux, double& uy, double& uz) {
+  const double s = x * x + y * y + z * z;
+  if (near_one(s) && div_safe(x) && div_safe(y) && div_safe(z)) {
+    const double len = sqrt_near_one(s), inv = rcp_near_one(len);
+    ux = div_near_one(x, len, inv); uy = div_near_one(y, len, inv); uz = div_near_one(z, len, inv);
+  } else {
+    const double len = sqrt(s);
+    ux = x / len; uy = y / len; uz = z / len;
+  }
+}
+
+// a / b for a divisor used many times: y = RN(1 / b).  The first correction
+// brings the quotient to within an ulp, the second is Markstein's.
+__device__ __forceinline__ double div_known(double a, double b, double y) {
+  if (!div_safe(a) || fabs(a) > 1e200) return a / b;
+  double q = a * y;
+  q = __fma_rn(__fma_rn(-q, b, a), y, q);
+  return __fma_rn(__fma_rn(-q, b, a), y, q);
+}
+
+// ---------------------------------------------------------------------------
 // periodic box, system/system.cpp:1083-1154
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ void apply_periodic(const Replica& R, double& dx, double& dy, double& dz) {
@@ -333,10 +397,9 @@ __device__ __forceinline__ void plane_enforce(const Replica& R, double zpos, int
     if (p.y < ylo) { p.y = ylo; p.vy = -p.vy; } else if (p.y > yhi) { p.y = yhi; p.vy = -p.vy; }
   }
   p.nz = 0.0;
-  double len_n = sqrt(p.nx * p.nx + p.ny * p.ny);
-  double inv_len = 1.0;
-  if (len_n != 0.0) inv_len = 1.0 / len_n;  // the reference recomputes the same sqrt
-  p.nx *= inv_len; p.ny *= inv_len;
+  const double nn = p.nx * p.nx + p.ny * p.ny;  // the reference recomputes the same sqrt
+  const double inv = nn != 0.0 ? inv_len(nn) : 1.0;
+  p.nx *= inv; p.ny *= inv;
 }
 
 // ConstraintSphere::enforce, constraints/constraint_sphere.cpp:38-81
@@ -349,8 +412,8 @@ __device__ __forceinline__ void sphere_enforce(double Rs, Part& p) {
   double n_dot_N = p.nx * Nx + p.ny * Ny + p.nz * Nz;
   p.vx -= v_dot_N * Nx; p.vy -= v_dot_N * Ny; p.vz -= v_dot_N * Nz;
   p.nx -= n_dot_N * Nx; p.ny -= n_dot_N * Ny; p.nz -= n_dot_N * Nz;
-  double inv_len = 1.0 / sqrt(p.nx * p.nx + p.ny * p.ny + p.nz * p.nz);
-  p.nx *= inv_len; p.ny *= inv_len; p.nz *= inv_len;
+  const double inv = inv_len(p.nx * p.nx + p.ny * p.ny + p.nz * p.nz);
+  p.nx *= inv; p.ny *= inv; p.nz *= inv;
 }
 
 // ConstraintCylinder::enforce, constraints/constraint_cylinder.cpp:38-71 (its
@@ -365,8 +428,8 @@ __device__ __forceinline__ void cylinder_enforce(const Replica& R, double rc, Pa
   double n_dot_N = p.nx * Nx + p.ny * Ny;
   p.vx -= v_dot_N * Nx; p.vy -= v_dot_N * Ny;
   p.nx -= n_dot_N * Nx; p.ny -= n_dot_N * Ny;
-  double inv_len = 1.0 / sqrt(p.nx * p.nx + p.ny * p.ny + p.nz * p.nz);
-  p.nx *= inv_len; p.ny *= inv_len; p.nz *= inv_len;
+  const double inv = inv_len(p.nx * p.nx + p.ny * p.ny + p.nz * p.nz);
+  p.nx *= inv; p.ny *= inv; p.nz *= inv;
   if (R.periodic) {
     if (p.z > R.zhi) p.z -= R.Lz;
     else if (p.z < R.zlo) p.z += R.Lz;
@@ -519,8 +582,8 @@ __device__ __forceinline__ void implicit_enforce(const ConsComp& C, const Replic
   double n_dot_N = p.nx * Nx + p.ny * Ny + p.nz * Nz;
   p.vx -= v_dot_N * Nx; p.vy -= v_dot_N * Ny; p.vz -= v_dot_N * Nz;
   p.nx -= n_dot_N * Nx; p.ny -= n_dot_N * Ny; p.nz -= n_dot_N * Nz;
-  double inv_len = 1.0 / sqrt(p.nx * p.nx + p.ny * p.ny + p.nz * p.nz);
-  p.nx *= inv_len; p.ny *= inv_len; p.nz *= inv_len;
+  const double inv = inv_len(p.nx * p.nx + p.ny * p.ny + p.nz * p.nz);
+  p.nx *= inv; p.ny *= inv; p.nz *= inv;
   enforce_periodic(R, p);
 }
 
@@ -568,8 +631,7 @@ __device__ __forceinline__ void rotate_director(const Program& P, const Replica&
       double Rxx = cs, Rxy = -sn, Ryx = sn, Ryy = cs;
       double nx = Rxx * p.nx + Rxy * p.ny;
       double ny = Ryx * p.nx + Ryy * p.ny;
-      double len = sqrt(nx * nx + ny * ny);
-      p.nx = nx / len; p.ny = ny / len;
+      set_unit(nx, ny, p.nx, p.ny);
     } else if (kind != CONS_NONE && kind != CONS_SLAB) {  // the slab does not rotate (constraint_slab.hpp:85-88)
       double U, V, W;
       surface_normal(P.cons[c], R, R.cons_p[c], p, U, V, W);
@@ -578,8 +640,7 @@ __device__ __forceinline__ void rotate_director(const Program& P, const Replica&
       double nx = U * dot * (1.0 - cs) + p.nx * cs + (-W * p.ny + V * p.nz) * sn;
       double ny = V * dot * (1.0 - cs) + p.ny * cs + (W * p.nx - U * p.nz) * sn;
       double nz = W * dot * (1.0 - cs) + p.nz * cs + (-V * p.nx + U * p.ny) * sn;
-      double len = sqrt(nx * nx + ny * ny + nz * nz);
-      p.nx = nx / len; p.ny = ny / len; p.nz = nz / len;
+      set_unit(nx, ny, nz, p.nx, p.ny, p.nz);
     }
   }
 }

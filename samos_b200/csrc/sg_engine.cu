@@ -1718,7 +1718,7 @@ static int abp_upload(sg_system* s) {
     A.dt = ip[0]; A.v0 = ip[1]; A.nu = ip[2]; A.mu = ip[3]; A.mur = ip[4];
     A.stoch = std::sqrt(ip[2] * ip[0]);
     A.flip = P.integ[0].nematic ? ip[0] / ip[7] : 0.0;
-    A.Rs = R.cons_p[0];
+    A.Rs = R.cons_p[0]; A.iRs = 1.0 / R.cons_p[0];
     A.temp = P.integ[0].temp;
     A.off = R.off; A.n = R.n; A.periodic = R.periodic; A.use_radii = P.pair[0].use_radii;
     A.nematic = P.integ[0].nematic; A.velocity = P.integ[0].velocity;

@@ -107,10 +107,9 @@ __device__ __forceinline__ void hot_plane_enforce(double xlo, double xhi, double
                                                   double Ly, Hp& p, int& dix, int& diy) {
   if (p.x <= xlo) { p.x += Lx; dix--; } else if (p.x > xhi) { p.x -= Lx; dix++; }
   if (p.y <= ylo) { p.y += Ly; diy--; } else if (p.y > yhi) { p.y -= Ly; diy++; }
-  double len_n = sqrt(p.nx * p.nx + p.ny * p.ny);
-  double inv_len = 1.0;
-  if (len_n != 0.0) inv_len = 1.0 / len_n;
-  p.nx *= inv_len; p.ny *= inv_len;
+  const double nn = p.nx * p.nx + p.ny * p.ny;
+  const double inv = nn != 0.0 ? inv_len(nn) : 1.0;
+  p.nx *= inv; p.ny *= inv;
 }
 
 // ConstraintPlane::rotate_director (constraint_plane.cpp:97-114)
@@ -119,8 +118,7 @@ __device__ __forceinline__ void hot_plane_rotate(Hp& p, double phi, bool velocit
   sincos(phi, &sn, &cs);
   double nx = cs * p.nx + -sn * p.ny;
   double ny = sn * p.nx + cs * p.ny;
-  double len = sqrt(nx * nx + ny * ny);
-  p.nx = nx / len; p.ny = ny / len;
+  set_unit(nx, ny, p.nx, p.ny);
   if (velocity) {  // ConstraintPlane::rotate_velocity (122-143)
     double vx = cs * p.vx + -sn * p.vy;
     double vy = sn * p.vx + cs * p.vy;
@@ -129,31 +127,30 @@ __device__ __forceinline__ void hot_plane_rotate(Hp& p, double phi, bool velocit
 }
 
 // ConstraintSphere::enforce (constraint_sphere.cpp:38-81)
-__device__ __forceinline__ void hot_sphere_enforce(double Rs, Hp& p) {
+__device__ __forceinline__ void hot_sphere_enforce(double Rs, double iRs, Hp& p) {
   double Rr = sqrt(p.x * p.x + p.y * p.y + p.z * p.z);
   double s = Rs / Rr;
   p.x *= s; p.y *= s; p.z *= s;
-  double Nx = p.x / Rs, Ny = p.y / Rs, Nz = p.z / Rs;
+  double Nx = div_known(p.x, Rs, iRs), Ny = div_known(p.y, Rs, iRs), Nz = div_known(p.z, Rs, iRs);
   double v_dot_N = p.vx * Nx + p.vy * Ny + p.vz * Nz;
   double n_dot_N = p.nx * Nx + p.ny * Ny + p.nz * Nz;
   p.vx -= v_dot_N * Nx; p.vy -= v_dot_N * Ny; p.vz -= v_dot_N * Nz;
   p.nx -= n_dot_N * Nx; p.ny -= n_dot_N * Ny; p.nz -= n_dot_N * Nz;
-  double inv_len = 1.0 / sqrt(p.nx * p.nx + p.ny * p.ny + p.nz * p.nz);
-  p.nx *= inv_len; p.ny *= inv_len; p.nz *= inv_len;
+  const double inv = inv_len(p.nx * p.nx + p.ny * p.ny + p.nz * p.nz);
+  p.nx *= inv; p.ny *= inv; p.nz *= inv;
 }
 
 // Constraint::rotate_director / rotate_velocity about the sphere normal
 // (constraint.cpp:96-150)
-__device__ __forceinline__ void hot_sphere_rotate(double Rs, Hp& p, double phi, bool velocity) {
-  double U = p.x / Rs, V = p.y / Rs, W = p.z / Rs;
+__device__ __forceinline__ void hot_sphere_rotate(double Rs, double iRs, Hp& p, double phi, bool velocity) {
+  double U = div_known(p.x, Rs, iRs), V = div_known(p.y, Rs, iRs), W = div_known(p.z, Rs, iRs);
   double cs, sn;
   sincos(phi, &sn, &cs);
   double dot = U * p.nx + V * p.ny + W * p.nz;
   double nx = U * dot * (1.0 - cs) + p.nx * cs + (-W * p.ny + V * p.nz) * sn;
   double ny = V * dot * (1.0 - cs) + p.ny * cs + (W * p.nx - U * p.nz) * sn;
   double nz = W * dot * (1.0 - cs) + p.nz * cs + (-V * p.nx + U * p.ny) * sn;
-  double len = sqrt(nx * nx + ny * ny + nz * nz);
-  p.nx = nx / len; p.ny = ny / len; p.nz = nz / len;
+  set_unit(nx, ny, nz, p.nx, p.ny, p.nz);
   if (velocity) {
     double dv = U * p.vx + V * p.vy + W * p.vz;
     double vx = U * dv * (1.0 - cs) + p.vx * cs + (-W * p.vy + V * p.vz) * sn;
@@ -163,31 +160,32 @@ __device__ __forceinline__ void hot_sphere_rotate(double Rs, Hp& p, double phi, 
   }
 }
 
-// Box/constraint scalars the shape routines read (plane: box; sphere: Rs).
-struct ShapeGeom { double xlo, xhi, Lx, ylo, yhi, Ly, Rs; };
+// Box/constraint scalars the shape routines read (plane: box; sphere: radius
+// Rs and iRs = RN(1 / Rs)).
+struct ShapeGeom { double xlo, xhi, Lx, ylo, yhi, Ly, Rs, iRs; };
 
 __device__ __forceinline__ ShapeGeom geom_of(const Replica& R) {
-  return ShapeGeom{R.xlo, R.xhi, R.Lx, R.ylo, R.yhi, R.Ly, R.cons_p[0]};
+  return ShapeGeom{R.xlo, R.xhi, R.Lx, R.ylo, R.yhi, R.Ly, R.cons_p[0], 1.0 / R.cons_p[0]};
 }
 
 template <int SHAPE>
 __device__ __forceinline__ void hot_enforce(const ShapeGeom& G, Hp& p, int& dix, int& diy) {
   if (SHAPE == HOT_PLANE) hot_plane_enforce(G.xlo, G.xhi, G.Lx, G.ylo, G.yhi, G.Ly, p, dix, diy);
-  else hot_sphere_enforce(G.Rs, p);
+  else hot_sphere_enforce(G.Rs, G.iRs, p);
 }
 
 template <int SHAPE>
 __device__ __forceinline__ double hot_project_torque(const ShapeGeom& G, const Hp& p) {
   if (SHAPE == HOT_PLANE) return 0.0 + p.tz;
-  const double Rs = G.Rs;
-  double Nx = p.x / Rs, Ny = p.y / Rs, Nz = p.z / Rs;
+  const double Rs = G.Rs, iRs = G.iRs;
+  double Nx = div_known(p.x, Rs, iRs), Ny = div_known(p.y, Rs, iRs), Nz = div_known(p.z, Rs, iRs);
   return 0.0 + (p.tx * Nx + p.ty * Ny + p.tz * Nz);
 }
 
 template <int SHAPE>
 __device__ __forceinline__ void hot_rotate(const ShapeGeom& G, Hp& p, double phi, bool velocity) {
   if (SHAPE == HOT_PLANE) hot_plane_rotate(p, phi, velocity);
-  else hot_sphere_rotate(G.Rs, p, phi, velocity);
+  else hot_sphere_rotate(G.Rs, G.iRs, p, phi, velocity);
 }
 
 // ---------------------------------------------------------------------------
