@@ -67,6 +67,7 @@ struct sg_system {
   std::vector<Replica> reps_h;
   Replica* reps = nullptr;
   std::vector<Clock> clk_h;
+  bool clk_fresh = true;  // clk_h holds what the device holds (false while a run goes on)
   Clock* clk = nullptr;
   Program prog{};
   std::vector<double*> tables;
@@ -87,6 +88,8 @@ struct sg_system {
   int* pin_blist = nullptr;
   CellSeg* pin_segs = nullptr;
   int* pin_res = nullptr;
+  struct RunEnd { RebuildStats rb; int status, pad; };
+  RunEnd* pin_end = nullptr;  // followed by the clocks
   cudaEvent_t ev_pin = nullptr;
   bool b_pending = false;  // ev_b0 / ev_b1 bracket a rebuild not yet added to the run's rebuild time
   int nblist = 0;
@@ -97,7 +100,8 @@ struct sg_system {
   int *rebuild = nullptr, *status = nullptr, *maxnb = nullptr;
   int *bstatus = nullptr;   // list-build status (overflow), separate from the run's status word
   void* xfer = nullptr;     // staging for host transfers in particle-id order (largest replica)
-  int* xerr = nullptr;      // set by the transfer kernels on an id outside the replica
+  int* xerr = nullptr;      // page-locked: set by the transfer kernels on an id outside the replica
+  int* xinv = nullptr;      // slot of each particle id (largest replica)
   int *exec_cnt = nullptr;  // steps executed in a batch (batched stepping)
   int *fire_cnt = nullptr;  // per replica: blocks of k_fire_b done (the last one runs the FIRE control)
   int64_t since_rebuild = 0, last_gap = 8;  // batch length follows the steps between rebuilds
@@ -225,9 +229,12 @@ static int push_clk(sg_system* s) {
   CU(s, cudaMemcpyAsync(s->clk, s->clk_h.data(), sizeof(Clock) * s->nrep, cudaMemcpyHostToDevice, s->stream));
   return SG_OK;
 }
+// the host copy of the clocks, brought up to date where a run may have moved on
 static int pull_clk(sg_system* s) {
+  if (s->clk_fresh) return SG_OK;
   CU(s, cudaMemcpyAsync(s->clk_h.data(), s->clk, sizeof(Clock) * s->nrep, cudaMemcpyDeviceToHost, s->stream));
   CU(s, cudaStreamSynchronize(s->stream));
+  s->clk_fresh = true;
   return SG_OK;
 }
 
@@ -307,9 +314,12 @@ int sg_create(int n_replicas, const int32_t* n_particles, int ntypes, sg_system*
   cudaMallocHost((void**)&s->pin_blist, sizeof(int) * std::max(1, s->nblocks));
   cudaMallocHost((void**)&s->pin_segs, sizeof(CellSeg) * n_replicas);
   cudaMallocHost((void**)&s->pin_res, sizeof(int) * 2);
+  cudaMallocHost((void**)&s->pin_end, sizeof(sg_system::RunEnd) + sizeof(Clock) * n_replicas);
+  cudaMallocHost((void**)&s->xerr, sizeof(int));
   cudaEventCreateWithFlags(&s->ev_pin, cudaEventDisableTiming);
-  if (!s->rebuild_h || !s->pin_blist || !s->pin_segs || !s->pin_res) {
-    for (void* h : {(void*)s->rebuild_h, (void*)s->pin_blist, (void*)s->pin_segs, (void*)s->pin_res})
+  if (!s->rebuild_h || !s->pin_blist || !s->pin_segs || !s->pin_res || !s->pin_end || !s->xerr) {
+    for (void* h : {(void*)s->rebuild_h, (void*)s->pin_blist, (void*)s->pin_segs, (void*)s->pin_res, (void*)s->pin_end,
+                  (void*)s->xerr})
       if (h) cudaFreeHost(h);
     if (s->ev_pin) cudaEventDestroy(s->ev_pin);
     m.free_all(); cudaStreamDestroy(s->stream); delete s; return SG_ERR_NOMEM;
@@ -363,7 +373,8 @@ int sg_destroy(sg_system* s) {
   cudaStreamSynchronize(s->stream);
   s->mem.free_all();
   for (double* t : s->tables) cudaFree(t);
-  for (void* h : {(void*)s->rebuild_h, (void*)s->pin_blist, (void*)s->pin_segs, (void*)s->pin_res})
+  for (void* h : {(void*)s->rebuild_h, (void*)s->pin_blist, (void*)s->pin_segs, (void*)s->pin_res, (void*)s->pin_end,
+                  (void*)s->xerr})
     if (h) cudaFreeHost(h);
   if (s->ev_pin) cudaEventDestroy(s->ev_pin);
   for (cudaEvent_t ev : {s->ev_run0, s->ev_run1, s->ev_k0, s->ev_k1, s->ev_t0, s->ev_t1, s->ev_b0, s->ev_b1})
@@ -419,7 +430,7 @@ __global__ void k_gather_ids(T* __restrict__ dst, const T* __restrict__ src, con
   if (k >= n) return;
   const int i = id[k];
   if ((unsigned)i < (unsigned)n) dst[k] = src[i];
-  else atomicOr(err, 1);
+  else *err = 1;
 }
 
 template <class T>
@@ -429,7 +440,60 @@ __global__ void k_scatter_ids(T* __restrict__ dst, const T* __restrict__ src, co
   if (k >= n) return;
   const int i = id[k];
   if ((unsigned)i < (unsigned)n) dst[i] = src[k];
-  else atomicOr(err, 1);
+  else *err = 1;
+}
+
+// Small multi-field transfers between page-locked host arrays and the slots,
+// without a copy per field: the kernels read or write the host arrays
+// themselves, every field in one launch.  A copy costs 5 us of latency
+// whatever its size, so a replica of 16,000 particles took 117 us for nine
+// fields (nine scatters, nine copies) and takes two launches now.  Host
+// accesses are consecutive (an id-order pass), slot accesses permuted.
+constexpr int XFER_FIELDS = 24;
+struct XferFields {
+  void* dev[XFER_FIELDS];
+  void* host[XFER_FIELDS];
+  unsigned ints;  // bit f: field f is int32
+};
+
+__global__ void k_inv_ids(int* __restrict__ inv, const int* __restrict__ id, int n, int* err) {
+  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= n) return;
+  const int i = id[k];
+  if ((unsigned)i < (unsigned)n) inv[i] = k;
+  else *err = 1;
+}
+
+__global__ void k_fields_out(XferFields F, const int* __restrict__ inv, int n, int* err) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x, f = blockIdx.y;
+  if (i >= n) return;
+  const int k = inv[i];
+  if ((unsigned)k >= (unsigned)n) { *err = 1; return; }
+  if (F.ints >> f & 1) static_cast<int*>(F.host[f])[i] = static_cast<const int*>(F.dev[f])[k];
+  else static_cast<double*>(F.host[f])[i] = static_cast<const double*>(F.dev[f])[k];
+}
+
+__global__ void k_fields_in(XferFields F, const int* __restrict__ inv, int n, int* err) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x, f = blockIdx.y;
+  if (i >= n) return;
+  const int k = inv[i];
+  if ((unsigned)k >= (unsigned)n) { *err = 1; return; }
+  if (F.ints >> f & 1) static_cast<int*>(F.dev[f])[k] = static_cast<const int*>(F.host[f])[i];
+  else static_cast<double*>(F.dev[f])[k] = static_cast<const double*>(F.host[f])[i];
+}
+
+// host memory that a kernel can address, from its first byte to its last
+static void* device_view(const void* host, size_t bytes) {
+  cudaPointerAttributes a{}, b{};
+  if (cudaPointerGetAttributes(&a, host) != cudaSuccess ||
+      cudaPointerGetAttributes(&b, static_cast<const char*>(host) + bytes - 1) != cudaSuccess) {
+    cudaGetLastError();
+    return nullptr;
+  }
+  if (a.type != cudaMemoryTypeHost || b.type != cudaMemoryTypeHost || !a.devicePointer || !b.devicePointer ||
+      static_cast<char*>(b.devicePointer) - static_cast<char*>(a.devicePointer) != (ptrdiff_t)bytes - 1)
+    return nullptr;
+  return a.devicePointer;
 }
 
 static int xfer_ready(sg_system* s) {
@@ -437,7 +501,7 @@ static int xfer_ready(sg_system* s) {
   int maxn = 0;
   for (int v : s->n) maxn = std::max(maxn, v);
   s->xfer = s->mem.alloc<double>(std::max(1, maxn));
-  s->xerr = s->mem.alloc<int>(1);
+  s->xinv = s->mem.alloc<int>(std::max(1, maxn));
   if (s->mem.err != cudaSuccess) { s->mem.err = cudaSuccess; return fail(s, SG_ERR_NOMEM, "transfer staging allocation failed"); }
   return SG_OK;
 }
@@ -451,7 +515,7 @@ static int xfer_field(sg_system* s, int replica, T* dev, T* host, bool to_device
   if (n == 0) return SG_OK;
   T* stage = (T*)s->xfer;
   const int g = (n + 255) / 256;
-  CU(s, cudaMemsetAsync(s->xerr, 0, sizeof(int), s->stream));
+  *s->xerr = 0;
   if (to_device) {
     CU(s, cudaMemcpyAsync(stage, host, sizeof(T) * n, cudaMemcpyHostToDevice, s->stream));
     k_gather_ids<T><<<g, 256, 0, s->stream>>>(dev + off, stage, s->st.id + off, n, s->xerr);
@@ -460,10 +524,8 @@ static int xfer_field(sg_system* s, int replica, T* dev, T* host, bool to_device
     CU(s, cudaMemcpyAsync(host, stage, sizeof(T) * n, cudaMemcpyDeviceToHost, s->stream));
   }
   CU(s, cudaGetLastError());
-  int bad = 0;
-  CU(s, cudaMemcpyAsync(&bad, s->xerr, sizeof(int), cudaMemcpyDeviceToHost, s->stream));
   CU(s, cudaStreamSynchronize(s->stream));
-  if (bad) return fail(s, SG_ERR_STATE, "corrupt id map");
+  if (*s->xerr) return fail(s, SG_ERR_STATE, "corrupt id map");
   return SG_OK;
 }
 
@@ -484,6 +546,11 @@ static int field_ptr(sg_system* s, const char* field, void** p, bool* is_int, in
   }
   return fail(s, SG_ERR_ARG, std::string("unknown particle field '") + field + "'");
 }
+
+// Nine fields from page-locked arrays, one copy per field against the two
+// kernels: 0.07 MB 91 and 39 us, 4.7 MB 174 and 126, 19 MB 425 and 396, 38 MB
+// both 760.
+static constexpr size_t kDirectBytes = 16 << 20;
 
 // Staging for `nf` fields of a replica (grown on demand, kept).
 static int xfer_multi_ready(sg_system* s, int nf) {
@@ -523,13 +590,36 @@ static int xfer_fields(sg_system* s, int replica, int nf, const char* const* fie
         if (h[k] < 1 || h[k] > s->ntypes) return fail(s, SG_ERR_ARG, "particle type outside 1..ntypes");
     }
   }
-  int rc = xfer_multi_ready(s, nf);
+  int rc = xfer_ready(s);
   if (rc) return rc;
   const int n = s->n[replica], off = s->off[replica];
   if (n == 0) return SG_OK;
   const int g = (n + 255) / 256;
   const size_t slice = (size_t)std::max(1, n);
-  CU(s, cudaMemsetAsync(s->xerr, 0, sizeof(int), s->stream));
+  size_t bytes = 0;
+  XferFields F{};
+  bool direct = nf <= XFER_FIELDS;
+  for (int i = 0; i < nf && direct; i++) {
+    const size_t b = (ints[i] ? sizeof(int) : sizeof(double)) * (size_t)n;
+    bytes += b;
+    direct = staged[i] && bytes <= kDirectBytes && (F.host[i] = device_view(hosts[i], b)) != nullptr &&
+             reinterpret_cast<uintptr_t>(F.host[i]) % (ints[i] ? sizeof(int) : sizeof(double)) == 0;
+    F.dev[i] = ints[i] ? (void*)((int*)dps[i] + off) : (void*)((double*)dps[i] + off);
+    if (ints[i]) F.ints |= 1u << i;
+  }
+  if (direct) {
+    *s->xerr = 0;
+    k_inv_ids<<<g, 256, 0, s->stream>>>(s->xinv, s->st.id + off, n, s->xerr);
+    if (to_device) k_fields_in<<<dim3(g, nf), 256, 0, s->stream>>>(F, s->xinv, n, s->xerr);
+    else k_fields_out<<<dim3(g, nf), 256, 0, s->stream>>>(F, s->xinv, n, s->xerr);
+    CU(s, cudaGetLastError());
+    CU(s, cudaStreamSynchronize(s->stream));
+    if (*s->xerr) return fail(s, SG_ERR_STATE, "corrupt id map");
+    if (to_device) { s->e1_applied = false; s->forces_fresh = false; }
+    return SG_OK;
+  }
+  if ((rc = xfer_multi_ready(s, nf))) return rc;
+  *s->xerr = 0;
   if (to_device) {
     for (int i = 0; i < nf; i++)
       if (staged[i])
@@ -560,10 +650,8 @@ static int xfer_fields(sg_system* s, int replica, int nf, const char* const* fie
                               cudaMemcpyDeviceToHost, s->stream));
   }
   CU(s, cudaGetLastError());
-  int bad = 0;
-  CU(s, cudaMemcpyAsync(&bad, s->xerr, sizeof(int), cudaMemcpyDeviceToHost, s->stream));
   CU(s, cudaStreamSynchronize(s->stream));
-  if (bad) return fail(s, SG_ERR_STATE, "corrupt id map");
+  if (*s->xerr) return fail(s, SG_ERR_STATE, "corrupt id map");
   for (int i = 0; i < nf; i++)  // surface normals: the one-field path
     if (!staged[i]) {
       rc = to_device ? sg_upload(s, replica, fields[i], hosts[i]) : sg_download(s, replica, fields[i], hosts[i]);
@@ -2160,6 +2248,7 @@ static int run_fire_batch(sg_system* s, int64_t K, bool needs_nl, int64_t* execu
       if ((rc = rebuild_pending(s, HOT_NONE, false, rebuild_ms))) return rc;
     }
   }
+  s->clk_fresh = false;
   if ((rc = pull_clk(s))) return rc;
   bool all = true;
   for (int r = 0; r < s->nrep; r++) all = all && s->clk_h[r].fire_conv_step >= 0;
@@ -2215,6 +2304,8 @@ static int run_impl(sg_system* s, int64_t steps, sg_run_stats* stats, bool drive
     step0 = s->clk_h[0].time_step;
   }
   int64_t done = 0;
+  bool last_flags = false;
+  s->clk_fresh = false;
   for (int64_t t = 0; t <= steps; t++) {
     const bool last = (t == steps);
     int rc;
@@ -2307,10 +2398,14 @@ static int run_impl(sg_system* s, int64_t steps, sg_run_stats* stats, bool drive
     s->since_rebuild++;
     if (needs_nl) {
       CU(s, cudaMemcpyAsync(s->rebuild_h, s->rebuild, sizeof(int) * s->nrep, cudaMemcpyDeviceToHost, s->stream));
-      CU(s, cudaStreamSynchronize(s->stream));
-      if ((rc = rebuild_pending(s, shape, last, &rebuild_ms))) return rc;
+      if (last && !driver) last_flags = true;  // read after the loop
+      else {
+        CU(s, cudaStreamSynchronize(s->stream));
+        if ((rc = rebuild_pending(s, shape, last, &rebuild_ms))) return rc;
+      }
     }
     if (driver && ((t & 15) == 15 || t == steps)) {  // converged replicas are frozen on the device
+      s->clk_fresh = false;
       if ((rc = pull_clk(s))) return rc;
       bool all = true;
       for (int r = 0; r < s->nrep; r++) all = all && s->clk_h[r].fire_conv_step >= 0;
@@ -2318,21 +2413,36 @@ static int run_impl(sg_system* s, int64_t steps, sg_run_stats* stats, bool drive
       if ((rc = refresh_active(s))) return rc;
     }
   }
+  // one wait for the run's results: status, rebuild statistics, clocks, and
+  // the last step's rebuild flags (enqueued in the loop)
   CU(s, cudaEventRecord(s->ev_run1, s->stream));
-  int st = 0;
-  RebuildStats rbs{};
-  CU(s, cudaMemcpyAsync(&st, s->status, sizeof(int), cudaMemcpyDeviceToHost, s->stream));
-  if (s->rb_used) CU(s, cudaMemcpyAsync(&rbs, s->rb_stats, sizeof(rbs), cudaMemcpyDeviceToHost, s->stream));
+  CU(s, cudaMemcpyAsync(&s->pin_end->status, s->status, sizeof(int), cudaMemcpyDeviceToHost, s->stream));
+  if (s->rb_used)
+    CU(s, cudaMemcpyAsync(&s->pin_end->rb, s->rb_stats, sizeof(RebuildStats), cudaMemcpyDeviceToHost, s->stream));
+  CU(s, cudaMemcpyAsync(s->pin_end + 1, s->clk, sizeof(Clock) * s->nrep, cudaMemcpyDeviceToHost, s->stream));
   CU(s, cudaStreamSynchronize(s->stream));
-  s->builds_run += rbs.builds;
-  s->maxnb_seen = std::max(s->maxnb_seen, rbs.maxnb);
-  rebuild_ms += 1e-6 * (double)rbs.ns;
+  if (last_flags) {
+    bool any = false;
+    for (int r = 0; r < s->nrep; r++) any = any || s->rebuild_h[r];
+    if (any) {
+      if (int rcb = rebuild_pending(s, shape, true, &rebuild_ms)) return rcb;
+      CU(s, cudaEventRecord(s->ev_run1, s->stream));
+      CU(s, cudaStreamSynchronize(s->stream));
+    }
+  }
+  const int st = s->pin_end->status;
+  if (s->rb_used) {
+    const RebuildStats& rbs = s->pin_end->rb;
+    s->builds_run += rbs.builds;
+    s->maxnb_seen = std::max(s->maxnb_seen, rbs.maxnb);
+    rebuild_ms += 1e-6 * (double)rbs.ns;
+  }
   if (st & ST_TIMEOUT) return grid_timeout(s);
   float run_ms = 0.f;
   CU(s, cudaEventElapsedTime(&run_ms, s->ev_run0, s->ev_run1));
   if (int rcb = flush_rebuild_time(s, &rebuild_ms)) return rcb;
-  int rc = pull_clk(s);
-  if (rc) return rc;
+  std::memcpy(s->clk_h.data(), s->pin_end + 1, sizeof(Clock) * s->nrep);
+  s->clk_fresh = true;
   if (conv_out)
     for (int r = 0; r < s->nrep; r++) conv_out[r] = s->clk_h[r].fire_conv_step >= 0 ? s->clk_h[r].fire_conv_step + 1 : -1;
   if (stats) {
