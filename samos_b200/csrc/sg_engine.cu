@@ -3,7 +3,7 @@
 // once per configuration and reused by every step.
 #include "samos_gpu.h"
 #include "sg_abp_launch.h"
-#include "sg_rebuild.cuh"
+#include "sg_flow.cuh"
 
 #include <algorithm>
 #include <cmath>
@@ -61,6 +61,12 @@ struct sg_system {
   int* rb_bsum = nullptr;
   unsigned long long* run_word = nullptr;  // step barrier of the resident run
   int run_per_sm = 0, run_kind = -1;       // its blocks per SM, and for which kernel
+  // two-launch Langevin / NVE / FIRE steps (sg_flow.cuh): positions and
+  // directors are in G[hot_buf] while flow_on
+  bool flow_on = false;
+  FlowConst* flow_fc = nullptr;
+  FlowKind flow_k{-1, 0, 0};
+  int flow_grid = 0;
   int rb_grid[3] = {0, 0, 0};  // blocks that fit the device at once, per shape
   bool rb_used = false;        // in the current run
   int *rep_blk0 = nullptr, *rep_nblk = nullptr;
@@ -299,7 +305,7 @@ int sg_create(int n_replicas, const int32_t* n_particles, int ntypes, sg_system*
   s->rebuild = m.alloc<int>(n_replicas);
   s->status = m.alloc<int>(1);
   s->bstatus = m.alloc<int>(1);
-  s->exec_cnt = m.alloc<int>(1);
+  s->exec_cnt = m.alloc<int>(2);
   s->fire_cnt = m.alloc<int>(n_replicas);
   s->maxnb = m.alloc<int>(1);
   s->epart = m.alloc<double>((size_t)(MAX_PAIR + MAX_ALIGN) * s->nblocks);
@@ -2199,14 +2205,119 @@ static int run_batch_unfused(sg_system* s, int64_t K, bool needs_nl, int64_t* ex
   return rebuild_pending(s, HOT_NONE, false, rebuild_ms);
 }
 
+// Langevin (BAOAB, BBK; constant temperature), NVE and FIRE on a periodic
+// plane whose forces can be reused from step to step: two launches a step with
+// the rebuilds enqueued (sg_flow.cuh).  NVE ensembles with aligners keep the
+// unfused path, which evaluates every replica's torques again when one of them
+// has rebuilt.
+static bool flow_program(const sg_system* s) {
+  const Program& P = s->prog;
+  if (!dev_rebuild(s) || P.ninteg != 1 || P.integ[0].group) return false;
+  for (int c = 0; c < P.nalign; c++)
+    if (P.align[c].kind == ALIGN_VICSEK) return false;
+  if (P.integ[0].kind == INT_FIRE) return fire_forces_reusable(s);
+  if (!integ_forces_reusable(s)) return false;
+  if (P.integ[0].kind == INT_LANGEVIN && P.integ[0].temp.kind != 0) return false;
+  return !(P.integ[0].kind == INT_NVE && P.nalign && s->nrep > 1);
+}
+
+// puts the records' fields back into the store (any other path reads that)
+static int flow_leave(sg_system* s) {
+  if (!s->flow_on) return SG_OK;
+  s->flow_on = false;
+  return hot_unpack(s, HOT_PLANE);
+}
+
+static int run_flow(sg_system* s, int64_t K, bool driver, int64_t* executed, double* rebuild_ms) {
+  int rc = dev_rebuild_ready(s);
+  if (rc) return rc;
+  const Program& P = s->prog;
+  const FlowKind kind = flow_kind(P);
+  if (kind.integ != s->flow_k.integ || kind.pair != s->flow_k.pair || kind.align != s->flow_k.align) {
+    int per = 0;
+    CU(s, flow_begin_blocks(kind, &per));
+    if (per < 1) return fail(s, SG_ERR_CUDA, "two-launch step does not fit the device");
+    s->flow_grid = std::min(148 * 16, per * s->sms);
+    s->flow_k = kind;
+  }
+  const int* al = driver && s->nact < s->nblocks ? s->act : nullptr;
+  const int na = driver ? s->nact : s->nblocks;
+  // start-of-step forces that are not those of the last step's own pass
+  const bool fresh = s->forces_fresh;
+  if (!fresh) {
+    if ((rc = flow_leave(s))) return rc;
+    if (!s->e1_applied) {
+      k_enforce<<<na, BLOCK, 0, s->stream>>>(s->prog, s->reps, s->blk_rep, s->cur, s->st, driver ? s->clk : nullptr, al);
+      LAUNCH_CHECK(s);
+    }
+    if ((rc = launch_force(s, s->dt_global, false, true, true, false, na, al))) return rc;
+  }
+  s->e1_applied = false;
+  if ((rc = hot_alloc(s, HOT_PLANE))) return rc;
+  if (!s->flow_on && (rc = hot_pack(s, HOT_PLANE))) return rc;
+  s->flow_on = true;
+  FlowArgs A{};
+  if (kind.integ == FLOW_LANGEVIN) {
+    if (!s->flow_fc) s->flow_fc = s->mem.alloc<FlowConst>(s->nrep);
+    if (!s->flow_fc) { s->mem.err = cudaSuccess; return fail(s, SG_ERR_NOMEM, "integrator constants"); }
+    CU(s, flow_const(P, s->reps, s->nrep, s->flow_fc, s->stream));
+    s->launches++;
+  }
+  if (kind.integ == FLOW_FIRE && s->fire_ordered && !s->fire_terms) {
+    s->fire_terms = s->mem.alloc<double>((size_t)3 * s->slots);
+    if (!s->fire_terms) { s->mem.err = cudaSuccess; return fail(s, SG_ERR_NOMEM, "FIRE term arrays"); }
+  }
+  A.reps = s->reps; A.blk_rep = s->blk_rep; A.clk = s->clk;
+  A.st = s->st; A.nl = s->nl; A.rebuild = s->rebuild; A.status = s->status; A.fc = s->flow_fc; A.Rn = s->Rn;
+  A.epart = s->epart; A.part = s->fire_part; A.alpha_mix = s->alpha_mix;
+  A.terms = s->fire_ordered ? s->fire_terms : nullptr; A.terms_stride = s->slots;
+  A.rep_blk0 = s->rep_blk0; A.rep_nblk = s->rep_nblk; A.fire_cnt = s->fire_cnt;
+  A.nblocks = s->nblocks; A.driver = driver ? 1 : 0;
+  A.blist = al; A.nblist = na; A.d = s->cur;
+  const bool flips = kind.integ != FLOW_LANGEVIN;  // the force pass writes the other record buffer
+  const int b0 = s->hot_buf, grid = std::max(1, std::min(s->flow_grid, na));
+  CU(s, cudaMemsetAsync(s->exec_cnt, 0, 2 * sizeof(int), s->stream));
+  A.Gin = A.G = s->G[b0];
+  CU(s, flow_begin(kind, P, A, rebuild_args(s, HOT_PLANE), kSortEvery, false, true, fresh, grid, s->stream));
+  s->launches++;
+  for (int64_t i = 0; i < K; i++) {
+    A.Gin = s->G[s->hot_buf];
+    if (flips) s->hot_buf = 1 - s->hot_buf;
+    A.G = s->G[s->hot_buf];
+    CU(s, flow_force(kind, P, A, s->stream));
+    CU(s, flow_begin(kind, P, A, rebuild_args(s, HOT_PLANE), kSortEvery, true, i + 1 < K, true, grid, s->stream));
+    s->launches += 2;
+  }
+  int ex[2] = {0, 0}, st = 0;
+  CU(s, cudaMemcpyAsync(ex, s->exec_cnt, sizeof(ex), cudaMemcpyDeviceToHost, s->stream));
+  CU(s, cudaMemcpyAsync(&st, s->status, sizeof(int), cudaMemcpyDeviceToHost, s->stream));
+  CU(s, cudaMemcpyAsync(s->rebuild_h, s->rebuild, sizeof(int) * s->nrep, cudaMemcpyDeviceToHost, s->stream));
+  CU(s, cudaStreamSynchronize(s->stream));
+  if (st & ST_TIMEOUT) return grid_timeout(s);
+  if (ex[0] < 1 || ex[0] > K) return fail(s, SG_ERR_CUDA, "two-launch steps: inconsistent step count");
+  if (flips) s->hot_buf = b0 ^ (int)(ex[0] & 1);
+  *executed = ex[0];
+  s->since_rebuild += ex[0];
+  s->forces_fresh = ex[1] == 0;
+  bool any = false;
+  for (int r = 0; r < s->nrep; r++) any = any || s->rebuild_h[r];
+  if (!any) return SG_OK;
+  // lists that did not fit: grown and rebuilt by the host
+  if ((rc = flow_leave(s))) return rc;
+  k_set_halt<<<(s->nrep + 127) / 128, 128, 0, s->stream>>>(s->clk, s->nrep, 0);
+  LAUNCH_CHECK(s);
+  return rebuild_pending(s, HOT_NONE, false, rebuild_ms);
+}
+
 // Blocks of the replicas whose minimiser has not converged (from clk_h).
 static int refresh_active(sg_system* s) {
-  s->act_h.clear();
+  std::vector<int> before;
+  before.swap(s->act_h);
   for (int r = 0; r < s->nrep; r++)
     if (s->clk_h[r].fire_conv_step < 0)
       for (int b = 0; b < s->rep_nblk_h[r]; b++) s->act_h.push_back(s->rep_blk0_h[r] + b);
   s->nact = (int)s->act_h.size();
-  if (s->nact == s->nblocks || s->nact == 0) return SG_OK;
+  if (s->nact == s->nblocks || s->nact == 0 || (s->act && s->act_h == before)) return SG_OK;
   if (!s->act) {
     s->act = s->mem.alloc<int>(s->nblocks);
     if (!s->act) { s->mem.err = cudaSuccess; return fail(s, SG_ERR_NOMEM, "active block list"); }
@@ -2303,6 +2414,8 @@ static int run_impl(sg_system* s, int64_t steps, sg_run_stats* stats, bool drive
     if (rcp) return rcp;
     step0 = s->clk_h[0].time_step;
   }
+  const bool flow = !fused && flow_program(s);
+  s->flow_on = false;
   int64_t done = 0;
   bool last_flags = false;
   s->clk_fresh = false;
@@ -2330,6 +2443,21 @@ static int run_impl(sg_system* s, int64_t steps, sg_run_stats* stats, bool drive
       else rc = hot_pack(s, shape);
       if (rc) return rc;
     }
+    if (!fused && !resc && !last && needs_nl && flow) {
+      int64_t ex = 0;
+      if ((rc = run_flow(s, std::min<int64_t>(driver ? 16 : kBatchDev, steps - t), driver, &ex, &rebuild_ms))) return rc;
+      done += ex;
+      t += ex - 1;
+      if (!driver) continue;
+      s->clk_fresh = false;
+      if ((rc = pull_clk(s))) return rc;
+      bool all = true;
+      for (int r = 0; r < s->nrep; r++) all = all && s->clk_h[r].fire_conv_step >= 0;
+      if (all) break;
+      if ((rc = refresh_active(s))) return rc;
+      continue;
+    }
+    if ((rc = flow_leave(s))) return rc;
     if (driver && t > 0 && !last && K > 1 && !s->profile && !resc) {
       int64_t ex = 0;
       bool all = false;
@@ -2413,6 +2541,7 @@ static int run_impl(sg_system* s, int64_t steps, sg_run_stats* stats, bool drive
       if ((rc = refresh_active(s))) return rc;
     }
   }
+  if (int rcf = flow_leave(s)) return rcf;
   // one wait for the run's results: status, rebuild statistics, clocks, and
   // the last step's rebuild flags (enqueued in the loop)
   CU(s, cudaEventRecord(s->ev_run1, s->stream));

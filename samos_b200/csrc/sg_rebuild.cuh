@@ -97,20 +97,25 @@ struct RebuildList {
   int blk[RB_MAX_REP + 1], cell[RB_MAX_REP + 1];  // first virtual block / cell of each
 };
 
-// Reads the flags; false when no replica is flagged.
-__device__ __forceinline__ bool rebuild_list(const RebuildArgs& A, int sort_every, RebuildList& L) {
+// Reads the flags; false when no replica is flagged.  running_only: not the
+// replicas whose minimiser has converged.
+__device__ __forceinline__ bool rebuild_list(const RebuildArgs& A, int sort_every, RebuildList& L,
+                                             bool running_only = false) {
   __shared__ int any;
   if (threadIdx.x == 0) any = 0;
   __syncthreads();
+  auto flagged = [&](int r) {
+    return __ldcg(A.rebuild + r) != 0 && !(running_only && A.clk[r].fire_conv_step >= 0);
+  };
   for (int r = threadIdx.x; r < A.nrep; r += blockDim.x)
-    if (__ldcg(A.rebuild + r)) any = 1;
+    if (flagged(r)) any = 1;
   __syncthreads();
   if (!any) return false;
   if (threadIdx.x < 32) {  // one warp puts the flagged replicas in order
     int n = 0, nb = 0, nc = 0, srt = 0;
     for (int r0 = 0; r0 < A.nrep; r0 += 32) {
       const int r = r0 + threadIdx.x;
-      const bool f = r < A.nrep && __ldcg(A.rebuild + r) != 0;
+      const bool f = r < A.nrep && flagged(r);
       const unsigned m = __ballot_sync(0xffffffffu, f);
       int b = f ? A.rep_nblk[r] : 0, c = f ? A.reps[r].ncell : 0;
       const int b_own = b, c_own = c;
