@@ -25,16 +25,6 @@ constexpr int RUN_NB = 16;
 // steps, arrivals in the low half and blocks that ask for a rebuild in the high
 // half.  A block that is one step ahead writes the other word, so every block
 // of a step reads the same requests.
-__device__ __forceinline__ unsigned long long ld_acquire64(const unsigned long long* p) {
-  unsigned long long v;
-  asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
-  return v;
-}
-
-__device__ __forceinline__ void red_release64(unsigned long long* p, unsigned long long v) {
-  asm volatile("red.release.gpu.global.add.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
-}
-
 template <int SHAPE, int ALIGN, bool SP, bool BYVAL>
 __global__ void __launch_bounds__(BLOCK, ABP_RUN_MINB)
 k_abp_run(const AbpParams* __restrict__ prm, const __grid_constant__ AbpParams pv, const int* __restrict__ blk_rep,
@@ -63,7 +53,7 @@ k_abp_run(const AbpParams* __restrict__ prm, const __grid_constant__ AbpParams p
   const uint64_t draws = (uint64_t)S.n * (uint64_t)((S.nematic ? 1 : 0) + D);
   uint64_t base = s_ctr;
 
-  GridBar bar{A.bar, 0u, A.status};
+  GridBar bar{A.bar, gridDim.x, 0u, 0u, A.status};
   unsigned long long asked[2] = {0ull, 0ull};
   unsigned target[2] = {0u, 0u};
 

@@ -99,8 +99,40 @@ cudaError_t flow_begin(const FlowKind& K, const Program& P, const FlowArgs& A, c
   return flow_dispatch(K, LaunchBegin{P, A, B, sort_every, tail, begin, pre, grid, stream});
 }
 
-cudaError_t flow_begin_blocks(const FlowKind& K, int* blocks_per_sm) {
+cudaError_t flow_begin_occupancy(const FlowKind& K, int* blocks_per_sm) {
   return flow_dispatch(K, BeginBlocks{blocks_per_sm});
+}
+
+struct LaunchRun {
+  const Program& P;
+  const FlowArgs& A;
+  const RebuildArgs& B;
+  D4 *G0, *G1;
+  unsigned long long* word;
+  int nsteps, sort_every, pre, grid;
+  cudaStream_t stream;
+  template <int I, int Q, int L> cudaError_t operator()() const {
+    LaunchRun a = *this;
+    void* args[] = {const_cast<Program*>(&P), const_cast<FlowArgs*>(&A), const_cast<RebuildArgs*>(&B), &a.G0, &a.G1,
+                    &a.word, &a.nsteps, &a.sort_every, &a.pre};
+    return cudaLaunchCooperativeKernel((const void*)k_flow_run<I, Q, L>, dim3(grid), dim3(BLOCK), args, 0, stream);
+  }
+};
+
+struct RunBlocks {
+  int* per;
+  template <int I, int Q, int L> cudaError_t operator()() const {
+    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(per, (const void*)k_flow_run<I, Q, L>, BLOCK, 0);
+  }
+};
+
+cudaError_t flow_run(const FlowKind& K, const Program& P, const FlowArgs& A, const RebuildArgs& B, D4* G0, D4* G1,
+                     unsigned long long* word, int nsteps, int sort_every, bool pre, int grid, cudaStream_t stream) {
+  return flow_dispatch(K, LaunchRun{P, A, B, G0, G1, word, nsteps, sort_every, pre, grid, stream});
+}
+
+cudaError_t flow_run_occupancy(const FlowKind& K, int* blocks_per_sm) {
+  return flow_dispatch(K, RunBlocks{blocks_per_sm});
 }
 
 }  // namespace sg

@@ -18,6 +18,7 @@
 namespace sg {
 
 enum { FLOW_LANGEVIN = 0, FLOW_NVE = 1, FLOW_FIRE = 2 };
+constexpr int FLOW_RUN_MINB = 6;  // resident runs: blocks per SM that the registers are bounded for
 constexpr int FLOW_ANY = -2;  // pair kind or aligner taken from the program (several components, types)
 
 // per-replica constants of a Langevin integrator at constant temperature
@@ -30,7 +31,7 @@ struct FlowArgs {
   const int* blk_rep;
   Clock* clk;
   const D4* Gin;  // k_flow_force
-  D4* G;          // records written (k_flow_force: NVE, FIRE) and moved on (k_flow_begin)
+  D4* G;          // records written (k_flow_force: NVE) and moved on (k_flow_begin)
   Dyn d;
   Stat st;
   NbList nl;
@@ -53,7 +54,11 @@ cudaError_t flow_const(const Program& P, const Replica* reps, int nrep, FlowCons
 cudaError_t flow_force(const FlowKind& K, const Program& P, const FlowArgs& A, cudaStream_t stream);
 cudaError_t flow_begin(const FlowKind& K, const Program& P, const FlowArgs& A, const RebuildArgs& B, int sort_every,
                        bool tail, bool begin, bool pre, int grid, cudaStream_t stream);
-cudaError_t flow_begin_blocks(const FlowKind& K, int* blocks_per_sm);
+cudaError_t flow_begin_occupancy(const FlowKind& K, int* blocks_per_sm);
+// many steps in one cooperative launch of `grid` blocks, state in G0
+cudaError_t flow_run(const FlowKind& K, const Program& P, const FlowArgs& A, const RebuildArgs& B, D4* G0, D4* G1,
+                     unsigned long long* word, int nsteps, int sort_every, bool pre, int grid, cudaStream_t stream);
+cudaError_t flow_run_occupancy(const FlowKind& K, int* blocks_per_sm);
 
 // ---------------------------------------------------------------------------
 // forces (and torque) of slot k, neighbours in list order; PAIR / ALIGN fixed
@@ -143,16 +148,17 @@ __device__ __forceinline__ bool flow_left_skin(const Replica& R, const NbList& n
 }
 
 // ---------------------------------------------------------------------------
-// Force pass and second half of a step.
+// Force pass and second half of a step for one block of particles; true when
+// one of this thread's has left its skin.  step: steps since the clocks were
+// last advanced.
 // ---------------------------------------------------------------------------
-template <int INTEG, int PAIR, int ALIGN>
-__global__ void __launch_bounds__(BLOCK, 8)
-k_flow_force(const __grid_constant__ Program P, const __grid_constant__ FlowArgs A) {
-  const int bid = A.blist ? A.blist[blockIdx.x] : (int)blockIdx.x;
+template <int INTEG, int PAIR, int ALIGN, bool COH>
+__device__ __forceinline__ bool flow_force_block(const Program& P, const FlowArgs& A, const D4* Gin, D4* Gout, int bid,
+                                                 int step) {
   const int r = A.blk_rep[bid];
   const Clock& C = A.clk[r];
-  if (C.halt) return;
-  if (INTEG == FLOW_FIRE && C.fire_conv_step >= 0) return;  // frozen (its partials are kept)
+  if (INTEG == FLOW_FIRE && C.fire_conv_step >= 0) return false;  // frozen (its partials are kept)
+  bool left = false;
   const Replica& R = A.reps[r];
   const int k = bid * BLOCK + threadIdx.x;
   const double* ip = R.integ_p[0];
@@ -161,9 +167,9 @@ k_flow_force(const __grid_constant__ Program P, const __grid_constant__ FlowArgs
   for (int i = 0; i < MAX_PAIR; i++) e[i] = 0.0;
   double v3[3] = {0.0, 0.0, 0.0}, fmax2 = 0.0;
   if (k - R.off < R.n) {
-    D4 g = ldg4(A.Gin + k);
+    D4 g = ld_rec<COH>(Gin + k);
     double fx, fy, tz;
-    flow_gather<PAIR, ALIGN, INTEG == FLOW_FIRE, false>(P, R, A.Gin, A.st, A.nl, k, g, fx, fy, tz, e);
+    flow_gather<PAIR, ALIGN, INTEG == FLOW_FIRE, COH>(P, R, Gin, A.st, A.nl, k, g, fx, fy, tz, e);
     A.d.fx[k] = fx; A.d.fy[k] = fy;
     double vx = A.d.vx[k], vy = A.d.vy[k];
     int dix = 0, diy = 0;
@@ -177,7 +183,7 @@ k_flow_force(const __grid_constant__ Program P, const __grid_constant__ FlowArgs
         vy = one_div_one_p_dt2 * (vy + dt2_over_mass * fy);
         if (B != 0.0) {
           const double stoch_fact = 0.5 * B * one_div_one_p_dt2 / sqrt(mass);
-          const uint64_t c0 = C.ctr[0] + (uint64_t)A.st.id[k] * 3u;
+          const uint64_t c0 = C.ctr[0] + (uint64_t)step * A.fc[r].draws + (uint64_t)A.st.id[k] * 3u;
           const size_t gi = (size_t)R.off + (size_t)A.st.id[k];
           const double rx = noise_gauss(R.seed[0], c0 + 0), ry = noise_gauss(R.seed[0], c0 + 1);
           A.Rn[3 * gi + 0] = rx; A.Rn[3 * gi + 1] = ry; A.Rn[3 * gi + 2] = noise_gauss(R.seed[0], c0 + 2);
@@ -207,7 +213,7 @@ k_flow_force(const __grid_constant__ Program P, const __grid_constant__ FlowArgs
       A.d.omega[k] = omega;
       A.d.tz[k] = tz;
       A.d.age[k] += dt;
-      stg4(A.G + k, g);
+      stg4(Gout + k, g);
     } else {  // k_fire_b
       const double dt_2 = 0.5 * C.fire_dt;
       vx += dt_2 * fx; vy += dt_2 * fy;
@@ -219,17 +225,17 @@ k_flow_force(const __grid_constant__ Program P, const __grid_constant__ FlowArgs
         const size_t q = (size_t)R.off + (size_t)A.st.id[k];
         A.terms[q] = v3[0]; A.terms[(size_t)A.terms_stride + q] = v3[1]; A.terms[(size_t)2 * A.terms_stride + q] = v3[2];
       }
-      flow_enforce(R, g, dix, diy);
-      stg4(A.G + k, g);
+      // (the enforce of the second half: flow_fire_end)
     }
     A.d.vx[k] = vx; A.d.vy[k] = vy;
     if (dix) A.d.ix[k] += dix;
     if (diy) A.d.iy[k] += diy;
     // skin test: no position changes between here and the next step's first half
-    if (flow_left_skin(R, A.nl, k, g) && A.rebuild[r] == 0) atomicOr(&A.rebuild[r], 1);
+    left = flow_left_skin(R, A.nl, k, g);
+    if (left && __ldcg(A.rebuild + r) == 0) atomicOr(&A.rebuild[r], 1);
     if (!(isfinite(g.x) && isfinite(g.y))) atomicOr(A.status, ST_NONFINITE);
   }
-  if (INTEG != FLOW_FIRE) return;
+  if (INTEG != FLOW_FIRE) return left;
   // FIRE: energies and sums per block, then the control in the replica's last block (k_fire_b)
   {
     constexpr int NE = PAIR == FLOW_ANY ? MAX_PAIR : 1;
@@ -253,7 +259,7 @@ k_flow_force(const __grid_constant__ Program P, const __grid_constant__ FlowArgs
   __syncthreads();
   if (threadIdx.x == 0) amlast = atomicAdd(&A.fire_cnt[r], 1) == A.rep_nblk[r] - 1;
   __syncthreads();
-  if (!amlast) return;
+  if (!amlast) return left;
   __threadfence();
   double sums[5];
   fire_sums(P, A.part, A.epart, A.nblocks, A.rep_blk0[r], A.rep_nblk[r], sums);
@@ -263,9 +269,18 @@ k_flow_force(const __grid_constant__ Program P, const __grid_constant__ FlowArgs
     if (threadIdx.x == 0) { sums[0] = o[0]; sums[1] = o[1]; sums[2] = o[2]; }
   }
   if (threadIdx.x == 0) {
-    fire_control(R, A.clk[r], r, 0, sums, A.driver, A.alpha_mix);
+    fire_control(R, A.clk[r], r, 0, sums, A.driver, A.alpha_mix, step);
     A.fire_cnt[r] = 0;
   }
+  return left;
+}
+
+template <int INTEG, int PAIR, int ALIGN>
+__global__ void __launch_bounds__(BLOCK, 8)
+k_flow_force(const __grid_constant__ Program P, const __grid_constant__ FlowArgs A) {
+  const int bid = A.blist ? A.blist[blockIdx.x] : (int)blockIdx.x;
+  if (A.clk[A.blk_rep[bid]].halt) return;
+  flow_force_block<INTEG, PAIR, ALIGN, false>(P, A, A.Gin, A.G, bid, 0);
 }
 
 // FIRE velocity mixing and the P <= 0 restart (k_fire_d)
@@ -281,17 +296,35 @@ __device__ __forceinline__ void flow_mix(const FlowArgs& A, const Clock& C, int 
   if (!(C.fire_P > 0.0)) { vx = 0.0; vy = 0.0; }
 }
 
+// End of a FIRE step for slot k: the second half's enforce (only the director
+// moves, and no aligner reads it, so it waits until here), then the mixing; a
+// replica that has just converged takes the enforce alone.
+__device__ __forceinline__ void flow_fire_end(const FlowArgs& A, D4* G, const Replica& R, const Clock& C, int r, int k) {
+  D4 g = ld4(G + k);
+  int dix = 0, diy = 0;
+  flow_enforce(R, g, dix, diy);
+  stg4(G + k, g);
+  if (C.fire_conv_step >= 0) return;
+  double vx = A.d.vx[k], vy = A.d.vy[k];
+  flow_mix(A, C, r, k, A.d.fx[k], A.d.fy[k], vx, vy);
+  A.d.vx[k] = vx; A.d.vy[k] = vy;
+}
+
 // First half of a step for slot k (k_langevin_a, k_nve_a, k_fire_d and
-// k_fire_a): pre, the start-of-step enforce is still to come; mix, FIRE's mixing.
+// k_fire_a): pre, the start-of-step enforce is still to come; mix, the end of
+// FIRE's last step too.
 template <int INTEG>
-__device__ __forceinline__ void flow_first_half(const Program& P, const FlowArgs& A, const Replica& R, const Clock& C,
-                                                int r, int k, bool pre, bool mix, uint64_t base) {
-  D4 g = ld4(A.G + k);
+__device__ __forceinline__ void flow_first_half(const Program& P, const FlowArgs& A, D4* G, const Replica& R,
+                                                const Clock& C, int r, int k, bool pre, bool mix, uint64_t base) {
+  D4 g = ld4(G + k);
   const double* ip = R.integ_p[0];
   const double fx = A.d.fx[k], fy = A.d.fy[k];
   double vx = A.d.vx[k], vy = A.d.vy[k];
   int dix = 0, diy = 0;
-  if (INTEG == FLOW_FIRE && mix) flow_mix(A, C, r, k, fx, fy, vx, vy);
+  if (INTEG == FLOW_FIRE && mix) {
+    flow_enforce(R, g, dix, diy);
+    flow_mix(A, C, r, k, fx, fy, vx, vy);
+  }
   if (pre) flow_enforce(R, g, dix, diy);
   if (INTEG == FLOW_LANGEVIN) {
     const double dt = ip[0], dt2 = 0.5 * dt, mass = A.st.mass[k];
@@ -356,10 +389,81 @@ __device__ __forceinline__ void flow_first_half(const Program& P, const FlowArgs
     const double cs = cos(dtheta), sn = sin(dtheta);
     set_unit(cs * g.z + -sn * g.w, sn * g.z + cs * g.w, g.z, g.w);
   }
-  stg4(A.G + k, g);
+  stg4(G + k, g);
   A.d.vx[k] = vx; A.d.vy[k] = vy;
   if (dix) A.d.ix[k] += dix;
   if (diy) A.d.iy[k] += diy;
+}
+
+// Rebuild of the replicas in L at the end of a step, and (again) their forces
+// with the new lists, the next step's enforce applied: by the first bar.n
+// blocks.  False: a barrier's wait ran out.  *over: the lists did not fit.
+template <int INTEG, int PAIR, int ALIGN>
+__device__ __forceinline__ bool flow_rebuild(const Program& P, const FlowArgs& A, const RebuildArgs& B, RebuildList& L,
+                                          GridBar& bar, bool again) {
+  const int t = threadIdx.x, nb = (int)bar.n;
+  auto slot = [&](int v, int& r) {  // particle slot of this thread in virtual block v, -1: none
+    const int s = list_find(L.blk, L.n, v);
+    r = L.rep[s];
+    const Replica& R = A.reps[r];
+    const int k = R.off + (v - L.blk[s]) * BLOCK + t;
+    return k - R.off < R.n ? k : -1;
+  };
+  int r;
+  if (INTEG == FLOW_FIRE)  // the mixing reads the forces that are replaced below
+    for (int v = blockIdx.x; v < L.nblk; v += nb) {
+      const int k = slot(v, r);
+      if (k >= 0) flow_fire_end(A, B.G, A.reps[r], A.clk[r], r, k);
+    }
+  if (!rebuild_phases<HOT_PLANE>(B, L, bar)) return false;
+  if (!again) return true;
+  if (!grid_wait(bar)) return false;
+  if ((__ldcg(B.bstatus) & ST_OVERFLOW) != 0) return true;
+  for (int v = blockIdx.x; v < L.nblk; v += nb) {
+    const int k = slot(v, r);
+    if (k < 0) continue;
+    D4 g = ld4(B.G + k);
+    int dix = 0, diy = 0;
+    flow_enforce(A.reps[r], g, dix, diy);
+    stg4(B.G + k, g);
+    if (dix) A.d.ix[k] += dix;
+    if (diy) A.d.iy[k] += diy;
+  }
+  if (!grid_wait(bar)) return false;
+  for (int v = blockIdx.x; v < L.nblk; v += nb) {
+    const int k = slot(v, r);
+    if (k < 0) continue;
+    double fx, fy, tz, e[MAX_PAIR];
+    const D4 g = ld4(B.G + k);
+    flow_gather<PAIR, ALIGN, false, true>(P, A.reps[r], B.G, A.st, A.nl, k, g, fx, fy, tz, e);
+    A.d.fx[k] = fx; A.d.fy[k] = fy;
+    if (INTEG == FLOW_NVE) A.d.tz[k] = tz;
+  }
+  return true;
+}
+
+// First half of the next step for the blocks taking part (begin), or the end
+// of this one, FIRE's mixing.
+template <int INTEG>
+__device__ __forceinline__ void flow_begin_blocks(const Program& P, const FlowArgs& A, D4* G, const int* rebuild,
+                                                  bool flagged, bool begin, bool tail, bool pre, int step) {
+  for (int v = blockIdx.x; v < A.nblist; v += gridDim.x) {
+    const int bid = A.blist ? A.blist[v] : v;
+    const int r = A.blk_rep[bid];
+    const Clock& C = A.clk[r];
+    // frozen, but for the end of the step that it converged in (the step
+    // counters still stand at the first of `step` steps)
+    if (INTEG == FLOW_FIRE && C.fire_conv_step >= 0 && !(tail && C.fire_conv_step == C.run_step + step - 1)) continue;
+    const Replica& R = A.reps[r];
+    const int k = bid * BLOCK + threadIdx.x;
+    if (k - R.off >= R.n) continue;
+    const bool redo = flagged && __ldcg(rebuild + r) != 0;  // cleared when every block has read it
+    if (begin && !(INTEG == FLOW_FIRE && C.fire_conv_step >= 0)) {
+      uint64_t base = 0;
+      if (INTEG == FLOW_LANGEVIN) base = C.ctr[0] + (uint64_t)step * A.fc[r].draws;
+      flow_first_half<INTEG>(P, A, G, R, C, r, k, tail ? !redo : pre, tail && !redo, base);
+    } else if (INTEG == FLOW_FIRE && (C.fire_conv_step >= 0 || !redo)) flow_fire_end(A, G, R, C, r, k);
+  }
 }
 
 // Counters and rebuild of the step just done (tail), first half of the next
@@ -373,72 +477,18 @@ k_flow_begin(const __grid_constant__ Program P, const __grid_constant__ FlowArgs
   const int t = threadIdx.x;
   if (B.clk[0].halt) return;  // set between launches only
   const unsigned long long t0 = global_ns();
-  GridBar bar{B.bar, 0u, B.status};
+  GridBar bar{B.bar, gridDim.x, 0u, 0u, B.status};
   // converged replicas are frozen: a request of their last iteration is dropped
   const bool flagged = tail && rebuild_list(B, sort_every, L, INTEG == FLOW_FIRE);
   bool over = false;
   if (flagged) {
-    if (INTEG == FLOW_FIRE)  // the mixing reads the forces that the rebuild replaces
-      for (int v = blockIdx.x; v < L.nblk; v += gridDim.x) {
-        const int s = list_find(L.blk, L.n, v), r = L.rep[s];
-        const Replica& R = A.reps[r];
-        const int k = R.off + (v - L.blk[s]) * BLOCK + t;
-        if (k - R.off >= R.n) continue;
-        double vx = A.d.vx[k], vy = A.d.vy[k];
-        flow_mix(A, A.clk[r], r, k, A.d.fx[k], A.d.fy[k], vx, vy);
-        A.d.vx[k] = vx; A.d.vy[k] = vy;
-      }
-    if (!rebuild_phases<HOT_PLANE>(B, L, bar)) return;
-    if (!grid_wait(bar)) return;
+    bar.n = rebuild_blocks(L);
+    if (blockIdx.x < bar.n && !flow_rebuild<INTEG, PAIR, ALIGN>(P, A, B, L, bar, begin)) return;
+    if (!grid_wait_all(bar)) return;  // the neighbours' records move on below
     over = (__ldcg(B.bstatus) & ST_OVERFLOW) != 0;
-    if (!over && begin) {
-      // the start-of-step enforce, then the forces with the new lists
-      for (int v = blockIdx.x; v < L.nblk; v += gridDim.x) {
-        const int s = list_find(L.blk, L.n, v);
-        const Replica& R = A.reps[L.rep[s]];
-        const int k = R.off + (v - L.blk[s]) * BLOCK + t;
-        if (k - R.off >= R.n) continue;
-        D4 g = ld4(A.G + k);
-        int dix = 0, diy = 0;
-        flow_enforce(R, g, dix, diy);
-        stg4(A.G + k, g);
-        if (dix) A.d.ix[k] += dix;
-        if (diy) A.d.iy[k] += diy;
-      }
-      if (!grid_wait(bar)) return;
-      for (int v = blockIdx.x; v < L.nblk; v += gridDim.x) {
-        const int s = list_find(L.blk, L.n, v);
-        const Replica& R = A.reps[L.rep[s]];
-        const int k = R.off + (v - L.blk[s]) * BLOCK + t;
-        if (k - R.off >= R.n) continue;
-        double fx, fy, tz, e[MAX_PAIR];
-        const D4 g = ld4(A.G + k);
-        flow_gather<PAIR, ALIGN, false, true>(P, R, A.G, A.st, A.nl, k, g, fx, fy, tz, e);
-        A.d.fx[k] = fx; A.d.fy[k] = fy;
-        if (INTEG == FLOW_NVE) A.d.tz[k] = tz;
-      }
-      if (!grid_wait(bar)) return;  // the neighbours' records move on below
-    }
   }
-  for (int v = blockIdx.x; v < A.nblist && (begin || INTEG == FLOW_FIRE); v += gridDim.x) {
-    const int bid = A.blist ? A.blist[v] : v;
-    const int r = A.blk_rep[bid];
-    const Clock& C = A.clk[r];
-    if (INTEG == FLOW_FIRE && C.fire_conv_step >= 0) continue;
-    const Replica& R = A.reps[r];
-    const int k = bid * BLOCK + t;
-    if (k - R.off >= R.n) continue;
-    const bool redo = flagged && __ldcg(B.rebuild + r) != 0;  // cleared by the last block below
-    if (begin && !over) {
-      uint64_t base = 0;
-      if (INTEG == FLOW_LANGEVIN) base = C.ctr[0] + (tail ? A.fc[r].draws : 0ull);
-      flow_first_half<INTEG>(P, A, R, C, r, k, tail ? !redo : pre != 0, tail && !redo, base);
-    } else if (INTEG == FLOW_FIRE && !redo) {  // the step ends with its mixing
-      double vx = A.d.vx[k], vy = A.d.vy[k];
-      flow_mix(A, C, r, k, A.d.fx[k], A.d.fy[k], vx, vy);
-      A.d.vx[k] = vx; A.d.vy[k] = vy;
-    }
-  }
+  if (begin || INTEG == FLOW_FIRE)
+    flow_begin_blocks<INTEG>(P, A, A.G, B.rebuild, flagged, begin && !over, tail, pre, tail ? 1 : 0);
   // the block that finishes last: every other has read the clocks and flags
   if (!tail) return;
   if (!grid_last(bar)) return;
@@ -451,6 +501,92 @@ k_flow_begin(const __grid_constant__ Program P, const __grid_constant__ FlowArgs
   if (INTEG == FLOW_FIRE && !over)
     for (int r = t; r < B.nrep; r += BLOCK)
       if (A.clk[r].fire_conv_step >= 0) B.rebuild[r] = 0;
+}
+
+// nsteps steps in one launch, for systems whose blocks are resident at once:
+// the two kernels above with a grid barrier in place of each launch.  Blocks
+// that ask for a rebuild say so as they arrive (words as in k_abp_run).
+template <int INTEG, int PAIR, int ALIGN>
+__global__ void __launch_bounds__(BLOCK, FLOW_RUN_MINB)
+k_flow_run(const __grid_constant__ Program P, const __grid_constant__ FlowArgs A, const __grid_constant__ RebuildArgs B,
+           D4* G0, D4* G1, unsigned long long* word, int nsteps, int sort_every, int pre) {
+  __shared__ RebuildList L;
+  __shared__ unsigned long long seen;
+  const int t = threadIdx.x;
+  GridBar bar{B.bar, gridDim.x, 0u, 0u, B.status};
+  unsigned long long asked[2] = {0ull, 0ull};
+  unsigned target[2] = {0u, 0u};
+  D4 *G = G0, *Gn = INTEG == FLOW_NVE ? G1 : G0;
+  flow_begin_blocks<INTEG>(P, A, G, B.rebuild, false, true, false, pre != 0, 0);
+  if (!grid_wait(bar)) return;
+  int done = 0;
+  bool over = false, rebuilt = false;
+  for (int step = 0; step < nsteps; step++) {
+    bool ask = false;
+    for (int v = blockIdx.x; v < A.nblist; v += gridDim.x)
+      ask |= flow_force_block<INTEG, PAIR, ALIGN, true>(P, A, G, Gn, A.blist ? A.blist[v] : v, step);
+    const int w = step & 1;
+    const bool block_asks = __syncthreads_or(ask) != 0;
+    target[w] += gridDim.x;
+    int ok = 1;
+    if (t == 0) {
+      red_release64(word + w, 1ull + (block_asks ? 1ull << 32 : 0ull));
+      unsigned long long x = ld_acquire64(word + w);
+      for (unsigned it = 0; (unsigned)x < target[w]; x = ld_acquire64(word + w))
+        if (++it >= GRID_SPIN_LIMIT) { atomicOr(B.status, ST_TIMEOUT); ok = 0; break; }
+      seen = x;
+    }
+    if (!__syncthreads_and(ok)) return;
+    { D4* x = G; G = Gn; Gn = x; }
+    done = step + 1;
+    const bool more = done < nsteps;
+    bool flagged = (unsigned)(seen >> 32) != (unsigned)asked[w];  // the same for every block
+    rebuilt = false;
+    if (flagged) {
+      asked[w] = seen >> 32;
+      const unsigned long long t0 = global_ns();
+      // (a minimiser's replica may have converged in the step that asked)
+      if (rebuild_list(B, sort_every, L, INTEG == FLOW_FIRE)) {
+        RebuildArgs Q = B;
+        Q.G = G;
+        if (!flow_rebuild<INTEG, PAIR, ALIGN>(P, A, Q, L, bar, more)) return;
+        if (!grid_wait(bar)) return;
+        over = (__ldcg(B.bstatus) & ST_OVERFLOW) != 0;
+        rebuilt = true;
+      }
+      if (more || INTEG == FLOW_FIRE)
+        flow_begin_blocks<INTEG>(P, A, G, B.rebuild, rebuilt, more && !over, true, false, step + 1);
+      if (!grid_wait(bar)) return;  // every block has read the flags
+      if (blockIdx.x == 0) {
+        if (rebuilt && !over) {
+          for (int s = t; s < L.n; s += BLOCK) B.builds[L.rep[s]]++;
+          if (t == 0) { B.stats->builds++; B.stats->ns += global_ns() - t0; }
+        }
+        if (!over)
+          for (int r = t; r < B.nrep; r += BLOCK) B.rebuild[r] = 0;
+      }
+      if (over) break;
+      if (more && !grid_wait(bar)) return;  // flags cleared before the next are set
+      continue;
+    }
+    if (more || INTEG == FLOW_FIRE)
+      flow_begin_blocks<INTEG>(P, A, G, B.rebuild, false, more, true, false, step + 1);
+    if (more && !grid_wait(bar)) return;
+  }
+  if (grid_last(bar)) {
+    if (t == 0) {
+      word[0] = 0ull; word[1] = 0ull;
+      B.executed[0] = done;
+      B.executed[1] = rebuilt ? 1 : 0;
+    }
+    for (int r = t; r < B.nrep; r += BLOCK) {
+      Clock& C = A.clk[r];
+      if (INTEG == FLOW_LANGEVIN) C.ctr[0] += (uint64_t)done * A.fc[r].draws;
+      C.run_step += done;
+      C.time_step += done;
+      if (over) C.halt = 1;
+    }
+  }
 }
 
 }  // namespace sg

@@ -703,7 +703,7 @@ static __global__ void k_fire_a(Program P, const Replica* __restrict__ reps, con
 // order, then a fixed tree over the threads (the same bits for a replica run
 // alone or inside an ensemble).  Returns P, |F|^2, |v|^2, max |F_i|^2, E on
 // thread 0.
-static __device__ void fire_sums(const Program& P, const double* part, const double* epart, int nblocks, int b0, int nb,
+static __device__ __forceinline__ void fire_sums(const Program& P, const double* part, const double* epart, int nblocks, int b0, int nb,
                           double out[5]) {
   __shared__ double red[5][BLOCK];
   const int t = threadIdx.x;
@@ -729,9 +729,10 @@ static __device__ void fire_sums(const Program& P, const double* part, const dou
 
 // FIRE's convergence test and dt / alpha control on the replica's sums
 // (integrator_fire.cpp:96-147).  alpha_mix[r] keeps the alpha the mixing step
-// must use (the value before this update).
-static __device__ void fire_control(const Replica& R, Clock& C, int r, int c, const double sums[5], int driver,
-                             double* alpha_mix) {
+// must use (the value before this update).  step: steps since the replica's
+// step counters were last advanced.
+static __device__ __forceinline__ void fire_control(const Replica& R, Clock& C, int r, int c, const double sums[5], int driver,
+                             double* alpha_mix, int step = 0) {
   if (C.fire_conv_step >= 0 || C.halt) return;
   const double* ip = R.integ_p[c];
   double Ps = sums[0], Fn = sums[1], Vn = sums[2], Fm = sums[3], E = sums[4];
@@ -744,7 +745,7 @@ static __device__ void fire_control(const Replica& R, Clock& C, int r, int c, co
                                      : (Fn / sqrt_ndof < ip[3] && fabs(E - C.fire_old_e) < ip[4]);
   if (conv) {
     C.fire_converged = 1;
-    if (driver) C.fire_conv_step = C.run_step;
+    if (driver) C.fire_conv_step = C.run_step + step;
     return;
   }
   alpha_mix[r] = C.fire_alpha;
@@ -775,7 +776,7 @@ static __device__ void fire_control(const Replica& R, Clock& C, int r, int c, co
 // `terms` (three arrays of `stride` doubles, indexed by replica offset + id).
 // One warp: 32 terms loaded at a time, then added in order through shuffles,
 // so every lane holds the same sequential sums.
-static __device__ void fire_ordered_sums(const double* __restrict__ terms, int stride, int off, int n, double out[3]) {
+static __device__ __forceinline__ void fire_ordered_sums(const double* __restrict__ terms, int stride, int off, int n, double out[3]) {
   const int lane = threadIdx.x & 31;
   double sP = 0.0, sF = 0.0, sV = 0.0;
   for (int base = 0; base < n; base += 32) {

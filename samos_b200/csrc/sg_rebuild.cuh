@@ -27,26 +27,47 @@ __device__ __forceinline__ unsigned ld_acquire(const unsigned* p) {
   return v;
 }
 
+__device__ __forceinline__ unsigned long long ld_acquire64(const unsigned long long* p) {
+  unsigned long long v;
+  asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+  return v;
+}
+
+__device__ __forceinline__ void red_release64(unsigned long long* p, unsigned long long v) {
+  asm volatile("red.release.gpu.global.add.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+}
+
 struct GridBar {
-  unsigned* cnt;    // [0] arrivals, [1] blocks done: both 0 between launches
+  unsigned* cnt;    // [0] arrivals, [1] blocks done, [2] arrivals of grid_wait_all: all 0 between launches
+  unsigned n;       // blocks that pass through the barriers: the first n of the launch
   unsigned passed;  // barriers passed by this block
+  unsigned passed_all;
   int* status;
 };
 
-__device__ __forceinline__ bool grid_wait(GridBar& g) {
-  g.passed++;
+template <bool BACKOFF>
+__device__ __forceinline__ bool grid_arrive_wait(unsigned* word, unsigned target, int* status) {
   __syncthreads();
   int ok = 1;
   if (threadIdx.x == 0) {
-    const unsigned target = g.passed * gridDim.x;
-    __threadfence();
-    atomicAdd(g.cnt, 1u);
+    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(word) : "memory");
     unsigned it = 0;
-    while (ld_acquire(g.cnt) < target && ++it < GRID_SPIN_LIMIT) {}
-    if (it >= GRID_SPIN_LIMIT) { atomicOr(g.status, ST_TIMEOUT); ok = 0; }
-    __threadfence();
+    while (ld_acquire(word) < target && ++it < GRID_SPIN_LIMIT)
+      if (BACKOFF) __nanosleep(100);
+    if (it >= GRID_SPIN_LIMIT) { atomicOr(status, ST_TIMEOUT); ok = 0; }
   }
   return __syncthreads_and(ok) != 0;
+}
+
+__device__ __forceinline__ bool grid_wait(GridBar& g) {
+  g.passed++;
+  return grid_arrive_wait<false>(g.cnt, g.passed * g.n, g.status);
+}
+
+// the same for every block of the launch, those included that have waited only here
+__device__ __forceinline__ bool grid_wait_all(GridBar& g) {
+  g.passed_all++;
+  return grid_arrive_wait<true>(g.cnt + 2, g.passed_all * gridDim.x, g.status);
 }
 
 // True on every thread of the block that finishes last; that block has put the
@@ -57,7 +78,7 @@ __device__ __forceinline__ bool grid_last(GridBar& g) {
   __syncthreads();
   if (threadIdx.x == 0) {
     last = atomicAdd(g.cnt + 1, 1u) == gridDim.x - 1;
-    if (last) { g.cnt[0] = 0; g.cnt[1] = 0; }
+    if (last) { g.cnt[0] = 0; g.cnt[1] = 0; g.cnt[2] = 0; }
     __threadfence();
   }
   __syncthreads();
@@ -171,11 +192,21 @@ __device__ __forceinline__ void rb_store_position(const RebuildArgs& A, int k, d
   }
 }
 
-// All phases for the replicas in L (every block of the launch takes part).
-// False: a barrier's wait ran out.
+// Blocks that take part in a rebuild: a barrier costs the more the more blocks
+// pass it (1,184 blocks 4 us, 148 blocks 1 us), so no more than there are blocks
+// of particles to rebuild.
+__device__ __forceinline__ unsigned rebuild_blocks(const RebuildList& L) {
+  return min(gridDim.x, (unsigned)max(32, L.nblk));
+}
+
+// All phases for the replicas in L, by the first bar.n blocks of the launch.
+// False: a barrier's wait ran out.  Always inlined: as one function called from
+// kernels with different register bounds it came out wrong (a caller's value in
+// place of a coordinate).
 template <int SHAPE>
-__device__ bool rebuild_phases(const RebuildArgs& A, RebuildList& L, GridBar& bar) {
-  const int t = threadIdx.x, nthr = gridDim.x * blockDim.x, gid = blockIdx.x * blockDim.x + t;
+__device__ __forceinline__ bool rebuild_phases(const RebuildArgs& A, RebuildList& L, GridBar& bar) {
+  const int nb = (int)bar.n;
+  const int t = threadIdx.x, nthr = nb * blockDim.x, gid = blockIdx.x * blockDim.x + t;
   __shared__ int shw[32];
   for (int v = gid; v < L.ncell; v += nthr) {  // (k_seg_zero)
     const int s = list_find(L.cell, L.n, v);
@@ -185,7 +216,7 @@ __device__ bool rebuild_phases(const RebuildArgs& A, RebuildList& L, GridBar& ba
   if (gid == 0) *A.bstatus = 0;
   if (!grid_wait(bar)) return false;
 
-  for (int v = blockIdx.x; v < L.nblk; v += gridDim.x) {  // (k_rb_bin)
+  for (int v = blockIdx.x; v < L.nblk; v += nb) {  // (k_rb_bin)
     const int s = list_find(L.blk, L.n, v);
     const Replica& R = A.reps[L.rep[s]];
     const int k = R.off + (v - L.blk[s]) * BLOCK + t;
@@ -208,7 +239,7 @@ __device__ bool rebuild_phases(const RebuildArgs& A, RebuildList& L, GridBar& ba
 
   // exclusive scan of the flagged cells' counts: a run of tiles per block
   const int tiles = (L.ncell + BLOCK * 4 - 1) / (BLOCK * 4);
-  const int per = (tiles + gridDim.x - 1) / gridDim.x;
+  const int per = (tiles + nb - 1) / nb;
   const int tile0 = min((int)blockIdx.x * per, tiles), tile1 = min(tile0 + per, tiles);
   auto cell_at = [&](int v) {
     const int s = list_find(L.cell, L.n, v);
@@ -258,7 +289,7 @@ __device__ bool rebuild_phases(const RebuildArgs& A, RebuildList& L, GridBar& ba
   }
   if (!grid_wait(bar)) return false;
 
-  for (int v = blockIdx.x; v < L.nblk; v += gridDim.x) {  // (k_rb_scatter)
+  for (int v = blockIdx.x; v < L.nblk; v += nb) {  // (k_rb_scatter)
     const int s = list_find(L.blk, L.n, v);
     const Replica& R = A.reps[L.rep[s]];
     const int k = R.off + (v - L.blk[s]) * BLOCK + t;
@@ -269,7 +300,7 @@ __device__ bool rebuild_phases(const RebuildArgs& A, RebuildList& L, GridBar& ba
   }
   if (!grid_wait(bar)) return false;
 
-  for (int v = blockIdx.x; v < L.nblk; v += gridDim.x) {  // (k_rb_rank)
+  for (int v = blockIdx.x; v < L.nblk; v += nb) {  // (k_rb_rank)
     const int s = list_find(L.blk, L.n, v);
     const Replica& R = A.reps[L.rep[s]];
     const int k = R.off + (v - L.blk[s]) * BLOCK + t;
@@ -286,7 +317,7 @@ __device__ bool rebuild_phases(const RebuildArgs& A, RebuildList& L, GridBar& ba
   }
   if (!grid_wait(bar)) return false;
 
-  for (int v = blockIdx.x; v < L.nblk; v += gridDim.x) {  // (k_rb_gather, k_rb_build, k_lane_order)
+  for (int v = blockIdx.x; v < L.nblk; v += nb) {  // (k_rb_gather, k_rb_build, k_lane_order)
     const int s = list_find(L.blk, L.n, v);
     const Replica& R = A.reps[L.rep[s]];
     const int k = R.off + (v - L.blk[s]) * BLOCK + t;
@@ -326,7 +357,7 @@ __device__ bool rebuild_phases(const RebuildArgs& A, RebuildList& L, GridBar& ba
   }
   if (L.any_sort) {
     if (!grid_wait(bar)) return false;
-    for (int v = blockIdx.x; v < L.nblk; v += gridDim.x) {  // (k_rb_copyback, k_hot_pack)
+    for (int v = blockIdx.x; v < L.nblk; v += nb) {  // (k_rb_copyback, k_hot_pack)
       const int s = list_find(L.blk, L.n, v);
       if (L.mode[s] != 2) continue;
       const Replica& R = A.reps[L.rep[s]];
@@ -379,8 +410,8 @@ k_tail_rebuild(Program P, RebuildArgs A, int sort_every) {
     if (threadIdx.x == 0) (*A.executed)++;
   }
   if (!rebuild_list(A, sort_every, L)) return;
-  GridBar bar{A.bar, 0u, A.status};
-  if (!rebuild_phases<SHAPE>(A, L, bar)) return;
+  GridBar bar{A.bar, rebuild_blocks(L), 0u, 0u, A.status};
+  if (blockIdx.x < bar.n && !rebuild_phases<SHAPE>(A, L, bar)) return;
   if (grid_last(bar)) rebuild_done(A, L, t0);
 }
 
