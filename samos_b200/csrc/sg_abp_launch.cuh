@@ -110,7 +110,7 @@ static cudaError_t launch_abp_run(const AbpRunLaunch* L, int* blocks_per_sm) {
   const void* f = (const void*)k_abp_run<SHAPE, ALIGN, SP, BYVAL>;
   if (!L) return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, f, BLOCK, 0);
   AbpRunLaunch A = *L;
-  void* args[] = {&A.abp, &A.abp0, &A.blk_rep, &A.G0, &A.G1, &A.H0, &A.H1, &A.rb, &A.word, &A.nsteps, &A.sort_every};
+  void* args[] = {&A.abp, &A.abp0, &A.blk_rep, &A.G0, &A.G1, &A.H0, &A.H1, &A.rb, &A.word, &A.nsteps};
   return cudaLaunchCooperativeKernel(f, dim3(A.nblocks), dim3(BLOCK), args, 0, A.stream);
 }
 template <int SHAPE, int ALIGN>

@@ -35,15 +35,16 @@ void launch_abp_sphere_none(const AbpLaunch& L);
 void launch_abp_sphere_polar(const AbpLaunch& L);
 void launch_abp_sphere_nematic(const AbpLaunch& L);
 
-// Many steps in one cooperative launch (k_abp_run).
+// Many steps in one cooperative launch (k_abp_run), up to the first that asks for a rebuild.
 struct AbpRunLaunch {
   const AbpParams* abp;
   AbpParams abp0;
   const int* blk_rep;
-  D4 *G0, *G1, *H0, *H1;  // state in G0 / H0
+  D4 *G0, *G1, *H0, *H1;  // state in G0 / H0 after an even number of steps
   RebuildArgs rb;
   unsigned long long* word;  // step barrier, two words, 0 between launches
-  int nsteps, sort_every, nblocks, nrep;
+  int nsteps;                // of the run: rb.executed counts those done
+  int nblocks, nrep;
   bool self_propulsion;
   cudaStream_t stream;
 };

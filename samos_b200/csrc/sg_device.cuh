@@ -128,11 +128,14 @@ __device__ __forceinline__ D4 ldg4(const D4* p) {
                : "=d"(v.x), "=d"(v.y), "=d"(v.z), "=d"(v.w) : "l"(p));
   return v;
 }
-// the same load for records that the kernel itself writes (between barriers)
+// The same load for records that the kernel itself writes (between barriers).
+// Volatile, so that it stays behind the barrier and the stores of stg4; no
+// memory clobber, which would have every replica parameter read again after
+// each record.
 __device__ __forceinline__ D4 ld4(const D4* p) {
   D4 v;
   asm volatile("ld.global.v4.f64 {%0,%1,%2,%3}, [%4];"
-               : "=d"(v.x), "=d"(v.y), "=d"(v.z), "=d"(v.w) : "l"(p) : "memory");
+               : "=d"(v.x), "=d"(v.y), "=d"(v.z), "=d"(v.w) : "l"(p));
   return v;
 }
 __device__ __forceinline__ void stg4(D4* p, const D4& v) {

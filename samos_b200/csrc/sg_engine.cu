@@ -69,6 +69,7 @@ struct sg_system {
   int flow_grid = 0, flow_run_grid = 0;
   int rb_grid[3] = {0, 0, 0};  // blocks that fit the device at once, per shape
   bool rb_used = false;        // in the current run
+  int rb_builds_seen = 0;      // of the run, when the host last looked
   int *rep_blk0 = nullptr, *rep_nblk = nullptr;
   std::vector<Replica> reps_h;
   Replica* reps = nullptr;
@@ -1990,6 +1991,7 @@ static int dev_rebuild_ready(sg_system* s) {
   if (!s->rb_used) {
     CU(s, cudaMemsetAsync(s->rb_stats, 0, sizeof(RebuildStats), s->stream));
     s->rb_used = true;
+    s->rb_builds_seen = 0;
   }
   s->builds_dev_new = true;
   return SG_OK;
@@ -2108,15 +2110,31 @@ static int run_resident(sg_system* s, int shape, int64_t K, int64_t* executed, d
   L.abp = s->abp; L.abp0 = s->abp0_h; L.blk_rep = s->blk_rep;
   L.G0 = s->G[b]; L.G1 = s->G[1 - b]; L.H0 = s->H[b]; L.H1 = s->H[1 - b];
   L.rb = rebuild_args(s, shape);
-  L.word = s->run_word; L.nsteps = (int)K; L.sort_every = kSortEvery;
+  L.word = s->run_word; L.nsteps = (int)K;
   L.nblocks = s->nblocks; L.nrep = s->nrep; L.self_propulsion = s->prog.next == 1; L.stream = s->stream;
-  CU(s, abp_run(s, shape, &L, nullptr));
-  s->launches++;
+  CU(s, cudaMemsetAsync(s->exec_cnt, 0, sizeof(int), s->stream));
+  int every = kSortEvery;
+  void* args[] = {&L.rb, &L.G0, &L.G1, &L.H0, &L.H1, &every};
+  const void* rebuild = shape == HOT_PLANE ? (const void*)k_run_rebuild<HOT_PLANE> : (const void*)k_run_rebuild<HOT_SPHERE>;
+  const dim3 rgrid(std::min(s->rb_grid[shape], std::max(32, s->nblocks)));
+  // a launch for every stretch between rebuilds that the last gap suggests, and
+  // one more
+  const int64_t stretches = std::min<int64_t>(16, 2 + K / std::max<int64_t>(1, s->last_gap));
+  for (int64_t i = 0; i < stretches; i++) {
+    CU(s, abp_run(s, shape, &L, nullptr));
+    CU(s, cudaLaunchCooperativeKernel(rebuild, rgrid, dim3(BLOCK), args, 0, s->stream));
+    s->launches += 2;
+  }
   int ex = 0, st = 0;
+  RebuildStats rb{};
   CU(s, cudaMemcpyAsync(&ex, s->exec_cnt, sizeof(int), cudaMemcpyDeviceToHost, s->stream));
   CU(s, cudaMemcpyAsync(&st, s->status, sizeof(int), cudaMemcpyDeviceToHost, s->stream));
+  CU(s, cudaMemcpyAsync(&rb, s->rb_stats, sizeof(rb), cudaMemcpyDeviceToHost, s->stream));
   CU(s, cudaMemcpyAsync(s->rebuild_h, s->rebuild, sizeof(int) * s->nrep, cudaMemcpyDeviceToHost, s->stream));
   CU(s, cudaStreamSynchronize(s->stream));
+  if (rb.builds > s->rb_builds_seen) s->last_gap = std::max<int64_t>(1, ex / (rb.builds - s->rb_builds_seen));
+  else s->last_gap = std::max<int64_t>(s->last_gap, ex);
+  s->rb_builds_seen = rb.builds;
   if (st & ST_TIMEOUT) return grid_timeout(s);
   if (ex < 1 || ex > K) return fail(s, SG_ERR_CUDA, "resident run: inconsistent step count");
   s->hot_buf = b ^ (int)(ex & 1);

@@ -399,8 +399,8 @@ __device__ __forceinline__ void flow_first_half(const Program& P, const FlowArgs
 // with the new lists, the next step's enforce applied: by the first bar.n
 // blocks.  False: a barrier's wait ran out.  *over: the lists did not fit.
 template <int INTEG, int PAIR, int ALIGN>
-__device__ __forceinline__ bool flow_rebuild(const Program& P, const FlowArgs& A, const RebuildArgs& B, RebuildList& L,
-                                          GridBar& bar, bool again) {
+__device__ __forceinline__ bool flow_rebuild(const Program& P, const FlowArgs& A, const RebuildArgs& B, D4* G, RebuildList& L,
+                                             RebuildScratch& Q, GridBar& bar, bool again) {
   const int t = threadIdx.x, nb = (int)bar.n;
   auto slot = [&](int v, int& r) {  // particle slot of this thread in virtual block v, -1: none
     const int s = list_find(L.blk, L.n, v);
@@ -413,19 +413,19 @@ __device__ __forceinline__ bool flow_rebuild(const Program& P, const FlowArgs& A
   if (INTEG == FLOW_FIRE)  // the mixing reads the forces that are replaced below
     for (int v = blockIdx.x; v < L.nblk; v += nb) {
       const int k = slot(v, r);
-      if (k >= 0) flow_fire_end(A, B.G, A.reps[r], A.clk[r], r, k);
+      if (k >= 0) flow_fire_end(A, G, A.reps[r], A.clk[r], r, k);
     }
-  if (!rebuild_phases<HOT_PLANE>(B, L, bar)) return false;
+  if (!rebuild_phases<HOT_PLANE>(B, G, nullptr, L, bar, Q)) return false;
   if (!again) return true;
   if (!grid_wait(bar)) return false;
   if ((__ldcg(B.bstatus) & ST_OVERFLOW) != 0) return true;
   for (int v = blockIdx.x; v < L.nblk; v += nb) {
     const int k = slot(v, r);
     if (k < 0) continue;
-    D4 g = ld4(B.G + k);
+    D4 g = ld4(G + k);
     int dix = 0, diy = 0;
     flow_enforce(A.reps[r], g, dix, diy);
-    stg4(B.G + k, g);
+    stg4(G + k, g);
     if (dix) A.d.ix[k] += dix;
     if (diy) A.d.iy[k] += diy;
   }
@@ -434,8 +434,8 @@ __device__ __forceinline__ bool flow_rebuild(const Program& P, const FlowArgs& A
     const int k = slot(v, r);
     if (k < 0) continue;
     double fx, fy, tz, e[MAX_PAIR];
-    const D4 g = ld4(B.G + k);
-    flow_gather<PAIR, ALIGN, false, true>(P, A.reps[r], B.G, A.st, A.nl, k, g, fx, fy, tz, e);
+    const D4 g = ld4(G + k);
+    flow_gather<PAIR, ALIGN, false, true>(P, A.reps[r], G, A.st, A.nl, k, g, fx, fy, tz, e);
     A.d.fx[k] = fx; A.d.fy[k] = fy;
     if (INTEG == FLOW_NVE) A.d.tz[k] = tz;
   }
@@ -474,6 +474,7 @@ __global__ void __launch_bounds__(BLOCK, 8)
 k_flow_begin(const __grid_constant__ Program P, const __grid_constant__ FlowArgs A, const __grid_constant__ RebuildArgs B,
              int sort_every, int tail, int begin, int pre) {
   __shared__ RebuildList L;
+  __shared__ RebuildScratch Q;
   const int t = threadIdx.x;
   if (B.clk[0].halt) return;  // set between launches only
   const unsigned long long t0 = global_ns();
@@ -483,7 +484,7 @@ k_flow_begin(const __grid_constant__ Program P, const __grid_constant__ FlowArgs
   bool over = false;
   if (flagged) {
     bar.n = rebuild_blocks(L);
-    if (blockIdx.x < bar.n && !flow_rebuild<INTEG, PAIR, ALIGN>(P, A, B, L, bar, begin)) return;
+    if (blockIdx.x < bar.n && !flow_rebuild<INTEG, PAIR, ALIGN>(P, A, B, A.G, L, Q, bar, begin)) return;
     if (!grid_wait_all(bar)) return;  // the neighbours' records move on below
     over = (__ldcg(B.bstatus) & ST_OVERFLOW) != 0;
   }
@@ -511,6 +512,7 @@ __global__ void __launch_bounds__(BLOCK, FLOW_RUN_MINB)
 k_flow_run(const __grid_constant__ Program P, const __grid_constant__ FlowArgs A, const __grid_constant__ RebuildArgs B,
            D4* G0, D4* G1, unsigned long long* word, int nsteps, int sort_every, int pre) {
   __shared__ RebuildList L;
+  __shared__ RebuildScratch Q;
   __shared__ unsigned long long seen;
   const int t = threadIdx.x;
   GridBar bar{B.bar, gridDim.x, 0u, 0u, B.status};
@@ -531,9 +533,10 @@ k_flow_run(const __grid_constant__ Program P, const __grid_constant__ FlowArgs A
     int ok = 1;
     if (t == 0) {
       red_release64(word + w, 1ull + (block_asks ? 1ull << 32 : 0ull));
-      unsigned long long x = ld_acquire64(word + w);
-      for (unsigned it = 0; (unsigned)x < target[w]; x = ld_acquire64(word + w))
+      unsigned long long x = ld_relaxed64(word + w);
+      for (unsigned it = 0; (unsigned)x < target[w]; x = ld_relaxed64(word + w))
         if (++it >= GRID_SPIN_LIMIT) { atomicOr(B.status, ST_TIMEOUT); ok = 0; break; }
+      fence_acquire();
       seen = x;
     }
     if (!__syncthreads_and(ok)) return;
@@ -547,9 +550,7 @@ k_flow_run(const __grid_constant__ Program P, const __grid_constant__ FlowArgs A
       const unsigned long long t0 = global_ns();
       // (a minimiser's replica may have converged in the step that asked)
       if (rebuild_list(B, sort_every, L, INTEG == FLOW_FIRE)) {
-        RebuildArgs Q = B;
-        Q.G = G;
-        if (!flow_rebuild<INTEG, PAIR, ALIGN>(P, A, Q, L, bar, more)) return;
+        if (!flow_rebuild<INTEG, PAIR, ALIGN>(P, A, B, G, L, Q, bar, more)) return;
         if (!grid_wait(bar)) return;
         over = (__ldcg(B.bstatus) & ST_OVERFLOW) != 0;
         rebuilt = true;

@@ -1259,19 +1259,23 @@ __device__ __forceinline__ void build_particle_packed(const Replica& R, int k, d
   // z-cells (a quasi-2-D box) the three columns of one x offset meet as well.
   int rs[27], rn[27], nr = 0;
   if (R.use_cell && c >= 1 && c + 1 < R.cnz) {
-    for (int ox = -1; ox <= 1; ox++) {
-      int ia = a + ox;
+    // all nine columns' ends requested before the first is used
+    int first[9], last[9];
+#pragma unroll
+    for (int m = 0; m < 9; m++) {
+      int ia = a + m / 3 - 1, ib = b + m % 3 - 1;
       if (ia < 0) ia = R.cnx - 1; else if (ia == R.cnx) ia = 0;
-      for (int oy = -1; oy <= 1; oy++) {
-        int ib = b + oy;
-        if (ib < 0) ib = R.cny - 1; else if (ib == R.cny) ib = 0;
-        const int f = R.cell_off + R.cny * R.cnz * ia + R.cnz * ib + (c - 1);
-        const int first = ld_int<COH>(cstart + f);
-        const int s0 = R.off + first - base0, n = ld_int<COH>(cstart + f + 2) + ld_int<COH>(ccnt + f + 2) - first;
-        if (n == 0) continue;
-        if (nr > 0 && rs[nr - 1] + rn[nr - 1] == s0) rn[nr - 1] += n;
-        else { rs[nr] = s0; rn[nr] = n; nr++; }
-      }
+      if (ib < 0) ib = R.cny - 1; else if (ib == R.cny) ib = 0;
+      const int f = R.cell_off + R.cny * R.cnz * ia + R.cnz * ib + (c - 1);
+      first[m] = ld_int<COH>(cstart + f);
+      last[m] = ld_int<COH>(cstart + f + 2) + ld_int<COH>(ccnt + f + 2);
+    }
+#pragma unroll
+    for (int m = 0; m < 9; m++) {
+      const int s0 = R.off + first[m] - base0, n = last[m] - first[m];
+      if (n == 0) continue;
+      if (nr > 0 && rs[nr - 1] + rn[nr - 1] == s0) rn[nr - 1] += n;
+      else { rs[nr] = s0; rn[nr] = n; nr++; }
     }
   } else {
     int cells[27];
@@ -1292,6 +1296,24 @@ __device__ __forceinline__ void build_particle_packed(const Replica& R, int k, d
   // one flat sweep over the runs' records (lanes of a warp stay together
   // across cell boundaries); each record requested one candidate ahead
   int ri = 0, pos = nr > 0 ? rs[0] : 0, end = nr > 0 ? rs[0] + rn[0] : 0;
+  // The pair test without branches.  The reference takes the difference from
+  // the lower id to the higher; the other direction only changes its sign, and
+  // the box is centred (xlo = -xhi), so the wrap and the squares are the same.
+  // Without periodicity the wrap adds a zero.
+  const double hx = R.xhi, hy = R.yhi, hz = R.zhi, cut2 = R.cut2;
+  const double Lx = R.periodic ? R.Lx : 0.0, Ly = R.periodic ? R.Ly : 0.0, Lz = R.periodic ? R.Lz : 0.0;
+  auto test = [&](const D4& cr) {
+    double dx = cr.x - x, dy = cr.y - y, dz = cr.z - z;
+    dx += dx > hx ? -Lx : dx < -hx ? Lx : 0.0;
+    dy += dy > hy ? -Ly : dy < -hy ? Ly : 0.0;
+    dz += dz > hz ? -Lz : dz < -hz ? Lz : 0.0;
+    if (dx * dx + dy * dy + dz * dz < cut2) {
+      const unsigned long long key = (unsigned long long)__double_as_longlong(cr.w);
+      const int jid = (int)(unsigned)(key >> 32);
+      if (jid < myid) { if (nlo < NB_LOCAL) lo[nlo] = key; nlo++; }
+      else if (jid != myid) { if (nup < NB_LOCAL) up[nup] = key; nup++; }
+    }
+  };
   D4 nxt = total > 0 ? ld_rec<COH>(cand + pos) : D4{0.0, 0.0, 0.0, 0.0};
   for (int t = 0; t < total; t++) {
     const D4 cr = nxt;
@@ -1299,19 +1321,7 @@ __device__ __forceinline__ void build_particle_packed(const Replica& R, int k, d
       if (++pos == end) { ri++; pos = rs[ri]; end = pos + rn[ri]; }
       nxt = ld_rec<COH>(cand + pos);
     }
-    {
-      const unsigned long long key = (unsigned long long)__double_as_longlong(cr.w);
-      const int jid = (int)(unsigned)(key >> 32);
-      if (jid == myid) continue;
-      double dx, dy, dz;
-      if (myid < jid) { dx = x - cr.x; dy = y - cr.y; dz = z - cr.z; }
-      else { dx = cr.x - x; dy = cr.y - y; dz = cr.z - z; }
-      apply_periodic(R, dx, dy, dz);
-      if (dx * dx + dy * dy + dz * dz < R.cut2) {
-        if (jid < myid) { if (nlo < NB_LOCAL) lo[nlo] = key; nlo++; }
-        else { if (nup < NB_LOCAL) up[nup] = key; nup++; }
-      }
-    }
+    test(cr);
   }
   if (nlo > NB_LOCAL || (!R.use_cell && nup > NB_LOCAL)) overflow = true;
   const int found = nlo + nup;

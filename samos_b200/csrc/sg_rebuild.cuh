@@ -21,17 +21,22 @@ namespace sg {
 // ---------------------------------------------------------------------------
 constexpr unsigned GRID_SPIN_LIMIT = 1u << 24;
 
-__device__ __forceinline__ unsigned ld_acquire(const unsigned* p) {
+// A waiting block polls with relaxed loads and takes one fence when the wait is
+// over: an acquire load drops the SM's L1 lines, and polling with it made the
+// loads of the blocks still at work beside the waiting one miss (list build of
+// ten blocks 40 us, now 19).
+__device__ __forceinline__ unsigned ld_relaxed(const unsigned* p) {
   unsigned v;
-  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
   return v;
 }
 
-__device__ __forceinline__ unsigned long long ld_acquire64(const unsigned long long* p) {
+__device__ __forceinline__ unsigned long long ld_relaxed64(const unsigned long long* p) {
   unsigned long long v;
-  asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+  asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
   return v;
 }
+__device__ __forceinline__ void fence_acquire() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
 
 __device__ __forceinline__ void red_release64(unsigned long long* p, unsigned long long v) {
   asm volatile("red.release.gpu.global.add.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
@@ -52,8 +57,9 @@ __device__ __forceinline__ bool grid_arrive_wait(unsigned* word, unsigned target
   if (threadIdx.x == 0) {
     asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(word) : "memory");
     unsigned it = 0;
-    while (ld_acquire(word) < target && ++it < GRID_SPIN_LIMIT)
+    while (ld_relaxed(word) < target && ++it < GRID_SPIN_LIMIT)
       if (BACKOFF) __nanosleep(100);
+    fence_acquire();
     if (it >= GRID_SPIN_LIMIT) { atomicOr(status, ST_TIMEOUT); ok = 0; }
   }
   return __syncthreads_and(ok) != 0;
@@ -86,7 +92,7 @@ __device__ __forceinline__ bool grid_last(GridBar& g) {
 }
 
 // ---------------------------------------------------------------------------
-constexpr int RB_MAX_REP = 512;  // replicas whose flags a block keeps in shared memory
+constexpr int RB_MAX_REP = 256;  // replicas whose flags a block keeps in shared memory
 
 struct RebuildStats { unsigned long long ns; int builds; int maxnb; };
 
@@ -100,7 +106,7 @@ struct RebuildArgs {
   Dyn cur, alt;
   Stat st, st_alt;
   NbList nl;
-  D4 *G, *H;        // packed records (HOT_PLANE / HOT_SPHERE)
+  D4 *G, *H;        // packed records (HOT_PLANE / HOT_SPHERE; a resident run passes its own)
   int *pcell, *cell_cnt, *cell_start, *cell_fill, *tmp, *perm, *bsum;
   D4* cand;
   uint8_t* lane_order;  // null: not kept
@@ -173,22 +179,22 @@ __device__ __forceinline__ int list_find(const int* first, int n, int v) {  // l
 
 // position of slot k as the list build sees it
 template <int SHAPE>
-__device__ __forceinline__ void rb_position(const RebuildArgs& A, int k, double& x, double& y, double& z) {
+__device__ __forceinline__ void rb_position(const RebuildArgs& A, const D4* G, int k, double& x, double& y, double& z) {
   if (SHAPE == HOT_NONE) { x = A.cur.x[k]; y = A.cur.y[k]; z = A.cur.z[k]; }
   else {
-    const D4 g = ld4(A.G + k);
+    const D4 g = ld4(G + k);
     x = g.x; y = g.y;
     z = SHAPE == HOT_PLANE ? A.cur.z[k] : g.z;
   }
 }
 template <int SHAPE>
-__device__ __forceinline__ void rb_store_position(const RebuildArgs& A, int k, double x, double y, double z) {
+__device__ __forceinline__ void rb_store_position(const RebuildArgs& A, D4* G, int k, double x, double y, double z) {
   if (SHAPE == HOT_NONE) { A.cur.x[k] = x; A.cur.y[k] = y; A.cur.z[k] = z; }
   else {
-    D4 g = ld4(A.G + k);
+    D4 g = ld4(G + k);
     g.x = x; g.y = y;
     if (SHAPE == HOT_SPHERE) g.z = z; else A.cur.z[k] = z;
-    stg4(A.G + k, g);
+    stg4(G + k, g);
   }
 }
 
@@ -199,12 +205,101 @@ __device__ __forceinline__ unsigned rebuild_blocks(const RebuildList& L) {
   return min(gridDim.x, (unsigned)max(32, L.nblk));
 }
 
+// List build of one particle with everything that a thread indexes by a running
+// number in shared memory (as local arrays, each access was a miss to L2 when
+// only a few blocks rebuild: list build of 160 blocks 31 us, with this 10): the
+// nine columns of the stencil away from the z faces, up to RB_SIDE neighbours a
+// side.  False: not that simple, nothing written; build_particle_packed does it.
+constexpr int RB_SIDE = 12;
+struct RebuildScratch {
+  int at[9][BLOCK], end[9][BLOCK];        // candidate records of each column
+  unsigned long long lo[RB_SIDE][BLOCK];  // (id << 32) | slot
+  int up[RB_SIDE][BLOCK];
+};
+
+__device__ __forceinline__ bool build_particle_small(const Replica& R, int k, double x, double y, double z, int myid,
+                                                     const NbList& nl, const D4* cand, const int* cstart,
+                                                     const int* ccnt, int* status, int* maxnb, RebuildScratch& Q) {
+  int a, b, c;
+  cell_of(R, x, y, z, a, b, c);
+  if (!(R.use_cell && c >= 1 && c + 1 < R.cnz)) return false;
+  const int t = threadIdx.x, base = R.off - cstart[R.cell_off];
+  int first[9], last[9], total = 0;
+#pragma unroll
+  for (int m = 0; m < 9; m++) {
+    int ia = a + m / 3 - 1, ib = b + m % 3 - 1;
+    if (ia < 0) ia = R.cnx - 1; else if (ia == R.cnx) ia = 0;
+    if (ib < 0) ib = R.cny - 1; else if (ib == R.cny) ib = 0;
+    const int f = R.cell_off + R.cny * R.cnz * ia + R.cnz * ib + (c - 1);
+    first[m] = cstart[f];
+    last[m] = cstart[f + 2] + ccnt[f + 2];
+  }
+  int nr = 0;
+#pragma unroll
+  for (int m = 0; m < 9; m++)
+    if (last[m] > first[m]) {
+      Q.at[nr][t] = base + first[m]; Q.end[nr][t] = base + last[m];
+      nr++;
+      total += last[m] - first[m];
+    }
+  const double hx = R.xhi, hy = R.yhi, hz = R.zhi, cut2 = R.cut2;
+  const double Lx = R.periodic ? R.Lx : 0.0, Ly = R.periodic ? R.Ly : 0.0, Lz = R.periodic ? R.Lz : 0.0;
+  int nlo = 0, nup = 0, run = 0, pos = nr ? Q.at[0][t] : 0, end = nr ? Q.end[0][t] : 0;
+  constexpr int U = 4;  // records in flight
+  for (int s = 0; s < total; s += U) {
+    D4 cr[U];
+#pragma unroll
+    for (int u = 0; u < U; u++)
+      if (s + u < total) {
+        if (pos == end) { run++; pos = Q.at[run][t]; end = Q.end[run][t]; }
+        cr[u] = ld4(cand + pos++);
+      }
+#pragma unroll
+    for (int u = 0; u < U; u++)
+      if (s + u < total) {  // (the test of build_particle_packed)
+        double dx = cr[u].x - x, dy = cr[u].y - y, dz = cr[u].z - z;
+        dx += dx > hx ? -Lx : dx < -hx ? Lx : 0.0;
+        dy += dy > hy ? -Ly : dy < -hy ? Ly : 0.0;
+        dz += dz > hz ? -Lz : dz < -hz ? Lz : 0.0;
+        if (dx * dx + dy * dy + dz * dz < cut2) {
+          const unsigned long long key = (unsigned long long)__double_as_longlong(cr[u].w);
+          const int jid = (int)(unsigned)(key >> 32);
+          if (jid < myid) { if (nlo < RB_SIDE) Q.lo[nlo][t] = key; nlo++; }
+          else if (jid != myid) { if (nup < RB_SIDE) Q.up[nup][t] = (int)(unsigned)key; nup++; }
+        }
+      }
+  }
+  if (nlo > RB_SIDE || nup > RB_SIDE) return false;
+  const int found = nlo + nup;
+  atomicMax(maxnb, found);
+  nl.ox[k] = x; nl.oy[k] = y; nl.oz[k] = z;
+  if (found > nl.cap) {
+    atomicOr(status, ST_OVERFLOW);
+    nl.cnt[k] = 0; nl.lo[k] = 0;
+    return true;
+  }
+  for (int i = 1; i < nlo; i++) {  // insertion sort by id (stable)
+    const unsigned long long v = Q.lo[i][t];
+    int m = i - 1;
+    for (; m >= 0; m--) {
+      const unsigned long long w = Q.lo[m][t];
+      if ((w >> 32) <= (v >> 32)) break;
+      Q.lo[m + 1][t] = w;
+    }
+    Q.lo[m + 1][t] = v;
+  }
+  for (int q = 0; q < nlo; q++) nl.nb[(size_t)q * nl.stride + k] = (int)(unsigned)Q.lo[q][t];
+  for (int q = 0; q < nup; q++) nl.nb[(size_t)(nlo + q) * nl.stride + k] = Q.up[q][t];
+  nl.cnt[k] = found; nl.lo[k] = nlo;
+  return true;
+}
+
 // All phases for the replicas in L, by the first bar.n blocks of the launch.
 // False: a barrier's wait ran out.  Always inlined: as one function called from
 // kernels with different register bounds it came out wrong (a caller's value in
 // place of a coordinate).
 template <int SHAPE>
-__device__ __forceinline__ bool rebuild_phases(const RebuildArgs& A, RebuildList& L, GridBar& bar) {
+__device__ __forceinline__ bool rebuild_phases(const RebuildArgs& A, D4* G, D4* H, RebuildList& L, GridBar& bar, RebuildScratch& Q) {
   const int nb = (int)bar.n;
   const int t = threadIdx.x, nthr = nb * blockDim.x, gid = blockIdx.x * blockDim.x + t;
   __shared__ int shw[32];
@@ -222,13 +317,13 @@ __device__ __forceinline__ bool rebuild_phases(const RebuildArgs& A, RebuildList
     const int k = R.off + (v - L.blk[s]) * BLOCK + t;
     if (k - R.off >= R.n) continue;
     double x, y, z;
-    rb_position<SHAPE>(A, k, x, y, z);
+    rb_position<SHAPE>(A, G, k, x, y, z);
     if (R.periodic) {
       bool ch = false;
       if (x < R.xlo) { x += R.Lx; ch = true; } else if (x > R.xhi) { x -= R.Lx; ch = true; }
       if (y < R.ylo) { y += R.Ly; ch = true; } else if (y > R.yhi) { y -= R.Ly; ch = true; }
       if (z < R.zlo) { z += R.Lz; ch = true; } else if (z > R.zhi) { z -= R.Lz; ch = true; }
-      if (ch) rb_store_position<SHAPE>(A, k, x, y, z);
+      if (ch) rb_store_position<SHAPE>(A, G, k, x, y, z);
     }
     int a, b, c;
     const int cl = cell_of(R, x, y, z, a, b, c);
@@ -312,7 +407,7 @@ __device__ __forceinline__ bool rebuild_phases(const RebuildArgs& A, RebuildList
     for (int q = 0; q < n; q++) rank += A.st.id[A.tmp[s0 + q]] < myid ? 1 : 0;
     A.perm[s0 + rank] = k;
     double x, y, z;
-    rb_position<SHAPE>(A, k, x, y, z);
+    rb_position<SHAPE>(A, G, k, x, y, z);
     stg4(A.cand + s0 + rank, D4{x, y, z, pack_id_slot(myid, L.mode[s] == 2 ? s0 + rank : k)});
   }
   if (!grid_wait(bar)) return false;
@@ -332,10 +427,10 @@ __device__ __forceinline__ bool rebuild_phases(const RebuildArgs& A, RebuildList
         Part p;
         load_dyn(A.cur, o, p);
         if (SHAPE != HOT_NONE) {
-          const D4 g = ld4(A.G + o);
+          const D4 g = ld4(G + o);
           p.x = g.x; p.y = g.y;
           if (SHAPE == HOT_PLANE) { p.nx = g.z; p.ny = g.w; }
-          else { const D4 h = ld4(A.H + o); p.z = g.z; p.nx = h.x; p.ny = h.y; p.nz = h.z; }
+          else { const D4 h = ld4(H + o); p.z = g.z; p.nx = h.x; p.ny = h.y; p.nz = h.z; }
         }
         store_dyn(A.alt, k, p);
         A.st_alt.r[k] = A.st.r[o]; A.st_alt.mass[k] = A.st.mass[o];
@@ -343,11 +438,13 @@ __device__ __forceinline__ bool rebuild_phases(const RebuildArgs& A, RebuildList
         x = p.x; y = p.y; z = p.z;
         myid = A.st.id[o];
       } else {
-        rb_position<SHAPE>(A, k, x, y, z);
+        rb_position<SHAPE>(A, G, k, x, y, z);
         myid = A.st.id[k];
       }
-      build_particle_packed<true>(R, k, x, y, z, myid, A.nl, A.cand, A.cell_start, A.cell_cnt, A.bstatus,
-                                  &A.stats->maxnb);
+      if (!build_particle_small(R, k, x, y, z, myid, A.nl, A.cand, A.cell_start, A.cell_cnt, A.bstatus,
+                                &A.stats->maxnb, Q))
+        build_particle_packed<true>(R, k, x, y, z, myid, A.nl, A.cand, A.cell_start, A.cell_cnt, A.bstatus,
+                                    &A.stats->maxnb);
     }
     if (A.lane_order) {
       __syncthreads();
@@ -368,10 +465,10 @@ __device__ __forceinline__ bool rebuild_phases(const RebuildArgs& A, RebuildList
       store_dyn(A.cur, k, p);
       A.st.r[k] = A.st_alt.r[k]; A.st.mass[k] = A.st_alt.mass[k];
       A.st.type[k] = A.st_alt.type[k]; A.st.id[k] = A.st_alt.id[k];
-      if (SHAPE == HOT_PLANE) stg4(A.G + k, D4{p.x, p.y, p.nx, p.ny});
+      if (SHAPE == HOT_PLANE) stg4(G + k, D4{p.x, p.y, p.nx, p.ny});
       if (SHAPE == HOT_SPHERE) {
-        stg4(A.G + k, D4{p.x, p.y, p.z, A.st_alt.r[k]});
-        stg4(A.H + k, D4{p.nx, p.ny, p.nz, 0.0});
+        stg4(G + k, D4{p.x, p.y, p.z, A.st_alt.r[k]});
+        stg4(H + k, D4{p.nx, p.ny, p.nz, 0.0});
       }
     }
   }
@@ -401,8 +498,9 @@ __device__ __forceinline__ void rebuild_done(const RebuildArgs& A, const Rebuild
 // (as k_tail_batch), and the flagged replicas' lists are rebuilt.
 template <int SHAPE>
 __global__ void __launch_bounds__(BLOCK)
-k_tail_rebuild(Program P, RebuildArgs A, int sort_every) {
+k_tail_rebuild(const __grid_constant__ Program P, const __grid_constant__ RebuildArgs A, int sort_every) {
   __shared__ RebuildList L;
+  __shared__ RebuildScratch Q;
   if (A.clk[0].halt) return;  // set between launches only: the same for every block
   const unsigned long long t0 = global_ns();
   if (blockIdx.x == 0) {
@@ -411,7 +509,23 @@ k_tail_rebuild(Program P, RebuildArgs A, int sort_every) {
   }
   if (!rebuild_list(A, sort_every, L)) return;
   GridBar bar{A.bar, rebuild_blocks(L), 0u, 0u, A.status};
-  if (blockIdx.x < bar.n && !rebuild_phases<SHAPE>(A, L, bar)) return;
+  if (blockIdx.x < bar.n && !rebuild_phases<SHAPE>(A, A.G, A.H, L, bar, Q)) return;
+  if (grid_last(bar)) rebuild_done(A, L, t0);
+}
+
+// Rebuild between two launches of a resident run: the state is in G0 / H0 after
+// an even number of steps, in G1 / H1 after an odd one.
+template <int SHAPE>
+__global__ void __launch_bounds__(BLOCK)
+k_run_rebuild(const __grid_constant__ RebuildArgs A, D4* G0, D4* G1, D4* H0, D4* H1, int sort_every) {
+  __shared__ RebuildList L;
+  __shared__ RebuildScratch Q;
+  if (A.clk[0].halt) return;
+  const unsigned long long t0 = global_ns();
+  const bool odd = *A.executed & 1;
+  if (!rebuild_list(A, sort_every, L)) return;
+  GridBar bar{A.bar, rebuild_blocks(L), 0u, 0u, A.status};
+  if (blockIdx.x < bar.n && !rebuild_phases<SHAPE>(A, odd ? G1 : G0, odd ? H1 : H0, L, bar, Q)) return;
   if (grid_last(bar)) rebuild_done(A, L, t0);
 }
 
