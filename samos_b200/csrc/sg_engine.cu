@@ -306,7 +306,7 @@ int sg_create(int n_replicas, const int32_t* n_particles, int ntypes, sg_system*
   s->rebuild = m.alloc<int>(n_replicas);
   s->status = m.alloc<int>(1);
   s->bstatus = m.alloc<int>(1);
-  s->exec_cnt = m.alloc<int>(2);
+  s->exec_cnt = m.alloc<int>(3);
   s->fire_cnt = m.alloc<int>(n_replicas);
   s->maxnb = m.alloc<int>(1);
   s->epart = m.alloc<double>((size_t)(MAX_PAIR + MAX_ALIGN) * s->nblocks);
@@ -2076,6 +2076,13 @@ static int run_batch(sg_system* s, int shape, int64_t K, bool needs_nl, int64_t*
   return rebuild_pending(s, shape, false, rebuild_ms);
 }
 
+// steps between rebuilds, from the device's count over the steps just done
+static void note_gap(sg_system* s, int64_t steps, int builds) {
+  if (builds > s->rb_builds_seen) s->last_gap = std::max<int64_t>(1, steps / (builds - s->rb_builds_seen));
+  else s->last_gap = std::max<int64_t>(s->last_gap, steps);
+  s->rb_builds_seen = builds;
+}
+
 // Resident runs (k_abp_run): the whole system on the device at once, steps and
 // rebuilds in one launch.  For every specialised program whose temperatures are
 // constant (the noise counters then advance by a fixed number a step), unless a
@@ -2132,9 +2139,7 @@ static int run_resident(sg_system* s, int shape, int64_t K, int64_t* executed, d
   CU(s, cudaMemcpyAsync(&rb, s->rb_stats, sizeof(rb), cudaMemcpyDeviceToHost, s->stream));
   CU(s, cudaMemcpyAsync(s->rebuild_h, s->rebuild, sizeof(int) * s->nrep, cudaMemcpyDeviceToHost, s->stream));
   CU(s, cudaStreamSynchronize(s->stream));
-  if (rb.builds > s->rb_builds_seen) s->last_gap = std::max<int64_t>(1, ex / (rb.builds - s->rb_builds_seen));
-  else s->last_gap = std::max<int64_t>(s->last_gap, ex);
-  s->rb_builds_seen = rb.builds;
+  note_gap(s, ex, rb.builds);
   if (st & ST_TIMEOUT) return grid_timeout(s);
   if (ex < 1 || ex > K) return fail(s, SG_ERR_CUDA, "resident run: inconsistent step count");
   s->hot_buf = b ^ (int)(ex & 1);
@@ -2301,38 +2306,49 @@ static int run_flow(sg_system* s, int64_t K, bool driver, int64_t* executed, dou
   A.blist = al; A.nblist = na; A.d = s->cur;
   const bool flips = kind.integ == FLOW_NVE;  // the force pass writes the other record buffer
   const int b0 = s->hot_buf, grid = std::max(1, std::min(s->flow_grid, na));
-  CU(s, cudaMemsetAsync(s->exec_cnt, 0, 2 * sizeof(int), s->stream));
-  A.Gin = A.G = s->G[b0];
-  const bool resident = na <= s->flow_run_grid;
-  if (resident) {
-    CU(s, flow_run(kind, P, A, rebuild_args(s, HOT_PLANE), s->G[b0], s->G[1 - b0], s->run_word, (int)K, kSortEvery, fresh,
-                   std::max(1, std::min(s->flow_run_grid, na)), s->stream));
-    s->launches++;
-  } else {
-  CU(s, flow_begin(kind, P, A, rebuild_args(s, HOT_PLANE), kSortEvery, false, true, fresh, grid, s->stream));
+  D4 *G0 = s->G[b0], *G1 = s->G[1 - b0];
+  CU(s, cudaMemsetAsync(s->exec_cnt, 0, 3 * sizeof(int), s->stream));
+  A.Gin = A.G = G0;
+  CU(s, flow_begin(kind, P, A, rebuild_args(s, HOT_PLANE), kSortEvery, false, true, fresh, 0, G0, G1, grid, s->stream));
   s->launches++;
-  for (int64_t i = 0; i < K; i++) {
-    A.Gin = s->G[s->hot_buf];
-    if (flips) s->hot_buf = 1 - s->hot_buf;
-    A.G = s->G[s->hot_buf];
-    CU(s, flow_force(kind, P, A, s->stream));
-    CU(s, flow_begin(kind, P, A, rebuild_args(s, HOT_PLANE), kSortEvery, true, i + 1 < K, true, grid, s->stream));
-    s->launches += 2;
-  }
-  }
+  const bool resident = na <= s->flow_run_grid;
+  if (!resident)
+    for (int64_t i = 0; i < K; i++) {
+      A.Gin = s->G[s->hot_buf];
+      if (flips) s->hot_buf = 1 - s->hot_buf;
+      A.G = s->G[s->hot_buf];
+      CU(s, flow_force(kind, P, A, s->stream));
+      CU(s, flow_begin(kind, P, A, rebuild_args(s, HOT_PLANE), kSortEvery, true, i + 1 < K, true, 0, G0, G1, grid,
+                       s->stream));
+      s->launches += 2;
+    }
   int ex[2] = {0, 0}, st = 0;
-  CU(s, cudaMemcpyAsync(ex, s->exec_cnt, sizeof(ex), cudaMemcpyDeviceToHost, s->stream));
-  CU(s, cudaMemcpyAsync(&st, s->status, sizeof(int), cudaMemcpyDeviceToHost, s->stream));
-  CU(s, cudaMemcpyAsync(s->rebuild_h, s->rebuild, sizeof(int) * s->nrep, cudaMemcpyDeviceToHost, s->stream));
-  CU(s, cudaStreamSynchronize(s->stream));
-  if (st & ST_TIMEOUT) return grid_timeout(s);
-  if (ex[0] < 1 || ex[0] > K) return fail(s, SG_ERR_CUDA, "two-launch steps: inconsistent step count");
+  RebuildStats rb{};
+  bool any = false;
+  do {
+    if (resident) {  // a launch for every stretch between rebuilds that the last gap suggests, and one more
+      const RebuildArgs B = rebuild_args(s, HOT_PLANE);
+      const int64_t stretches = std::min<int64_t>(16, 2 + (K - ex[0]) / std::max<int64_t>(1, s->last_gap));
+      for (int64_t i = 0; i < stretches; i++) {
+        CU(s, flow_run(kind, P, A, B, G0, G1, s->run_word, (int)K, std::max(1, na), s->stream));
+        CU(s, flow_begin(kind, P, A, B, kSortEvery, true, true, true, (int)K, G0, G1, grid, s->stream));
+        s->launches += 2;
+      }
+    }
+    CU(s, cudaMemcpyAsync(ex, s->exec_cnt, sizeof(ex), cudaMemcpyDeviceToHost, s->stream));
+    CU(s, cudaMemcpyAsync(&st, s->status, sizeof(int), cudaMemcpyDeviceToHost, s->stream));
+    CU(s, cudaMemcpyAsync(&rb, s->rb_stats, sizeof(rb), cudaMemcpyDeviceToHost, s->stream));
+    CU(s, cudaMemcpyAsync(s->rebuild_h, s->rebuild, sizeof(int) * s->nrep, cudaMemcpyDeviceToHost, s->stream));
+    CU(s, cudaStreamSynchronize(s->stream));
+    if (st & ST_TIMEOUT) return grid_timeout(s);
+    if (ex[0] < 1 || ex[0] > K) return fail(s, SG_ERR_CUDA, "two-launch steps: inconsistent step count");
+    for (int r = 0; r < s->nrep; r++) any = any || s->rebuild_h[r];
+  } while (resident && ex[0] < K && !any);  // a stretch that ended early has begun its next step
+  note_gap(s, ex[0], rb.builds);
   if (flips) s->hot_buf = b0 ^ (int)(ex[0] & 1);
   *executed = ex[0];
   s->since_rebuild += ex[0];
   s->forces_fresh = ex[1] == 0;
-  bool any = false;
-  for (int r = 0; r < s->nrep; r++) any = any || s->rebuild_h[r];
   if (!any) return SG_OK;
   // lists that did not fit: grown and rebuilt by the host
   if ((rc = flow_leave(s))) return rc;

@@ -74,11 +74,13 @@ struct LaunchBegin {
   const Program& P;
   const FlowArgs& A;
   const RebuildArgs& B;
-  int sort_every, tail, begin, pre, grid;
+  D4 *G0, *G1;
+  int sort_every, tail, begin, pre, nsteps, grid;
   cudaStream_t stream;
   template <int I, int Q, int L> cudaError_t operator()() const {
-    int se = sort_every, ta = tail, be = begin, pr = pre;
-    void* args[] = {const_cast<Program*>(&P), const_cast<FlowArgs*>(&A), const_cast<RebuildArgs*>(&B), &se, &ta, &be, &pr};
+    LaunchBegin a = *this;
+    void* args[] = {const_cast<Program*>(&P), const_cast<FlowArgs*>(&A), const_cast<RebuildArgs*>(&B), &a.G0, &a.G1,
+                    &a.sort_every, &a.tail, &a.begin, &a.pre, &a.nsteps};
     return cudaLaunchCooperativeKernel((const void*)k_flow_begin<I, Q, L>, dim3(grid), dim3(BLOCK), args, 0, stream);
   }
 };
@@ -95,8 +97,8 @@ cudaError_t flow_force(const FlowKind& K, const Program& P, const FlowArgs& A, c
 }
 
 cudaError_t flow_begin(const FlowKind& K, const Program& P, const FlowArgs& A, const RebuildArgs& B, int sort_every,
-                       bool tail, bool begin, bool pre, int grid, cudaStream_t stream) {
-  return flow_dispatch(K, LaunchBegin{P, A, B, sort_every, tail, begin, pre, grid, stream});
+                       bool tail, bool begin, bool pre, int nsteps, D4* G0, D4* G1, int grid, cudaStream_t stream) {
+  return flow_dispatch(K, LaunchBegin{P, A, B, G0, G1, sort_every, tail, begin, pre, nsteps, grid, stream});
 }
 
 cudaError_t flow_begin_occupancy(const FlowKind& K, int* blocks_per_sm) {
@@ -109,12 +111,12 @@ struct LaunchRun {
   const RebuildArgs& B;
   D4 *G0, *G1;
   unsigned long long* word;
-  int nsteps, sort_every, pre, grid;
+  int nsteps, grid;
   cudaStream_t stream;
   template <int I, int Q, int L> cudaError_t operator()() const {
     LaunchRun a = *this;
     void* args[] = {const_cast<Program*>(&P), const_cast<FlowArgs*>(&A), const_cast<RebuildArgs*>(&B), &a.G0, &a.G1,
-                    &a.word, &a.nsteps, &a.sort_every, &a.pre};
+                    &a.word, &a.nsteps};
     return cudaLaunchCooperativeKernel((const void*)k_flow_run<I, Q, L>, dim3(grid), dim3(BLOCK), args, 0, stream);
   }
 };
@@ -127,8 +129,8 @@ struct RunBlocks {
 };
 
 cudaError_t flow_run(const FlowKind& K, const Program& P, const FlowArgs& A, const RebuildArgs& B, D4* G0, D4* G1,
-                     unsigned long long* word, int nsteps, int sort_every, bool pre, int grid, cudaStream_t stream) {
-  return flow_dispatch(K, LaunchRun{P, A, B, G0, G1, word, nsteps, sort_every, pre, grid, stream});
+                     unsigned long long* word, int nsteps, int grid, cudaStream_t stream) {
+  return flow_dispatch(K, LaunchRun{P, A, B, G0, G1, word, nsteps, grid, stream});
 }
 
 cudaError_t flow_run_occupancy(const FlowKind& K, int* blocks_per_sm) {
