@@ -81,6 +81,12 @@ __device__ __forceinline__ int cell3(const Geo& G, double x, double y, double z,
   return G.cny * G.cnz * a + G.cnz * b + c;
 }
 
+__global__ void k_st_zero(int m, int* cnt, int* fill, int* overflow) {
+  const int v = blockIdx.x * blockDim.x + threadIdx.x;
+  if (v < m) { cnt[v] = 0; fill[v] = 0; }
+  if (v == 0) *overflow = 0;
+}
+
 __global__ void k_st_bin(Geo G, const double* __restrict__ x, const double* __restrict__ y,
                          const double* __restrict__ z, int* pcell, int* cnt) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -146,11 +152,90 @@ __global__ void k_st_rank(int n, const int* __restrict__ pcell, const int* __res
   slots[s0 + rank] = i;
 }
 
+// Neighbours a side that the fast search keeps in shared memory.
+constexpr int kSide = 16;
+constexpr int kForceThreads = 128;
+
+// The neighbours of one particle away from the z faces, lower ids sorted and
+// higher ids in stencil order, in shared memory: three cells of a column are
+// consecutive in `slots`, four candidates are in flight, the test has no
+// branches (the sign of the difference does not change the wrap in a centred
+// box, nor the square).  With the candidates one after the other and the finds
+// in local memory the kernel was a chain of misses: 65 us for 30,011 particles.
+// False: not that simple, search_all does it.
+__device__ __forceinline__ bool search_columns(const Geo& G, const double* __restrict__ x, const double* __restrict__ y,
+                                               const double* __restrict__ z, const int* __restrict__ start,
+                                               const int* __restrict__ cnt, const int* __restrict__ slots, int i,
+                                               double xi, double yi, double zi, int (*lo)[kForceThreads],
+                                               int (*up)[kForceThreads], int (*at)[kForceThreads],
+                                               int (*end)[kForceThreads], int& nlo, int& nup) {
+  int a, b, c;
+  cell3(G, xi, yi, zi, a, b, c);
+  if (!(G.use_cell && c >= 1 && c + 1 < G.cnz)) return false;
+  const int t = threadIdx.x;
+  int first[9], last[9];
+#pragma unroll
+  for (int m = 0; m < 9; m++) {
+    int ia = a + m / 3 - 1, ib = b + m % 3 - 1;
+    if (ia < 0) ia = G.cnx - 1; else if (ia == G.cnx) ia = 0;
+    if (ib < 0) ib = G.cny - 1; else if (ib == G.cny) ib = 0;
+    const int f = G.cny * G.cnz * ia + G.cnz * ib + (c - 1);
+    first[m] = start[f];
+    last[m] = start[f + 2] + cnt[f + 2];
+  }
+  int nr = 0, total = 0;
+#pragma unroll
+  for (int m = 0; m < 9; m++)
+    if (last[m] > first[m]) {
+      at[nr][t] = first[m]; end[nr][t] = last[m];
+      nr++;
+      total += last[m] - first[m];
+    }
+  const double hx = G.xhi, hy = G.yhi, hz = G.zhi;
+  const double Lx = G.periodic ? G.Lx : 0.0, Ly = G.periodic ? G.Ly : 0.0, Lz = G.periodic ? G.Lz : 0.0;
+  int run = 0, pos = nr ? at[0][t] : 0, stop = nr ? end[0][t] : 0;
+  nlo = nup = 0;
+  constexpr int U = 4;
+  for (int s = 0; s < total; s += U) {
+    int j[U];
+    double dx[U], dy[U], dz[U];
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      j[u] = i;
+      if (s + u < total) {
+        if (pos == stop) { run++; pos = at[run][t]; stop = end[run][t]; }
+        j[u] = slots[pos++];
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < U; u++) { dx[u] = x[j[u]] - xi; dy[u] = y[j[u]] - yi; dz[u] = z[j[u]] - zi; }
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      dx[u] += dx[u] > hx ? -Lx : dx[u] < -hx ? Lx : 0.0;
+      dy[u] += dy[u] > hy ? -Ly : dy[u] < -hy ? Ly : 0.0;
+      dz[u] += dz[u] > hz ? -Lz : dz[u] < -hz ? Lz : 0.0;
+      if (j[u] != i && dx[u] * dx[u] + dy[u] * dy[u] + dz[u] * dz[u] < G.cut2) {
+        if (j[u] < i) { if (nlo < kSide) lo[nlo][t] = j[u]; nlo++; }
+        else { if (nup < kSide) up[nup][t] = j[u]; nup++; }
+      }
+    }
+  }
+  if (nlo > kSide || nup > kSide) return false;
+  for (int p = 1; p < nlo; p++) {  // stable insertion sort by id
+    const int v = lo[p][t];
+    int q = p - 1;
+    for (; q >= 0 && lo[q][t] > v; q--) lo[q + 1][t] = lo[q][t];
+    lo[q + 1][t] = v;
+  }
+  return true;
+}
+
 constexpr int kLocal = 64;
 
 // one particle: lower-id neighbours in ascending id, then higher-id ones in
 // the reference's list order (27-cell stencil; ascending id on the N^2 path)
-__global__ void k_st_forces(Geo G, const double* __restrict__ x, const double* __restrict__ y,
+__global__ void __launch_bounds__(kForceThreads)
+k_st_forces(Geo G, const double* __restrict__ x, const double* __restrict__ y,
                             const double* __restrict__ z, const double* __restrict__ nx,
                             const double* __restrict__ ny, const double* __restrict__ nz,
                             const double* __restrict__ rad, const int* __restrict__ start,
@@ -162,66 +247,83 @@ __global__ void k_st_forces(Geo G, const double* __restrict__ x, const double* _
   if (i >= G.n) return;
   const double xi = x[i], yi = y[i], zi = z[i];
   const double nxi = nx[i], nyi = ny[i], nzi = nz[i], ri = rad[i];
-  int a, b, c;
-  cell3(G, xi, yi, zi, a, b, c);
-  int cells[27];
-  int ncells = 0;
-  for (int ox = -1; ox <= 1; ox++)
-    for (int oy = -1; oy <= 1; oy++)
-      for (int oz = -1; oz <= 1; oz++) {
-        int ia = a + ox, ib = b + oy, ic = c + oz;
-        if (ia < 0) ia = G.cnx - 1; else if (ia == G.cnx) ia = 0;
-        if (ib < 0) ib = G.cny - 1; else if (ib == G.cny) ib = 0;
-        if (ic < 0) ic = G.cnz - 1; else if (ic == G.cnz) ic = 0;
-        const int cl = G.cny * G.cnz * ia + G.cnz * ib + ic;
-        bool dup = false;
-        if (!G.use_cell)
-          for (int q = 0; q < ncells; q++) dup = dup || cells[q] == cl;
-        if (!dup) cells[ncells++] = cl;
-      }
-  int lo[kLocal], up[kLocal];
+  __shared__ int slo[kSide][kForceThreads], sup[kSide][kForceThreads], sat[9][kForceThreads], send[9][kForceThreads];
+  const int t = threadIdx.x;
+  int llo[kLocal], lup[kLocal];
   int nlo = 0, nup = 0;
-  bool over = false;
-  for (int m = 0; m < ncells; m++) {
-    const int cl = cells[m], s0 = start[cl], e = s0 + cnt[cl];
-    for (int s = s0; s < e; s++) {
-      const int j = slots[s];
-      if (j == i) continue;
-      double dx, dy, dz;
-      if (i < j) { dx = xi - x[j]; dy = yi - y[j]; dz = zi - z[j]; }
-      else { dx = x[j] - xi; dy = y[j] - yi; dz = z[j] - zi; }
-      wrap(G, dx, dy, dz);
-      if (dx * dx + dy * dy + dz * dz < G.cut2) {
-        if (j < i) { if (nlo < kLocal) lo[nlo++] = j; else over = true; }
-        else { if (nup < kLocal) up[nup++] = j; else over = true; }
+  const bool columns = search_columns(G, x, y, z, start, cnt, slots, i, xi, yi, zi, slo, sup, sat, send, nlo, nup);
+  if (!columns) {
+    nlo = nup = 0;
+    int a, b, c;
+    cell3(G, xi, yi, zi, a, b, c);
+    int cells[27];
+    int ncells = 0;
+    for (int ox = -1; ox <= 1; ox++)
+      for (int oy = -1; oy <= 1; oy++)
+        for (int oz = -1; oz <= 1; oz++) {
+          int ia = a + ox, ib = b + oy, ic = c + oz;
+          if (ia < 0) ia = G.cnx - 1; else if (ia == G.cnx) ia = 0;
+          if (ib < 0) ib = G.cny - 1; else if (ib == G.cny) ib = 0;
+          if (ic < 0) ic = G.cnz - 1; else if (ic == G.cnz) ic = 0;
+          const int cl = G.cny * G.cnz * ia + G.cnz * ib + ic;
+          bool dup = false;
+          if (!G.use_cell)
+            for (int q = 0; q < ncells; q++) dup = dup || cells[q] == cl;
+          if (!dup) cells[ncells++] = cl;
+        }
+    bool over = false;
+    for (int m = 0; m < ncells; m++) {
+      const int cl = cells[m], s0 = start[cl], e = s0 + cnt[cl];
+      for (int s = s0; s < e; s++) {
+        const int j = slots[s];
+        if (j == i) continue;
+        double dx, dy, dz;
+        if (i < j) { dx = xi - x[j]; dy = yi - y[j]; dz = zi - z[j]; }
+        else { dx = x[j] - xi; dy = y[j] - yi; dz = z[j] - zi; }
+        wrap(G, dx, dy, dz);
+        if (dx * dx + dy * dy + dz * dz < G.cut2) {
+          if (j < i) { if (nlo < kLocal) llo[nlo++] = j; else over = true; }
+          else { if (nup < kLocal) lup[nup++] = j; else over = true; }
+        }
       }
     }
-  }
-  if (over) {  // more than kLocal neighbours on one side: flag this particle
-    const double bad = nan("");
-    fx[i] = bad; fy[i] = bad; fz[i] = bad; tx[i] = bad; ty[i] = bad; tz[i] = bad;
-    atomicAdd(overflow, 1);
-    return;
-  }
-  for (int p = 1; p < nlo; p++) {  // stable insertion sort by id
-    int v = lo[p], q = p - 1;
-    while (q >= 0 && lo[q] > v) { lo[q + 1] = lo[q]; q--; }
-    lo[q + 1] = v;
-  }
-  if (!G.use_cell)
-    for (int p = 1; p < nup; p++) {
-      int v = up[p], q = p - 1;
-      while (q >= 0 && up[q] > v) { up[q + 1] = up[q]; q--; }
-      up[q + 1] = v;
+    if (over) {  // more than kLocal neighbours on one side: flag this particle
+      const double bad = nan("");
+      fx[i] = bad; fy[i] = bad; fz[i] = bad; tx[i] = bad; ty[i] = bad; tz[i] = bad;
+      atomicAdd(overflow, 1);
+      return;
     }
+    for (int p = 1; p < nlo; p++) {  // stable insertion sort by id
+      int v = llo[p], q = p - 1;
+      while (q >= 0 && llo[q] > v) { llo[q + 1] = llo[q]; q--; }
+      llo[q + 1] = v;
+    }
+    if (!G.use_cell)
+      for (int p = 1; p < nup; p++) {
+        int v = lup[p], q = p - 1;
+        while (q >= 0 && lup[q] > v) { lup[q + 1] = lup[q]; q--; }
+        lup[q + 1] = v;
+      }
+  }
   double Fx = 0.0, Fy = 0.0, Fz = 0.0, Tx = 0.0, Ty = 0.0, Tz = 0.0;
-  for (int t = 0; t < nlo + nup; t++) {
-    const int j = t < nlo ? lo[t] : up[t - nlo];
-    double dx = x[j] - xi, dy = y[j] - yi, dz = z[j] - zi;
+  const int found = nlo + nup;
+  auto neighbour = [&](int q) {
+    return columns ? (q < nlo ? slo[q][t] : sup[q - nlo][t]) : q < nlo ? llo[q] : lup[q - nlo];
+  };
+  // the next neighbour's values requested before this one's are used
+  int j = 0 < found ? neighbour(0) : i;
+  double xn = x[j], yn = y[j], zn = z[j], rn = rad[j], un = nx[j], vn = ny[j], wn = nz[j];
+  for (int q = 0; q < found; q++) {
+    double dx = xn - xi, dy = yn - yi, dz = zn - zi;
+    const double rj = rn, onx = un, ony = vn, onz = wn;
+    if (q + 1 < found) {
+      j = neighbour(q + 1);
+      xn = x[j]; yn = y[j]; zn = z[j]; rn = rad[j]; un = nx[j]; vn = ny[j]; wn = nz[j];
+    }
     wrap(G, dx, dy, dz);
     const double r_sq = dx * dx + dy * dy + dz * dz;
     const double rd = sqrt(r_sq);
-    const double sig = use_radii ? ri + rad[j] : a_soft;
+    const double sig = use_radii ? ri + rj : a_soft;
     if (rd < sig) {
       const double diff = sig - rd;
       double ff;
@@ -229,7 +331,6 @@ __global__ void k_st_forces(Geo G, const double* __restrict__ x, const double* _
       Fx -= ff * dx; Fy -= ff * dy; Fz -= ff * dz;
     }
     if (align_kind >= 0 && r_sq <= rc * rc) {
-      const double onx = nx[j], ony = ny[j], onz = nz[j];
       const double tau_x = nyi * onz - nzi * ony;
       const double tau_y = nzi * onx - nxi * onz;
       const double tau_z = nxi * ony - nyi * onx;
@@ -338,10 +439,8 @@ extern "C" int sg_compute_static(int n, double lx, double ly, double lz, int per
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const int m = (int)ncell;
   // every call reuses the same scratch: clear what has to start at zero
-  if (cudaMemsetAsync(cnt, 0, sizeof(int) * m, st) != cudaSuccess) return SG_ERR_CUDA;
-  if (cudaMemsetAsync(fill, 0, sizeof(int) * m, st) != cudaSuccess) return SG_ERR_CUDA;
-  if (cudaMemsetAsync(overflow, 0, sizeof(int), st) != cudaSuccess) return SG_ERR_CUDA;
-  const int tb = 128, nbk = (n + tb - 1) / tb, nsc = (m + kScanTile - 1) / kScanTile;
+  k_st_zero<<<(m + 255) / 256, 256, 0, st>>>(m, cnt, fill, overflow);
+  const int tb = kForceThreads, nbk = (n + tb - 1) / tb, nsc = (m + kScanTile - 1) / kScanTile;
   k_st_bin<<<nbk, tb, 0, st>>>(G, x, y, z, pcell, cnt);
   k_st_scan_blocks<<<nsc, kScanTile, 0, st>>>(cnt, m, bsum);
   k_st_scan_final<<<nsc, kScanTile, 0, st>>>(cnt, m, bsum, nsc, start);
