@@ -191,13 +191,22 @@ __device__ __forceinline__ void hot_rotate(const ShapeGeom& G, Hp& p, double phi
 // ---------------------------------------------------------------------------
 // the hot step kernel
 // ---------------------------------------------------------------------------
-template <int SHAPE, bool ENERGY>
-__global__ void __launch_bounds__(BLOCK, 4)
-k_hot_step(Program P, const Replica* __restrict__ reps, const int* __restrict__ blk_rep,
+// PAIR / ALIGN: HOT_ANY, any program of these shapes through its component
+// loops; otherwise one pair potential and at most one aligner of one particle
+// type under one `brownian` integrator, their kinds known at compile time.
+// With the loops every neighbour went through the switch over the potentials and
+// the tables of the types; 500,009 particles with morse + polar: 81 us a step,
+// with the kinds fixed and the next neighbour's record requested ahead 46.
+constexpr int HOT_ANY = -2, HOT_ALIGN_NONE = -1;
+
+template <int SHAPE, bool ENERGY, int PAIR = HOT_ANY, int ALIGN = HOT_ANY>
+__global__ void __launch_bounds__(BLOCK, PAIR == HOT_ANY ? 4 : 6)
+k_hot_step(const __grid_constant__ Program P, const Replica* __restrict__ reps, const int* __restrict__ blk_rep,
            const Clock* __restrict__ clk, const D4* __restrict__ Gin, D4* __restrict__ Gout,
            const D4* __restrict__ Hin, D4* __restrict__ Hout, Dyn d, Stat st, NbList nl,
            int* __restrict__ rebuild, int* __restrict__ status, double dt_global, int apply_e1, int last,
            double* epart, int nblocks) {
+  constexpr bool ONE = PAIR != HOT_ANY;
   const int r = my_replica(blk_rep);
   if (clk[r].halt) return;  // batched stepping: a rebuild is pending
   const Replica& R = reps[r];
@@ -218,32 +227,43 @@ k_hot_step(Program P, const Replica* __restrict__ reps, const int* __restrict__ 
       }
     }
     p.id = st.id[k];
-    p.type = P.ntypes > 1 ? st.type[k] : 1;
+    p.type = !ONE && P.ntypes > 1 ? st.type[k] : 1;
     p.fx = 0.0; p.fy = 0.0; p.fz = 0.0; p.tx = 0.0; p.ty = 0.0; p.tz = 0.0;
     p.vx = 0.0; p.vy = 0.0; p.vz = 0.0;
 
     // ---- forces and torques (pair c and aligner c share sweep c) ----------
     const int cnt = nl.cnt[k], lo = nl.lo[k];
-    const int nloops = P.npair > P.nalign ? P.npair : P.nalign;
+    const int nloops = ONE ? 1 : P.npair > P.nalign ? P.npair : P.nalign;
     bool need_r = false;
-    for (int c = 0; c < P.npair; c++) need_r = need_r || P.pair[c].use_radii;
+    for (int c = 0; c < (ONE ? 1 : P.npair); c++) need_r = need_r || P.pair[c].use_radii;
     Part me;  // view for pair_term
     me.r = p.r; me.type = p.type;
     for (int c = 0; c < nloops; c++) {
-      const bool hp = c < P.npair, ha = c < P.nalign;
-      const PairComp pc = P.pair[hp ? c : 0];
-      const int akind = ha ? P.align[c].kind : -1;
+      const bool hp = ONE || c < P.npair, ha = ONE ? ALIGN != HOT_ALIGN_NONE : c < P.nalign;
+      PairComp pc = P.pair[hp ? c : 0];
+      if (ONE) pc.kind = PAIR;
+      const int akind = ONE ? ALIGN : ha ? P.align[c].kind : -1;
       const bool app = ha && P.align[c].has_pp;
       double Jg = ha ? R.align_J[c] : 0.0;
       if (akind == ALIGN_NEMATIC) Jg = 2.0 * Jg;
       const double rcg = ha ? R.align_rcut[c] : 0.0;
       const double* g = R.pair_g[hp ? c : 0];
-#pragma unroll 2
+      // the next neighbour's record requested before this one is used
+      int jn = 0 < cnt ? __ldg(nl.nb + k) : k;
+      int jnn = 1 < cnt ? __ldg(nl.nb + (size_t)nl.stride + k) : k;
+      D4 gn = ldg4(Gin + jn), hn{0.0, 0.0, 0.0, 0.0};
+      if (SHAPE != HOT_PLANE && ha) hn = ldg4(Hin + jn);
       for (int q = 0; q < cnt; q++) {
-        const int j = __ldg(nl.nb + (size_t)q * nl.stride + k);
+        const int j = jn;
+        const D4 gj = gn, hj = hn;
+        if (q + 1 < cnt) {
+          jn = jnn;
+          gn = ldg4(Gin + jn);
+          if (SHAPE != HOT_PLANE && ha) hn = ldg4(Hin + jn);
+          jnn = q + 2 < cnt ? __ldg(nl.nb + (size_t)(q + 2) * nl.stride + k) : k;
+        }
         Nb o;
         double dx, dy, dz;
-        const D4 gj = ldg4(Gin + j);
         if (SHAPE == HOT_PLANE) {
           o.x = gj.x; o.y = gj.y; o.nx = gj.z; o.ny = gj.w; o.nz = 0.0;
           o.r = need_r ? __ldg(st.r + j) : 1.0;
@@ -252,16 +272,16 @@ k_hot_step(Program P, const Replica* __restrict__ reps, const int* __restrict__ 
           if (dy > R.yhi) dy -= R.Ly; else if (dy < R.ylo) dy += R.Ly;
         } else {
           o.x = gj.x; o.y = gj.y; o.z = gj.z; o.r = gj.w;
-          if (ha) { const D4 hj = ldg4(Hin + j); o.nx = hj.x; o.ny = hj.y; o.nz = hj.z; }
+          if (ha) { o.nx = hj.x; o.ny = hj.y; o.nz = hj.z; }
           dx = o.x - p.x; dy = o.y - p.y; dz = o.z - p.z;
           apply_periodic(R, dx, dy, dz);
         }
-        o.type = (P.ntypes > 1) ? __ldg(st.type + j) : 1;
+        o.type = !ONE && P.ntypes > 1 ? __ldg(st.type + j) : 1;
         const double r_sq = (SHAPE == HOT_PLANE) ? dx * dx + dy * dy : dx * dx + dy * dy + dz * dz;
         const bool upper = q >= lo;
         if (hp) {
           double ff, pe;
-          if (pair_term(pc, g, P.ntypes, me, o, r_sq, 1.0, ff, pe)) {
+          if (pair_term(pc, g, ONE ? 1 : P.ntypes, me, o, r_sq, 1.0, ff, pe)) {
             p.fx -= ff * dx; p.fy -= ff * dy;
             if (SHAPE != HOT_PLANE) p.fz -= ff * dz;
             if (ENERGY && upper) e[c] += pe;
@@ -315,8 +335,9 @@ k_hot_step(Program P, const Replica* __restrict__ reps, const int* __restrict__ 
     int dix = 0, diy = 0;
     bool aged = false, vset = false, wset = false;
     double age = 0.0;
-    for (int c = 0; c < P.ninteg; c++) {
-      const IntegComp ic = P.integ[c];
+    for (int c = 0; c < (ONE ? 1 : P.ninteg); c++) {
+      IntegComp ic = P.integ[c];
+      if (ONE) ic.kind = INT_BROWNIAN;
       const double* ip = R.integ_p[c];
       const uint32_t seed = R.seed[c];
       uint64_t base = clk[r].ctr[c];
