@@ -449,7 +449,8 @@ __device__ __forceinline__ void cylinder_enforce(const Replica& R, double rc, Pa
 // ConstraintGaussianBump (A exp(-x^2/a - y^2/b) - z, constraint_gaussian_bump.cpp:58-75).
 // a0 is the replica's first shape parameter (torus c, ellipsoid a, peanut a,
 // hourglass R, bump A), C.b2 / C.b3 the second and third.
-__host__ __device__ __forceinline__ void implicit_gradient(const ConsComp& C, const Replica& R, double a0, double x,
+template <class CC>
+__host__ __device__ __forceinline__ void implicit_gradient(const CC& C, const Replica& R, double a0, double x,
                                                            double y, double z, double& gx, double& gy, double& gz) {
   if (C.kind == CONS_TORUS) {
     double sqr_xy = sqrt(x * x + y * y);
@@ -494,7 +495,8 @@ __host__ __device__ __forceinline__ void implicit_gradient(const ConsComp& C, co
     gz = -1.0;
   }
 }
-__host__ __device__ __forceinline__ double implicit_value(const ConsComp& C, const Replica& R, double a0, double x,
+template <class CC>
+__host__ __device__ __forceinline__ double implicit_value(const CC& C, const Replica& R, double a0, double x,
                                                           double y, double z) {
   if (C.kind == CONS_TORUS) {
     double ft = a0 - sqrt(x * x + y * y);
@@ -530,7 +532,8 @@ __host__ __device__ __forceinline__ double implicit_value(const ConsComp& C, con
 
 // compute_normal of the curved surfaces (sphere x/R; cylinder x/r, y/r, 0,
 // constraint_cylinder.hpp:76-80; implicit: the normalised gradient)
-__host__ __device__ __forceinline__ void surface_normal(const ConsComp& C, const Replica& R, double a0, const Part& p,
+template <class CC>
+__host__ __device__ __forceinline__ void surface_normal(const CC& C, const Replica& R, double a0, const Part& p,
                                                         double& Nx, double& Ny, double& Nz) {
   if (C.kind == CONS_SPHERE) { Nx = p.x / a0; Ny = p.y / a0; Nz = p.z / a0; }
   else if (C.kind == CONS_CYLINDER) { Nx = p.x / a0; Ny = p.y / a0; Nz = 0.0; }
@@ -564,7 +567,8 @@ __device__ __forceinline__ void plane_walls_enforce(const Replica& R, double l, 
 
 // Constraint::enforce, constraints/constraint.cpp:40-87 (SHAKE along the
 // gradient at the start point, then the tangent projections)
-__device__ __forceinline__ void implicit_enforce(const ConsComp& C, const Replica& R, double a0, Part& p) {
+template <class CC>
+__device__ __forceinline__ void implicit_enforce(const CC& C, const Replica& R, double a0, Part& p) {
   double ref_gx, ref_gy, ref_gz;
   implicit_gradient(C, R, a0, p.x, p.y, p.z, ref_gx, ref_gy, ref_gz);
   int iter = 0;
@@ -592,7 +596,8 @@ __device__ __forceinline__ void implicit_enforce(const ConsComp& C, const Replic
 
 // Constrainer::enforce (constrainer.hpp:73-77); ConstraintNone::enforce
 // (constraint_none.hpp:58-62)
-__device__ __forceinline__ void enforce_all(const Program& P, const Replica& R, Part& p) {
+template <class PT>
+__device__ __forceinline__ void enforce_all(const PT& P, const Replica& R, Part& p) {
   for (int c = 0; c < P.ncons; c++) {
     int kind = P.cons[c].kind;
     if (kind == CONS_PLANE) plane_enforce(R, R.cons_p[c], P.cons[c].unlimited, p);
@@ -609,7 +614,8 @@ __device__ __forceinline__ void enforce_all(const Program& P, const Replica& R, 
 // Constraint::project_torque (constraint.cpp:158-173, sphere normal
 // constraint_sphere.hpp:76) and ConstraintPlane::project_torque
 // (constraint_plane.cpp:150-162)
-__device__ __forceinline__ double project_torque(const Program& P, const Replica& R, const Part& p) {
+template <class PT>
+__device__ __forceinline__ double project_torque(const PT& P, const Replica& R, const Part& p) {
   double val = 0.0;
   for (int c = 0; c < P.ncons; c++) {
     int kind = P.cons[c].kind;
@@ -626,7 +632,8 @@ __device__ __forceinline__ double project_torque(const Program& P, const Replica
 
 // Constraint::rotate_director (Rodrigues, constraint.cpp:96-119) and
 // ConstraintPlane::rotate_director (constraint_plane.cpp:97-114)
-__device__ __forceinline__ void rotate_director(const Program& P, const Replica& R, Part& p, double phi) {
+template <class PT>
+__device__ __forceinline__ void rotate_director(const PT& P, const Replica& R, Part& p, double phi) {
   for (int c = 0; c < P.ncons; c++) {
     int kind = P.cons[c].kind;
     if (kind == CONS_PLANE || kind == CONS_PLANE_WALLS) {
@@ -650,7 +657,8 @@ __device__ __forceinline__ void rotate_director(const Program& P, const Replica&
 
 // Constraint::rotate_velocity (constraint.cpp:128-150) and the plane
 // variant (constraint_plane.cpp:122-143)
-__device__ __forceinline__ void rotate_velocity(const Program& P, const Replica& R, Part& p, double phi) {
+template <class PT>
+__device__ __forceinline__ void rotate_velocity(const PT& P, const Replica& R, Part& p, double phi) {
   for (int c = 0; c < P.ncons; c++) {
     int kind = P.cons[c].kind;
     if (kind == CONS_PLANE || kind == CONS_PLANE_WALLS) {
@@ -680,7 +688,8 @@ __device__ __forceinline__ void rotate_velocity(const Program& P, const Replica&
 // ---------------------------------------------------------------------------
 struct Nb { double x, y, z, r, nx, ny, nz, vx, vy, vz, age; int type; };
 
-__device__ __forceinline__ double phase_factor(const PairComp& C, double age, double dt) {
+template <class QC>
+__device__ __forceinline__ double phase_factor(const QC& C, double age, double dt) {
   return 0.5 * (1.0 + value_get(C.phase, (int)(age / dt)));
 }
 __device__ __forceinline__ double phase_pair(double ai, double aj) {
@@ -692,7 +701,8 @@ __device__ __forceinline__ double phase_pair(double ai, double aj) {
 // soft: pair_soft_potential.cpp:57-117; lj: pair_lj_potential.cpp:54-122;
 // morse: pair_morse_potential.cpp:52-120; gaussian:
 // pair_gaussian_potential.cpp:55-126.
-__device__ __forceinline__ bool pair_term(const PairComp& C, const double* g, int ntypes,
+template <class QC>
+__device__ __forceinline__ bool pair_term(const QC& C, const double* g, int ntypes,
                                           const Part& me, const Nb& o, double r_sq,
                                           double alpha, double& ff, double& pe) {
   const double* t = C.table + ((size_t)(me.type - 1) * ntypes + (size_t)(o.type - 1)) * PAIR_NPARAM;

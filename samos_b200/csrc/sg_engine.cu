@@ -4,6 +4,7 @@
 #include "samos_gpu.h"
 #include "sg_abp_launch.h"
 #include "sg_hot_launch.h"
+#include "sg_generic_launch.h"
 #include "sg_flow.cuh"
 
 #include <algorithm>
@@ -1638,22 +1639,15 @@ static int step_unfused(sg_system* s, bool energy, bool driver) {
 static constexpr int kGenMinb[2] = {8, 6};
 static constexpr int kGenTuneReps = 3;  // timed steps per candidate (after one untimed)
 
-extern "C++" {
-template <bool ENERGY>
-static void launch_generic(sg_system* s, int minb, bool apply_e1) {
-  const int nb = s->nblocks;
-  if (minb == 6)
-    k_step_brownian<ENERGY, 6><<<nb, BLOCK, 0, s->stream>>>(s->prog, s->reps, s->blk_rep, s->clk, s->cur, s->alt,
-                                                            s->st, s->nl, s->rebuild, s->status, s->dt_global,
-                                                            apply_e1 ? 1 : 0, s->epart, nb, s->gmask, s->grank,
-                                                            s->slots);
-  else
-    k_step_brownian<ENERGY, 8><<<nb, BLOCK, 0, s->stream>>>(s->prog, s->reps, s->blk_rep, s->clk, s->cur, s->alt,
-                                                            s->st, s->nl, s->rebuild, s->status, s->dt_global,
-                                                            apply_e1 ? 1 : 0, s->epart, nb, s->gmask, s->grank,
-                                                            s->slots);
+static void launch_generic(sg_system* s, int minb, bool apply_e1, bool energy) {
+  GenericLaunch L{};
+  L.prog = &s->prog; L.reps = s->reps; L.blk_rep = s->blk_rep; L.clk = s->clk;
+  L.cur = s->cur; L.alt = s->alt; L.st = s->st; L.nl = s->nl; L.rebuild = s->rebuild; L.status = s->status;
+  L.dt_global = s->dt_global; L.apply_e1 = apply_e1 ? 1 : 0; L.energy = energy;
+  L.epart = s->epart; L.nblocks = s->nblocks; L.slots = s->slots; L.gmask = s->gmask; L.grank = s->grank;
+  L.minb = minb; L.stream = s->stream;
+  launch_generic_step(L);
 }
-}  // extern "C++"
 
 // One generic fused step.  `may_tune`: a step launched on its own (not in a
 // batch, whose halted kernels would time as empty), which may serve as one
@@ -1668,8 +1662,7 @@ static int step_fused(sg_system* s, bool apply_e1, bool energy, bool may_tune = 
   }
   const int minb = s->gen_pin ? s->gen_pin : s->gen_minb;
   if (s->profile) CU(s, cudaEventRecord(s->ev_k0, s->stream));
-  if (energy) launch_generic<true>(s, minb, apply_e1);
-  else launch_generic<false>(s, minb, apply_e1);
+  launch_generic(s, minb, apply_e1, energy);
   LAUNCH_CHECK(s);
   if (s->profile) CU(s, cudaEventRecord(s->ev_k1, s->stream));
   std::swap(s->cur, s->alt);

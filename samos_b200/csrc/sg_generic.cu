@@ -1,0 +1,44 @@
+// sg_generic.cu -- launches of the generic fused step (k_step_brownian): the
+// Vicsek model on a plane and soft + polar `brownian` particles on a curved
+// surface with their kinds fixed, every other program through the loops.
+#include "sg_generic_launch.h"
+
+namespace sg {
+
+template <bool ENERGY, int MINB, int CONS, int PAIR, int ALIGN, int INTEG>
+static void launch(const GenericLaunch& L) {
+  k_step_brownian<ENERGY, MINB, CONS, PAIR, ALIGN, INTEG><<<L.nblocks, BLOCK, 0, L.stream>>>(
+      *L.prog, L.reps, L.blk_rep, L.clk, L.cur, L.alt, L.st, L.nl, L.rebuild, L.status, L.dt_global, L.apply_e1, L.epart,
+      L.nblocks, L.gmask, L.grank, L.slots);
+}
+
+template <int MINB>
+static bool launch_fixed(const GenericLaunch& L) {
+  const Program& P = *L.prog;
+  if (P.ntypes != 1 || P.npair != 1 || P.pair[0].kind != PAIR_SOFT || P.pair[0].phase_in || P.nalign != 1 ||
+      P.align[0].has_pp || P.next || P.ncons != 1 || P.ninteg != 1 || P.integ[0].group)
+    return false;
+  const int cons = P.cons[0].kind, align = P.align[0].kind, integ = P.integ[0].kind;
+#define GEN_MIX(C, A, I) \
+  if (cons == C && align == A && integ == I) return launch<false, MINB, C, PAIR_SOFT, A, I>(L), true;
+  GEN_MIX(CONS_PLANE, ALIGN_VICSEK, INT_VICSEK)
+  GEN_MIX(CONS_CYLINDER, ALIGN_POLAR, INT_BROWNIAN)
+  GEN_MIX(CONS_TORUS, ALIGN_POLAR, INT_BROWNIAN)
+  GEN_MIX(CONS_ELLIPSOID, ALIGN_POLAR, INT_BROWNIAN)
+  GEN_MIX(CONS_PEANUT, ALIGN_POLAR, INT_BROWNIAN)
+  GEN_MIX(CONS_HOURGLASS, ALIGN_POLAR, INT_BROWNIAN)
+  GEN_MIX(CONS_GAUSSIAN_BUMP, ALIGN_POLAR, INT_BROWNIAN)
+#undef GEN_MIX
+  return false;
+}
+
+void launch_generic_step(const GenericLaunch& L) {
+  if (L.energy) {
+    if (L.minb == 6) launch<true, 6, GEN_ANY, GEN_ANY, GEN_ANY, GEN_ANY>(L);
+    else launch<true, 8, GEN_ANY, GEN_ANY, GEN_ANY, GEN_ANY>(L);
+  } else if (L.minb == 6) {
+    if (!launch_fixed<6>(L)) launch<false, 6, GEN_ANY, GEN_ANY, GEN_ANY, GEN_ANY>(L);
+  } else if (!launch_fixed<8>(L)) launch<false, 8, GEN_ANY, GEN_ANY, GEN_ANY, GEN_ANY>(L);
+}
+
+}  // namespace sg

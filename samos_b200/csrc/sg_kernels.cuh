@@ -33,7 +33,8 @@ __device__ __forceinline__ void fetch_nb(const Dyn& d, const Stat& st, int j, co
   if (nd.age) o.age = d.age[j];
 }
 
-__device__ __forceinline__ Need program_needs(const Program& P) {
+template <class PT>
+__device__ __forceinline__ Need program_needs(const PT& P) {
   Need nd{false, P.ntypes > 1, false, false, false};
   for (int c = 0; c < P.npair; c++) {
     if (P.pair[c].use_radii) nd.r = true;
@@ -52,8 +53,11 @@ __device__ __forceinline__ Need program_needs(const Program& P) {
 // separate accumulators, so sharing the neighbour sweep keeps each one's
 // summation order.  Pair energies are counted once, on the lower id.
 // ---------------------------------------------------------------------------
-template <bool ENERGY>
-__device__ void compute_ft(const Program& P, const Replica& R, const Dyn& d, const Stat& st,
+// AHEAD: the next neighbour's fields are requested before this one's are used
+// (programs with their kinds fixed; with every field a neighbour may have, the
+// registers would not hold two).
+template <bool ENERGY, bool AHEAD = false, class PT = Program>
+__device__ __forceinline__ void compute_ft(const PT& P, const Replica& R, const Dyn& d, const Stat& st,
                            const NbList& nl, int k, Part& me, double dt, bool with_pair,
                            bool with_align, double* epair, double* ealign) {
   me.fx = 0.0; me.fy = 0.0; me.fz = 0.0;
@@ -65,7 +69,7 @@ __device__ void compute_ft(const Program& P, const Replica& R, const Dyn& d, con
   const int nloops = npair > nalign ? npair : nalign;
   for (int c = 0; c < nloops; c++) {
     const bool hp = c < npair, ha = c < nalign;
-    PairComp pc; AlignComp ac;
+    auto pc = P.pair[0]; auto ac = P.align[0];
     double a_i = 1.0, Jg = 0.0, rcg = 0.0;
     int akind = -1;
     if (hp) { pc = P.pair[c]; if (pc.phase_in) a_i = phase_factor(pc, me.age, dt); }
@@ -75,10 +79,21 @@ __device__ void compute_ft(const Program& P, const Replica& R, const Dyn& d, con
       if (akind == ALIGN_NEMATIC) Jg = 2.0 * Jg;  // pair_nematic_aligner.cpp:37
     }
     const double* g = R.pair_g[hp ? c : 0];
+    Nb next;
+    int jn = 0;
+    if (AHEAD && cnt > 0) {
+      fetch_nb(d, st, nl.nb[k], nd, next);
+      if (cnt > 1) jn = nl.nb[(size_t)nl.stride + k];
+    }
     for (int q = 0; q < cnt; q++) {
-      const int j = nl.nb[(size_t)q * nl.stride + k];
       Nb o;
-      fetch_nb(d, st, j, nd, o);
+      if (AHEAD) {
+        o = next;
+        if (q + 1 < cnt) {
+          fetch_nb(d, st, jn, nd, next);
+          if (q + 2 < cnt) jn = nl.nb[(size_t)(q + 2) * nl.stride + k];
+        }
+      } else fetch_nb(d, st, nl.nb[(size_t)q * nl.stride + k], nd, o);
       double dx = o.x - me.x, dy = o.y - me.y, dz = o.z - me.z;
       apply_periodic(R, dx, dy, dz);
       const double r_sq = dx * dx + dy * dy + dz * dz;
@@ -161,7 +176,8 @@ __device__ __forceinline__ void block_reduce_store(double (&v)[NV], double* out,
 // ---------------------------------------------------------------------------
 
 // IntegratorBrownian::integrate, integrators/integrator_brownian.cpp:42-124
-__device__ __forceinline__ void integ_brownian(const Program& P, const Replica& R, const IntegComp& ic,
+template <class PT, class IC>
+__device__ __forceinline__ void integ_brownian(const PT& P, const Replica& R, const IC& ic,
                                                const double* ip, uint32_t seed, uint64_t base,
                                                int run_step, int n, uint64_t g, Part& p) {
   const double dt = ip[0], v0 = ip[1], nu = ip[2], mu = ip[3], mur = ip[4];
@@ -200,7 +216,8 @@ __device__ __forceinline__ void integ_brownian(const Program& P, const Replica& 
 }
 
 // IntegratorBrownianPos::integrate, integrators/integrator_brownian_pos.cpp:37-84
-__device__ __forceinline__ void integ_brownian_pos(const Program& P, const Replica& R, const IntegComp& ic,
+template <class PT, class IC>
+__device__ __forceinline__ void integ_brownian_pos(const PT& P, const Replica& R, const IC& ic,
                                                    const double* ip, uint32_t seed, uint64_t base,
                                                    int run_step, uint64_t g, Part& p) {
   const double dt = ip[0], mu = ip[3];
@@ -222,7 +239,8 @@ __device__ __forceinline__ void integ_brownian_pos(const Program& P, const Repli
 }
 
 // IntegratorBrownianAlign::integrate, integrators/integrator_brownian_align.cpp:41-76
-__device__ __forceinline__ void integ_brownian_align(const Program& P, const Replica& R, const IntegComp& ic,
+template <class PT, class IC>
+__device__ __forceinline__ void integ_brownian_align(const PT& P, const Replica& R, const IC& ic,
                                                      const double* ip, uint32_t seed, uint64_t base,
                                                      int n, uint64_t g, Part& p) {
   const double dt = ip[0], nu = ip[2], mur = ip[4];
@@ -241,7 +259,8 @@ __device__ __forceinline__ void integ_brownian_align(const Program& P, const Rep
 // velocity follows the (normalised) Vicsek torque vector, v0 tau + mu F, and
 // is turned by a uniform angle of width eta sqrt(dt); one uniform draw per
 // particle.
-__device__ __forceinline__ void integ_vicsek(const Program& P, const Replica& R, const double* ip, uint32_t seed,
+template <class PT>
+__device__ __forceinline__ void integ_vicsek(const PT& P, const Replica& R, const double* ip, uint32_t seed,
                                              uint64_t base, uint64_t g, Part& p) {
   const double dt = ip[0], v0 = ip[1], eta = ip[2], mu = ip[3];
   const double noise = eta * sqrt(dt);
@@ -342,15 +361,54 @@ __global__ void k_force(Program P, const Replica* __restrict__ reps, const int* 
 // MINB: blocks per SM the register allocation is bounded for (8: 64
 // registers with some spills, 6: 80); the engine times both on a run's first
 // steps and keeps the faster, since which one wins depends on the program.
-template <bool ENERGY, int MINB>
+// CONS / PAIR / ALIGN / INTEG: GEN_ANY, any program; otherwise one component of
+// each, one particle type, no groups and no external potential, the kinds known
+// at compile time, so that no branch over the other kinds and none of their
+// registers are left (GEN_MIX, sg_generic.cu).
+constexpr int GEN_ANY = -2;
+
+// A Program whose counts and kinds are constants of the type.
+template <int CONS, int PAIR, int ALIGN, int INTEG>
+struct FixedProgram {
+  struct Pair {
+    static constexpr int kind = PAIR, phase_in = 0;
+    int use_radii, shifted, has_pp;
+    Value phase;
+    const double* table;
+  };
+  struct Align { static constexpr int kind = ALIGN, has_pp = 0; const double* table; };
+  struct Ext { static constexpr int has_params = 0; const double* type_alpha; };
+  struct Cons { static constexpr int kind = CONS; int unlimited, max_iter; double b2, b3, tol; };
+  struct Integ { static constexpr int kind = INTEG, group = 0; int nematic, velocity; Value temp; };
+  static constexpr int ntypes = 1, npair = 1, nalign = 1, next = 0, ncons = 1, ninteg = 1;
+  Pair pair[1];
+  Align align[1];
+  Ext ext[1];
+  Cons cons[1];
+  Integ integ[1];
+  __device__ __forceinline__ explicit FixedProgram(const Program& P)
+      : pair{{P.pair[0].use_radii, P.pair[0].shifted, P.pair[0].has_pp, P.pair[0].phase, P.pair[0].table}},
+        align{{P.align[0].table}}, ext{{nullptr}},
+        cons{{P.cons[0].unlimited, P.cons[0].max_iter, P.cons[0].b2, P.cons[0].b3, P.cons[0].tol}},
+        integ{{P.integ[0].nematic, P.integ[0].velocity, P.integ[0].temp}} {}
+};
+template <int CONS, int PAIR, int ALIGN, int INTEG>
+__device__ __forceinline__ decltype(auto) program_of(const Program& P) {
+  if constexpr (CONS == GEN_ANY) return (P);
+  else return FixedProgram<CONS, PAIR, ALIGN, INTEG>(P);
+}
+
+template <bool ENERGY, int MINB, int CONS = GEN_ANY, int PAIR = GEN_ANY, int ALIGN = GEN_ANY, int INTEG = GEN_ANY>
 __global__ void __launch_bounds__(BLOCK, MINB)
-k_step_brownian(Program P, const Replica* __restrict__ reps, const int* __restrict__ blk_rep,
+k_step_brownian(const __grid_constant__ Program P0, const Replica* __restrict__ reps, const int* __restrict__ blk_rep,
                 const Clock* __restrict__ clk, Dyn cur, Dyn nxt, Stat st, NbList nl,
                 int* __restrict__ rebuild, int* __restrict__ status, double dt_global, int apply_e1,
                 double* epart, int nblocks, const uint8_t* __restrict__ gmask, const int* __restrict__ grank,
                 int slots) {
   const int r = my_replica(blk_rep);
   if (clk[r].halt) return;  // batched stepping: a rebuild is pending, this step does not run
+  constexpr bool FIXED = CONS != GEN_ANY;
+  const auto& P = program_of<CONS, PAIR, ALIGN, INTEG>(P0);
   const Replica& R = reps[r];
   const int k = blockIdx.x * BLOCK + threadIdx.x;
   double e[MAX_PAIR + MAX_ALIGN];
@@ -360,10 +418,10 @@ k_step_brownian(Program P, const Replica* __restrict__ reps, const int* __restri
     Part p;
     load_dyn(cur, k, p);
     p.id = st.id[k]; p.type = st.type[k]; p.r = st.r[k]; p.mass = st.mass[k];
-    compute_ft<ENERGY>(P, R, cur, st, nl, k, p, dt_global, true, true, e, e + MAX_PAIR);
+    compute_ft<ENERGY, FIXED>(P, R, cur, st, nl, k, p, dt_global, true, true, e, e + MAX_PAIR);
     const int run_step = clk[r].run_step;
     for (int c = 0; c < P.ninteg; c++) {
-      const IntegComp ic = P.integ[c];
+      const auto ic = P.integ[c];
       const uint64_t base = clk[r].ctr[c];
       // a grouped integrator moves its members only, drawing in group order
       // (IntegratorBrownian::integrate loops over the group's particles)
