@@ -1,0 +1,249 @@
+"""Runs whose steps and list rebuilds are enqueued together (resident runs, the
+two-launch Langevin / NVE / FIRE steps, the packed and generic kernels with
+their kinds fixed) against the same runs one step at a time with host-driven
+rebuilds and the general kernels (profiling mode): every field, exactly."""
+import numpy as np
+import pytest
+
+from samos_b200 import Engine, engine
+from samos_b200.ensemble import SphereReplica, plane_fire_ensemble, quench_disks, sphere_ensemble
+from scenarios import drive, plane_disks, sphere_disks, surface_disks
+
+pytestmark = pytest.mark.gpu
+
+FIELDS = ("x", "y", "z", "vx", "vy", "vz", "nx", "ny", "nz", "fx", "fy", "fz", "tau_x", "tau_y", "tau_z", "omega", "age",
+          "ix", "iy")
+SOFT = ("soft", {"k": "10", "use_particle_radii": ""})
+LJ = ("lj", {"epsilon": "1", "sigma": "1", "rcut": "2.5", "shifted": ""})
+MORSE = ("morse", {"D": "1", "a": "2", "re": "2", "rcut": "2.5", "shifted": ""})
+GAUSS = ("gaussian", {"A": "2", "B": "-1", "alpha": "1", "beta": "3", "rA": "0", "rB": "1.5", "rcut": "2.5"})
+
+
+def abp(**kw):
+    return [("brownian", dict({"v0": "8", "nu": "0.5", "mu": "1", "mur": "1", "seed": "4"}, **kw))]
+
+
+def both(make, steps, prepare=lambda e: None):
+    """The engines of the enqueued and the stepwise run."""
+    out = []
+    for stepwise in (False, True):
+        e = make()
+        prepare(e)
+        e.set_profiling(stepwise)
+        st = [e.run(s) for s in steps]
+        out.append((e, sum(s.nlist_builds for s in st)))
+    return out
+
+
+def same(runs, fields=FIELDS):
+    (a, builds), (b, want) = runs
+    assert builds == want
+    for r in range(len(a.n)):
+        for f in fields:
+            np.testing.assert_array_equal(a.download(f, replica=r), b.download(f, replica=r), err_msg=f"{f} replica {r}")
+        assert a.energy(0, 0, r) == b.energy(0, 0, r)
+    a.close()
+    b.close()
+    return builds
+
+
+def lattice(n, seed, phi=0.6):
+    """Unit disks on a jittered square lattice in a periodic box."""
+    rng = np.random.default_rng(seed)
+    m, a = int(np.ceil(np.sqrt(n))), float(np.sqrt(np.pi / phi))
+    L, k, th = max(m * a, 8.0), np.arange(n), rng.uniform(0, 2 * np.pi, n)
+    z = np.zeros(n)
+    return dict(x=-L / 2 + (k % m + 0.5) * a + rng.uniform(-0.1, 0.1, n),
+                y=-L / 2 + (k // m + 0.5) * a + rng.uniform(-0.1, 0.1, n), z=z, vx=rng.normal(0, 1, n),
+                vy=rng.normal(0, 1, n), vz=z, nx=np.cos(th), ny=np.sin(th), nz=z, radius=np.ones(n),
+                mass=rng.uniform(0.5, 2.0, n)), L
+
+
+# the block edges, and the largest system that a resident run still takes (592 blocks)
+@pytest.mark.parametrize("n", [1, 127, 128, 129, 3000, 592 * 128])
+@pytest.mark.parametrize("align,extra", [("polar", {}), ("nematic", {"nematic": "", "tau": "0.5"}),
+                                         (None, {"min_val": "0.3"})])
+def test_resident_plane_run(n, align, extra):
+    parts, L = plane_disks(n, 0.6, seed=n)
+    L = max(L, 9.0)
+
+    def make():
+        e = Engine(n)
+        drive(e, parts, (L, L, 10.0), nlist=(2.4, 0.3), pairs=[SOFT], aligns=[(align, {"J": "1.0"})] if align else [],
+              externals=[("self_propulsion", {"alpha": "0.5"})] if align is None else [], dt=1e-3,
+              integrators=abp(**extra)).commit()
+        return e
+
+    steps = (149, 60, 1)  # the tuner's steps first
+    assert same(both(make, steps)) >= (1 if n > 1000 else 0)
+
+
+@pytest.mark.parametrize("sizes", [(65,), (500, 64, 1291)])
+def test_resident_sphere_run(sizes):
+    def make():
+        reps = []
+        for i, n in enumerate(sizes):
+            parts, R = sphere_disks(n, seed=50 + i)
+            reps.append(SphereReplica(parts=parts, R=R, v0=5.0 + i, J=0.3 * i, nu=0.2, seed=7 + i))
+        return sphere_ensemble(reps)
+
+    assert same(both(make, (149, 90))) >= 1
+
+
+@pytest.mark.parametrize("n", [60, 1500, 592 * 128 + 1])
+@pytest.mark.parametrize("method", ["baoab", "bbk"])
+def test_langevin_two_launch_and_resident(n, method):
+    parts, L = lattice(n, 3)
+
+    def make():
+        e = Engine(n)
+        drive(e, parts, (L, L, 10.0), nlist=(2.8, 0.3), pairs=[LJ], aligns=[("polar", {"J": "0.2"})], dt=2e-3,
+              integrators=[("langevin", {"gamma": "1", "seed": "7", "method": method, "min_val": "0.5"})]).commit()
+        return e
+
+    assert same(both(make, (160, 40))) >= 1
+
+
+@pytest.mark.parametrize("pair,align,params,sizes", [
+    (SOFT, "polar", {"limit": "0.01", "angle_limit": "0.02"}, (1500,)), (SOFT, "nematic", {"limit": "0.05"}, (129,)),
+    (LJ, None, {"limit": "0.02"}, (1500,)), (MORSE, "polar", {"limit": "0.02"}, (700,)),
+    (SOFT, None, {"limit": "0.02"}, (300, 900))])
+def test_nve_two_launch_and_resident(pair, align, params, sizes):
+    def make():
+        systems = [lattice(n, 9 + n) for n in sizes]
+        e = Engine(list(sizes))
+        for r, (parts, L) in enumerate(systems):
+            e.set_box(L, L, 10.0, True, replica=r)
+            for f, v in parts.items():
+                e.upload(f, v, replica=r)
+        from samos_b200 import Simulation
+        sim = Simulation(e)
+        sim.nlist(2.8, 0.3)
+        sim.constraint("plane", {})
+        sim.pair_potential(*pair)
+        if align:
+            sim.pair_align(align, {"J": "1"})
+        sim.timestep(5e-3)
+        sim.integrator("nve", dict(params))
+        sim.commit()
+        return e
+
+    assert same(both(make, (120, 45))) >= 1
+
+
+@pytest.mark.parametrize("sizes", [(200,), (300, 512, 900, 130)])
+@pytest.mark.parametrize("ordered", [False, True])
+def test_fire_minimiser_and_plain_run(sizes, ordered):
+    insts = [quench_disks(n, 0.87, 20 + n) for n in sizes]
+    runs = []
+    for stepwise in (False, True):
+        e = plane_fire_ensemble(insts, fmax=1e-6)
+        e.set_fire_order(ordered)
+        e.build_nlist()
+        e.set_profiling(stepwise)
+        conv, st = e.minimize(30000)
+        state = [e.fire_state(r) for r in range(len(sizes))]
+        e.run(40)
+        runs.append((e, conv, state))
+    (a, ca, sa), (b, cb, sb) = runs
+    np.testing.assert_array_equal(ca, cb)
+    assert (ca > 0).all()
+    np.testing.assert_array_equal(sa, sb)
+    same(((a, 0), (b, 0)))
+
+
+@pytest.mark.parametrize("pair", [LJ, MORSE, GAUSS])
+@pytest.mark.parametrize("align", [None, "polar", "nematic"])
+@pytest.mark.parametrize("shape", ["plane", "sphere"])
+def test_packed_step_with_its_kinds_fixed(pair, align, shape):
+    n = 900
+    if shape == "plane":
+        parts, L = lattice(n, 5)
+        box, periodic, cons = (L, L, 10.0), True, ("plane", {})
+    else:
+        parts, R = sphere_disks(n, R=24.0, seed=6)
+        box, periodic, cons = (60.0, 60.0, 60.0), False, ("sphere", {"r": repr(R)})
+    runs = []
+    for path in (0, 1):  # 1: the general kernels on the unpacked store
+        e = Engine(n)
+        drive(e, parts, box, periodic, nlist=(2.8, 0.3), constraint=cons, pairs=[pair],
+              aligns=[(align, {"J": "0.5"})] if align else [], dt=2e-5 if pair is LJ else 1e-3, integrators=abp()).commit()
+        e.set_path(path)
+        e.set_profiling(bool(path))
+        e.run(80)
+        runs.append(e)
+    for f in FIELDS:
+        np.testing.assert_array_equal(runs[0].download(f), runs[1].download(f), err_msg=f)
+
+
+@pytest.mark.parametrize("kind,shape", [("torus", dict(c=14.0, a=5.0)), ("cylinder", dict(r=8.0)),
+                                        ("ellipsoid", dict(a=16.0, b=14.0, c=12.0))])
+def test_curved_step_with_its_kinds_fixed(kind, shape):
+    # a second type that no particle has keeps the general kernel on the other side
+    n = 700
+    try:
+        parts = surface_disks(kind, n, seed=8, **shape)
+    except KeyError:
+        parts = surface_disks(kind, n, seed=8, Lz=40.0, **shape)
+    runs = []
+    for ntypes in (1, 2):
+        e = Engine(n, ntypes=ntypes)
+        drive(e, parts, (60.0, 60.0, 60.0), True, nlist=(2.4, 0.3), constraint=(kind, {k: repr(v) for k, v in shape.items()}),
+              pairs=[("soft", {"k": "10"})], aligns=[("polar", {"J": "0.2"})], dt=1e-3, integrators=abp(), ntypes=ntypes).commit()
+        e.run(60)
+        runs.append(e)
+    for f in FIELDS:
+        np.testing.assert_array_equal(runs[0].download(f), runs[1].download(f), err_msg=f)
+
+
+@pytest.mark.parametrize("integrator", ["brownian", "langevin"])
+def test_lists_that_outgrow_their_capacity_inside_a_run(integrator):
+    # spread out at the list build, then put into pairs of clumps that do not see
+    # the next pair: up to 44 neighbours where the first lists hold 32
+    n = 44 * 9
+    parts, L = lattice(n, 4, phi=0.05)
+    rng = np.random.default_rng(5)
+    centre = np.arange(n) // 44
+    crowd = dict(x=(centre % 3 - 1) * L / 3 + rng.uniform(-0.9, 0.9, n), y=(centre // 3 - 1) * L / 3 + rng.uniform(-0.9, 0.9, n))
+
+    def make():
+        e = Engine(n)
+        integ = abp() if integrator == "brownian" else [("langevin", {"gamma": "1", "seed": "7", "min_val": "0.1"})]
+        drive(e, parts, (L, L, 10.0), nlist=(2.4, 0.3), pairs=[("soft", {"k": "0.01", "a": "2.0"})],
+              aligns=[("polar", {"J": "0.1"})], dt=1e-3, integrators=integ).commit()
+        return e
+
+    assert same(both(make, (130, 30), prepare=lambda e: e.upload_fields(crowd))) >= 1
+
+
+@pytest.mark.parametrize("n", [1, 255, 257, 4099])
+@pytest.mark.parametrize("pinned", ["all", "some"])
+def test_multi_field_transfers_from_page_locked_arrays(n, pinned):
+    rng = np.random.default_rng(n)
+    parts, L = plane_disks(n, 0.5, seed=2)
+    e = Engine(n)
+    drive(e, parts, (max(L, 9.0),) * 2 + (10.0,), nlist=(2.4, 0.3), pairs=[SOFT], integrators=abp()).commit()
+    want = {f: rng.normal(size=n) for f in ("vx", "vy", "omega", "radius")}
+    want["ix"] = rng.integers(-5, 5, n).astype(np.int32)
+    send = {f: engine.pinned_copy(v, v.dtype) if pinned == "all" or i % 2 else v for i, (f, v) in enumerate(want.items())}
+    e.upload_fields(send)
+    out = {f: engine.pinned_empty(n, v.dtype) if pinned == "all" or i % 2 == 0 else np.empty_like(v)
+           for i, (f, v) in enumerate(want.items())}
+    got = e.download_fields(list(want), out=out)
+    for f in want:
+        np.testing.assert_array_equal(got[f], want[f], err_msg=f)
+        np.testing.assert_array_equal(e.download(f), want[f], err_msg=f)
+
+
+@pytest.mark.parametrize("crowd", [10, 30, 45])
+def test_static_forces_with_more_finds_than_the_fast_search_keeps(crowd):
+    from samos_b200 import engine as E
+    from test_zz_no_alloc import OUT_FIELDS, engine_forces, overflow_count, static_forces
+    parts, L = plane_disks(1500, 0.2, seed=41)
+    rng = np.random.default_rng(41)
+    parts["x"][:crowd], parts["y"][:crowd] = rng.uniform(-0.8, 0.8, crowd), rng.uniform(-0.8, 0.8, crowd)
+    want = engine_forces(parts, (L, L, 10.0), (2.4, 0.3), 10.0, "polar", 0.3)
+    got = static_forces(E.load(), parts, (L, L, 10.0), (2.4, 0.3), 10.0, E.ALIGN["polar"], 0.3)
+    assert overflow_count(E.load()) == 0
+    for f in OUT_FIELDS:
+        np.testing.assert_array_equal(got[f], want[f], err_msg=f)
