@@ -73,6 +73,7 @@ __device__ __forceinline__ f2_t f2_mul(f2_t a, f2_t b) {
   asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
   return d;
 }
+__device__ __forceinline__ float2 pair_at(const float* p, int i) { return make_float2(p[2 * i], p[2 * i + 1]); }
 __device__ __forceinline__ f2_t f2_relu(f2_t a) { return f2_pack(fmaxf(f2_lo(a), 0.f), fmaxf(f2_hi(a), 0.f)); }
 
 // one warp's slots and staged edges: features as packed pairs (e, e), the unit
@@ -97,7 +98,8 @@ __device__ __forceinline__ EdgeSlot edge_slot(const sg_view& V, const double* __
   EdgeSlot L{0, 0.0, 0.0, 0.0, 0.0, 0.f};
   const int i = i0 + lane;
   if (lane < EDGE_P && i < V.slots) {
-    const double2 b = reinterpret_cast<const double2*>(box)[i];
+    // the caller's arrays need no more than their element's alignment
+    const double2 b = make_double2(box[2 * i], box[2 * i + 1]);
     L.Lx = b.x; L.Ly = b.y;
     const int c = V.nb_cnt_device[i];
     L.x = V.x_device[i]; L.y = V.y_device[i];
@@ -690,8 +692,10 @@ k_ml_l2(sg_view V, const double* __restrict__ box, double rc, const float* __res
         }
       __syncwarp();
     }
-    if (lane < EDGE_P && i0 + lane < V.slots)
-      reinterpret_cast<float2*>(disp)[i0 + lane] = make_float2(dx, dy);
+    if (lane < EDGE_P && i0 + lane < V.slots) {
+      disp[2 * (i0 + lane)] = dx;
+      disp[2 * (i0 + lane) + 1] = dy;
+    }
   }
 }
 
@@ -722,8 +726,7 @@ k_ml_l2_bwd(sg_view V, const double* __restrict__ box, double rc, const float* _
   EdgeSlot next = edge_slot(V, box, i0, lane);
   for (; i0 < V.slots; i0 += step) {
     if (lane < EDGE_P && next.Lx > 0.0) {
-      const float2 d = reinterpret_cast<const float2*>(disp)[i0 + lane],
-                   t = reinterpret_cast<const float2*>(target)[i0 + lane];
+      const float2 d = pair_at(disp, i0 + lane), t = pair_at(target, i0 + lane);
       const float ex = d.x - t.x, ey = d.y - t.y;
       lsum += ex * ex + ey * ey;
       dsh[warp][lane] = make_float2(2.f * ex * inv_n, 2.f * ey * inv_n);
@@ -736,7 +739,7 @@ k_ml_l2_bwd(sg_view V, const double* __restrict__ box, double rc, const float* _
       const int n = stage_edges(V, i0, t0, total, rc, lane, S);
       for (int e = lane; e < n; e += 32) {
         const int j = S.j[e];
-        const float2 d = reinterpret_cast<const float2*>(disp)[j], t = reinterpret_cast<const float2*>(target)[j];
+        const float2 d = pair_at(disp, j), t = pair_at(target, j);
         const float2 gi = dsh[warp][S.p[e]], u = S.u[e];
         const float gw = gi.x * u.x + gi.y * u.y;
         // the vector from j to i is exactly the opposite

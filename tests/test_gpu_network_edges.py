@@ -66,3 +66,27 @@ def test_forward_and_gradient_match_the_reference_network(n, phi):
         size = int(np.prod(s))
         assert np.linalg.norm(got[o:o + size] - want[o:o + size]) < 2e-2 * max(np.linalg.norm(want[o:o + size]), 1e-12), name
     eng.close()
+
+
+def test_box_and_target_need_only_their_elements_alignment():
+    import torch
+
+    from samos_b200.ensemble import plane_fire_ensemble, quench_disks
+    from samos_b200.warmstart import WarmStartNet
+
+    insts = [quench_disks(150, 0.86, 35)]
+    eng = plane_fire_ensemble(insts)
+    eng.build_nlist()
+    net = WarmStartNet(seed=3)
+    box = net.box_array(eng, (0,))
+    tgt = net.slot_targets(eng, [np.random.default_rng(4).normal(0.0, 0.3, (150, 2))])
+    loss = net.loss_and_grad(eng, box, tgt, 150)
+    grad = net.grad.clone()
+
+    def shifted(t):
+        flat = t.reshape(-1)
+        return torch.cat((flat[:1], flat))[1:]
+
+    assert net.loss_and_grad(eng, shifted(box), shifted(tgt), 150) == loss
+    assert torch.equal(net.grad, grad)
+    eng.close()
