@@ -7,6 +7,8 @@
 #include "sg_generic_launch.h"
 #include "sg_flow.cuh"
 
+#include <cuda.h>
+
 #include <algorithm>
 #include <cmath>
 #include <cstdio>
@@ -491,17 +493,33 @@ __global__ void k_fields_in(XferFields F, const int* __restrict__ inv, int n, in
   else static_cast<double*>(F.dev[f])[k] = static_cast<const double*>(F.host[f])[i];
 }
 
-// host memory that a kernel can address, from its first byte to its last
+// Host memory that a kernel can address, all of it inside one page-locked
+// allocation or registration: two of them can hold an array's ends and leave
+// its middle pageable.  (The driver entry point comes through the runtime, so
+// that the library does not link the driver library.)
 static void* device_view(const void* host, size_t bytes) {
-  cudaPointerAttributes a{}, b{};
-  if (cudaPointerGetAttributes(&a, host) != cudaSuccess ||
-      cudaPointerGetAttributes(&b, static_cast<const char*>(host) + bytes - 1) != cudaSuccess) {
+  typedef CUresult (*GetAttributeFn)(void*, CUpointer_attribute, CUdeviceptr);
+  static const GetAttributeFn get = [] {
+    void* f = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    if (cudaGetDriverEntryPoint("cuPointerGetAttribute", &f, cudaEnableDefault, &q) != cudaSuccess ||
+        q != cudaDriverEntryPointSuccess)
+      f = nullptr;
+    return reinterpret_cast<GetAttributeFn>(f);
+  }();
+  cudaPointerAttributes a{};
+  if (!get || cudaPointerGetAttributes(&a, host) != cudaSuccess) {
     cudaGetLastError();
     return nullptr;
   }
-  if (a.type != cudaMemoryTypeHost || b.type != cudaMemoryTypeHost || !a.devicePointer || !b.devicePointer ||
-      static_cast<char*>(b.devicePointer) - static_cast<char*>(a.devicePointer) != (ptrdiff_t)bytes - 1)
+  if (a.type != cudaMemoryTypeHost || !a.devicePointer) return nullptr;
+  const CUdeviceptr p = (CUdeviceptr)(uintptr_t)a.devicePointer;
+  CUdeviceptr start = 0;
+  size_t size = 0;
+  if (get(&start, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, p) != CUDA_SUCCESS ||
+      get(&size, CU_POINTER_ATTRIBUTE_RANGE_SIZE, p) != CUDA_SUCCESS)
     return nullptr;
+  if (p < start || p - start > size || bytes > size - (size_t)(p - start)) return nullptr;
   return a.devicePointer;
 }
 

@@ -247,3 +247,28 @@ def test_static_forces_with_more_finds_than_the_fast_search_keeps(crowd):
     assert overflow_count(E.load()) == 0
     for f in OUT_FIELDS:
         np.testing.assert_array_equal(got[f], want[f], err_msg=f)
+
+
+def test_transfer_of_an_array_with_only_its_ends_page_locked():
+    import torch
+    n, page = 4096, 4096
+    parts, L = plane_disks(n, 0.5, seed=2)
+    e = Engine(n)
+    drive(e, parts, (L, L, 10.0), nlist=(2.4, 0.3), pairs=[SOFT], integrators=abp()).commit()
+    store = np.zeros(8 * n + page, np.uint8)
+    base = -store.ctypes.data % page
+    a = store[base:base + 8 * n].view(np.float64)
+    a[:] = np.arange(n)
+    rt = torch.cuda.cudart()
+    ends = (a.ctypes.data, a.ctypes.data + 8 * n - page)
+    for p in ends:
+        assert int(rt.cudaHostRegister(p, page, 0)) == 0
+    try:  # refused by the copies, not read by a kernel
+        with pytest.raises(engine.EngineError):
+            e.upload_fields({"vx": a})
+        with pytest.raises(engine.EngineError):
+            e.download_fields(["vx"], out={"vx": a})
+    finally:
+        for p in ends:
+            rt.cudaHostUnregister(p)
+    e.close()
