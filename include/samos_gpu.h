@@ -91,7 +91,8 @@ int  sg_download(sg_system* s, int replica, const char* field, void* host);
  * src/dump/dump.cpp:504-708): the same as one sg_upload / sg_download per
  * field, but every copy is enqueued back to back and the call waits once.
  * From page-locked host arrays (sg_host_alloc) the copies run at the link's
- * bandwidth.                                                                */
+ * bandwidth; up to 16 MB of them are read or written by one kernel instead of
+ * a copy per field.                                                         */
 int  sg_upload_fields(sg_system* s, int replica, int nfields, const char* const* fields,
                       const void* const* hosts);
 int  sg_download_fields(sg_system* s, int replica, int nfields, const char* const* fields,
@@ -258,7 +259,9 @@ int  sg_set_path(sg_system* s, int path);
  * tiled sweeps); all variants compute the same bits.  By default the engine's autotuner times every variant on the
  * first steps of a run and keeps the fastest; sg_set_variant pins one
  * (-1 re-enables tuning), sg_get_variant reports the choice (-1 = not yet
- * tuned).  No reference counterpart.                                        */
+ * tuned).  Without a pin, a system whose blocks are all resident at once is
+ * then stepped many steps per launch (same bits); a pinned one is stepped with
+ * its variant, one launch a step.  No reference counterpart.                */
 int  sg_set_variant(sg_system* s, int variant);
 int  sg_get_variant(const sg_system* s);
 /* Neighbour-list build kernel: 0 = automatic (lanes of a team share one

@@ -12,6 +12,9 @@
 // (With the rebuild inside the kernel, its registers came out of the step loop:
 // 65,536 particles on a sphere took 21 us a step instead of 13.)  The terms are
 // abp_pair_term and abp_advance, in the step kernels' order: same bits.
+// Bound by the step's own chain (records, FP64 terms, barrier): 2,000 disks for
+// 100 steps and the read-back 1.68 ms with a launch a step, 0.88 so; 65,536
+// particles on a sphere for 60 steps 1.56 and 1.05 ms.
 #pragma once
 #include "sg_abp_launch.h"
 

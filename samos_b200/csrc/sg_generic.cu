@@ -1,6 +1,10 @@
 // sg_generic.cu -- launches of the generic fused step (k_step_brownian): the
 // Vicsek model on a plane and soft + polar `brownian` particles on a curved
-// surface with their kinds fixed, every other program through the loops.
+// surface with their kinds fixed, every other program through the loops.  The
+// line is drawn by kinds alone, since the fixed kernel was the faster one at
+// every size (27 -> 16 us a step for 131,101 Vicsek particles, 21 -> 12 for
+// 50,021 on a torus); a mix without an instance here, several types, groups,
+// phase-in, external potentials and steps that report energies keep the loops.
 #include "sg_generic_launch.h"
 
 namespace sg {
