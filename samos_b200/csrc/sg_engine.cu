@@ -1966,15 +1966,18 @@ static int rebuild_pending(sg_system* s, int shape, bool last, double* rebuild_m
   return SG_OK;
 }
 
-// Rebuilds enqueued with the steps: taken up to kDevRebuildSlots slots.  60 steps
-// against the host-driven rebuild: 256 replicas 47 and 51 ms, 500,009 particles
-// 2.90 and 3.02, 4,194,304 disks 21.9 and 21.9; above that a step outlasts the
-// host's round trip, and the separate kernels of rebuild_flagged run each phase
-// at its own occupancy.
-static constexpr int kDevRebuildSlots = 5 << 20;
+// Rebuilds enqueued with the steps, for replicas of up to kDevRebuildReplica
+// slots.  20 steps from a random start (four rebuilds) against the host-driven
+// rebuild: 262,144 disks 1.37 and 1.82 ms, 524,288 2.09 and 2.45, 1,048,576 3.96
+// and 4.13, 2,097,152 6.78 and 6.49, 4,194,304 12.7 and 11.7: there the separate
+// kernels of rebuild_flagged run each phase at its own occupancy, and the round
+// trip is hidden.  256 replicas, 4 million slots, a few rebuilt after each step:
+// 47 and 51 ms for 60 steps.
+static constexpr int kDevRebuildSlots = 5 << 20, kDevRebuildReplica = 3 << 19;
 
 static bool dev_rebuild(const sg_system* s) {
-  return s->has_nlist && s->nrep <= RB_MAX_REP && s->slots <= kDevRebuildSlots && s->build_mode <= 1 && !s->profile &&
+  return s->has_nlist && s->nrep <= RB_MAX_REP && s->slots <= kDevRebuildSlots &&
+         *std::max_element(s->n.begin(), s->n.end()) <= kDevRebuildReplica && s->build_mode <= 1 && !s->profile &&
          !(s->abp_on && s->abp_variant == 8);
 }
 
